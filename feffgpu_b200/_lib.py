@@ -22,7 +22,7 @@ NOALLOC_SCRATCH_BYTES = 32 << 20    # FG_NOALLOC_SCRATCH_BYTES of include/feffgp
 
 # every entry point of include/feffgpu_b200.h
 EXPORTS = ("fg_stage_create", "fg_stage_destroy", "fg_stage_get_info", "fg_stage_lmax", "fg_stage_xk",
-           "fg_last_error", "fg_cchi", "fg_cchi_backward_workspace", "fg_cchi_backward", "fg_chi_fine",
+           "fg_last_error", "fg_cchi", "fg_cchi_ws", "fg_cchi_workspace", "fg_cchi_backward_workspace", "fg_cchi_backward", "fg_chi_fine",
            "fg_chi_fine_backward", "fg_chi_reduce_workspace", "fg_chi_reduce", "fg_chi_reduce_noalloc",
            "fg_chi_reduce_backward_workspace",
            "fg_chi_reduce_backward", "fg_set_kernel_timing", "fg_kernel_time_ms", "fg_fp32_fma_peak", "fg_set_launch",
@@ -63,6 +63,8 @@ _SIGS = {
     "fg_stage_xk": (C.c_int, [_P, _P]),
     "fg_last_error": (C.c_char_p, []),
     "fg_cchi": (C.c_int, [_P, C.c_int, C.c_int64, C.c_int32, _P, C.c_int32, _P, _P, _P, _P, _P]),
+    "fg_cchi_workspace": (C.c_size_t, [_P, C.c_int64, C.c_int32]),
+    "fg_cchi_ws": (C.c_int, [_P, C.c_int, C.c_int64, C.c_int32, _P, C.c_int32, _P, _P, _P, _P, _P, C.c_size_t, _P]),
     "fg_cchi_backward_workspace": (C.c_size_t, [_P, C.c_int64, C.c_int32]),
     "fg_cchi_backward": (C.c_int, [_P, C.c_int, C.c_int64, C.c_int32, _P, C.c_int32, _P, _P, _P, _P, _P, C.c_size_t,
                                    _P]),

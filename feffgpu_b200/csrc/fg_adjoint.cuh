@@ -18,7 +18,7 @@
 #pragma once
 #include <type_traits>
 
-#include "fg_kernels.cuh"
+#include "fg_shared.cuh"
 
 namespace fg {
 

@@ -406,7 +406,7 @@ FusedShape fused_shape(const fg_stage *s)
     return f;
 }
 
-StageView view(const fg_stage *s) { return StageView{s->E, s->L1, s->nph1, s->num_sms, s->ilinit, s->max_smem}; }
+StageView view(const fg_stage *s) { return StageView{s->E, s->L1, s->nph1, s->num_sms, s->ilinit, s->max_smem, s->iorder}; }
 
 // Calls F::template run<R, EDGE>(tables) for the stage's precision and initial-state class.
 // The kernels of the stage's edge class (l_init + 1) and lambda order (EDGE + 3 at order 3)
@@ -434,6 +434,13 @@ template <class F> fg_status by_kind(const fg_stage *s, fg_precision prec, F &&f
     }
 }
 
+// Bytes of the shared form's workspace in the larger of the two precisions (0 where it does not apply)
+size_t share_bytes(const fg_stage *s, int64_t n, int nleg_max)
+{
+    return std::max(share_plan(n, nleg_max, s->E, s->L1, false, s->iorder, s->ilinit).total,
+                    share_plan(n, nleg_max, s->E, s->L1, true, s->iorder, s->ilinit).total);
+}
+
 // Host-side checks of a batch's sizes and pointers; k_validate checks the contents (indices) on the device and
 // reports through the call's status word.
 fg_status check_paths(const fg_paths *P)
@@ -450,9 +457,16 @@ fg_status check_paths(const fg_paths *P)
 
 }  // namespace
 
-extern "C" fg_status fg_cchi(const fg_stage *s, fg_precision prec, int64_t B, int32_t nleg, const void *coords,
-                             int32_t coords_f64, const int64_t *ipots, void *cchi, void *reff, int32_t *bad_ipot,
-                             void *stream)
+extern "C" size_t fg_cchi_workspace(const fg_stage *s, int64_t B, int32_t nleg)
+{
+    if (!s || B < 0 || nleg < 2 || nleg > kMaxLeg) return 0;
+    const size_t n = share_bytes(s, B, nleg);
+    return n ? kCounterBytes + n : 0;
+}
+
+extern "C" fg_status fg_cchi_ws(const fg_stage *s, fg_precision prec, int64_t B, int32_t nleg, const void *coords,
+                                int32_t coords_f64, const int64_t *ipots, void *cchi, void *reff, int32_t *bad_ipot,
+                                void *workspace, size_t workspace_bytes, void *stream)
 {
     g_err.clear();
     if (!s) return fail(FG_ERR_VALUE, "null stage");
@@ -464,8 +478,16 @@ extern "C" fg_status fg_cchi(const fg_stage *s, fg_precision prec, int64_t B, in
     const StageView sv = view(s);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return by_kind(s, prec, [&](auto L, const auto &T) {
-        return decltype(L)::cchi(sv, T, B, nleg, coords, coords_f64, ipots, cchi, reff, bad_ipot, fwd_warps(s), st);
+        return decltype(L)::cchi(sv, T, B, nleg, coords, coords_f64, ipots, cchi, reff, bad_ipot, fwd_warps(s),
+                                 static_cast<unsigned char *>(workspace), workspace ? workspace_bytes : 0, st);
     });
+}
+
+extern "C" fg_status fg_cchi(const fg_stage *s, fg_precision prec, int64_t B, int32_t nleg, const void *coords,
+                             int32_t coords_f64, const int64_t *ipots, void *cchi, void *reff, int32_t *bad_ipot,
+                             void *stream)
+{
+    return fg_cchi_ws(s, prec, B, nleg, coords, coords_f64, ipots, cchi, reff, bad_ipot, nullptr, 0, stream);
 }
 
 extern "C" size_t fg_cchi_backward_workspace(const fg_stage *s, int64_t B, int32_t nleg)
@@ -536,7 +558,7 @@ extern "C" fg_status fg_chi_fine_backward(const fg_stage *s, fg_precision prec, 
 extern "C" size_t fg_chi_reduce_workspace(const fg_stage *s, const fg_paths *P, int32_t NK)
 {
     if (!s || !P || NK < 0) return 0;
-    return fused_workspace(P, NK);
+    return fused_workspace(P, NK) + share_bytes(s, P->n, P->nleg_max);
 }
 
 extern "C" fg_status fg_chi_reduce(const fg_stage *s, fg_precision prec, const fg_paths *P, int32_t NK,
@@ -558,7 +580,8 @@ extern "C" fg_status fg_chi_reduce(const fg_stage *s, fg_precision prec, const f
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (fg_status rc = by_kind(s, prec, [&](auto L, const auto &T) {
             return decltype(L)::fused(sv, T, P, NK, q, S, span, rows, cchi_save, reff_save,
-                                      static_cast<unsigned char *>(workspace), fused_shape(s), st);
+                                      static_cast<unsigned char *>(workspace), fused_shape(s), st, nullptr,
+                                      static_cast<unsigned char *>(workspace) + need, workspace_bytes - need);
         }))
         return rc;
     return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st);
@@ -583,7 +606,9 @@ extern "C" fg_status fg_chi_reduce_words(const fg_stage *s, fg_precision prec, c
     if (fg_status rc = by_kind(s, prec, [&](auto L, const auto &T) {
             return decltype(L)::fused(sv, T, P, NK, q, S, span, nullptr, cchi_save, reff_save,
                                       static_cast<unsigned char *>(workspace), fused_shape(s), st,
-                                      reinterpret_cast<unsigned long long *>(words));
+                                      reinterpret_cast<unsigned long long *>(words),
+                                      static_cast<unsigned char *>(workspace) + kCounterBytes,
+                                      workspace_bytes - kCounterBytes);
         }))
         return rc;
     return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st);

@@ -40,6 +40,36 @@ __device__ __forceinline__ void canon_mn(int MM, int r, int &m1, int &m2)
     m2 = r % (2 * MM + 1) - MM;
 }
 
+// Canonical entry r of one scatterer's rotation table D(beta), il = 1..L1, into column r of out (row stride DS).
+template <typename R>
+__device__ __forceinline__ void rotation_column(R *out, const Tables<R> &T, double b, int MM, int DS, int r)
+{
+    const int L1 = T.L1;
+    int m1, m2;
+    canon_mn(MM, r, m1, m2);
+    const double c = cos(b), c2 = cos(0.5 * b), s2 = sin(0.5 * b);
+    out += r;
+    const double *xf = T.xfac + (m1 + 3) * 7 + (m2 + 3);
+    double dm1 = 0.0, d0 = 0.0;
+    const int lseed = min(L1, 4);
+    for (int l = 0; l < lseed; ++l) {             // l <= 3: Wigner's explicit sum
+        const double dl = wigner_small(l, m1, m2, c2, s2, seed_table(T));
+        out[(size_t)(l + 1) * DS] = (R)(dl * xf[(size_t)(l + 1) * 49]);
+        dm1 = d0;
+        d0 = dl;
+    }
+    // the three-term recursion: its coefficient loads do not depend on it, so the unrolled trips issue them
+    // ahead of the dependent multiply-adds
+#pragma unroll 4
+    for (int l = lseed; l < L1; ++l) {
+        const double *q = T.rc + (((size_t)(l - 1) * 7 + (m1 + 3)) * 7 + (m2 + 3)) * 3;
+        const double dl = fma(fma(q[0], c, -q[1]), d0, -q[2] * dm1);
+        out[(size_t)(l + 1) * DS] = (R)(dl * xf[(size_t)(l + 1) * 49]);
+        dm1 = d0;
+        d0 = dl;
+    }
+}
+
 // Warp-cooperative setup of one path: geometry (FP64), Euler phases, rotation tables of legs 1..nsc (unless
 // tables is false: the adjoint forms them with their derivatives) and the termination's rotation matrices.
 // coords: (nleg, 3) angstrom (float or double), ipots: (nleg).
@@ -80,33 +110,8 @@ __device__ void path_setup(WarpPath<R> &g, R *dh, const Tables<R> &T, const CT *
     }
     // rotation tables D^(k), k = 1..nsc, il = 1..L1
     const int NC = ncanon(MM), DS = dstride(MM), L1 = T.L1;
-    for (int task = lane; tables && task < nsc * NC; task += 32) {
-        const int k = task / NC + 1, r = task % NC;
-        int m1, m2;
-        canon_mn(MM, r, m1, m2);
-        const double b = g.beta[k];
-        const double c = cos(b), c2 = cos(0.5 * b), s2 = sin(0.5 * b);
-        R *out = dh + (size_t)(k - 1) * (L1 + 1) * DS + r;
-        const double *xf = T.xfac + (m1 + 3) * 7 + (m2 + 3);
-        double dm1 = 0.0, d0 = 0.0;
-        const int lseed = min(L1, 4);
-        for (int l = 0; l < lseed; ++l) {             // l <= 3: Wigner's explicit sum
-            const double dl = wigner_small(l, m1, m2, c2, s2, seed_table(T));
-            out[(size_t)(l + 1) * DS] = (R)(dl * xf[(size_t)(l + 1) * 49]);
-            dm1 = d0;
-            d0 = dl;
-        }
-        // the three-term recursion: its coefficient loads do not depend on it, so the unrolled trips issue them
-        // ahead of the dependent multiply-adds
-#pragma unroll 4
-        for (int l = lseed; l < L1; ++l) {
-            const double *q = T.rc + (((size_t)(l - 1) * 7 + (m1 + 3)) * 7 + (m2 + 3)) * 3;
-            const double dl = fma(fma(q[0], c, -q[1]), d0, -q[2] * dm1);
-            out[(size_t)(l + 1) * DS] = (R)(dl * xf[(size_t)(l + 1) * 49]);
-            dm1 = d0;
-            d0 = dl;
-        }
-    }
+    for (int task = lane; tables && task < nsc * NC; task += 32)
+        rotation_column<R>(dh + (size_t)(task / NC) * (L1 + 1) * DS, T, g.beta[task / NC + 1], MM, DS, task % NC);
     // termination rotation matrices at the absorber (beta_nleg), l_t <= 3
     for (int task = lane; task < T.nterm * 49; task += 32) {
         const int t = task / 49, m1 = (task % 49) / 7 - 3, m2 = task % 7 - 3;

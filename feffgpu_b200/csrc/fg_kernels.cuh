@@ -60,8 +60,10 @@ __device__ __forceinline__ C2<R> path_energy(const WarpPath<R> &g, const R *dh, 
 template <typename R, int EDGE, typename CT>
 __global__ void __launch_bounds__(256) k_cchi(Tables<R> T, const CT *__restrict__ coords,
                                                const int64_t *__restrict__ ipots, int64_t B, int nleg,
-                                               C2<R> *__restrict__ out, R *__restrict__ reff, int *bad, size_t wbytes)
+                                               C2<R> *__restrict__ out, R *__restrict__ reff, int *bad, size_t wbytes,
+                                               const int *gate)
 {
+    if (gate && !*(volatile const int *)gate) return;       // the shared-matrix form took the call
     using K = Kinds<EDGE>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -172,6 +174,36 @@ struct PathsDev {
     const int *row;
 };
 
+// One path's weighted fine-grid terms from its signal (load(e)), each added exactly to the path's row: amplitude and
+// unwrapped phase (into amp and pha), interpolation, deg exp(-2 sigma2 q^2) a(q) sin(phi(q) + 2 q reff).
+template <typename R, class Load>
+__device__ __forceinline__ void path_terms(const PathsDev &P, int64_t p, int E, int NK, int lane,
+                                           const double *__restrict__ q, const double *__restrict__ S,
+                                           const int *__restrict__ span, const Load &load, double *amp, double *pha,
+                                           double rf, unsigned long long *racc, int *status)
+{
+    amp_phase<R>(E, lane, load, amp, pha);
+    __syncwarp();
+    const double wdeg = P.deg[p], s2 = P.sigma2 ? P.sigma2[p] : 0.0;
+    unsigned long long *acc_row = racc + (size_t)P.row[p] * NK;
+    for (int k0 = 0; k0 < NK; k0 += 32) {
+        const int k = k0 + lane;
+        if (k < NK) {
+            const int lo = span[2 * k], hi = span[2 * k + 1];
+            double a = 0.0, ph = 0.0;
+            for (int j = lo; j < hi; ++j) {
+                const double sv = S[(size_t)k * E + j];
+                a += sv * amp[j];
+                ph += sv * pha[j];
+            }
+            const double qk = q[k];
+            const double damp = s2 != 0.0 ? exp(-2.0 * s2 * qk * qk) : 1.0;   // exact 1 without sigma^2
+            const double v = wdeg * a * sin_arg<R>(ph + 2.0 * qk * rf) * damp;
+            if (!fixed_add(acc_row + k, (size_t)P.nrows * NK, v)) atomicOr(status, kBadRange);
+        }
+    }
+}
+
 // Fused forward: every path of the batch, all leg counts, from one work queue (costliest first); per path the
 // signal at all E, its amplitude and unwrapped phase, and the weighted fine-grid terms
 // deg exp(-2 sigma2 q^2) a(q) sin(phi(q) + 2 q reff), each added exactly to its row (fixed_add).  The batch's
@@ -189,11 +221,12 @@ __global__ void __launch_bounds__(128, MINB)
     k_fused(Tables<R> T, PathsDev P, int NK, const double *__restrict__ q, const double *__restrict__ S,
             const int *__restrict__ span, unsigned long long *__restrict__ racc, C2<R> *__restrict__ cchi_save,
             double *__restrict__ reff_save, unsigned long long *counter, int *status, int nsc_max, size_t wbytes,
-            int stage_t)
+            int stage_t, const int *gate)
 {
     using K = Kinds<EDGE>;
     extern __shared__ __align__(16) unsigned char smem[];
     if (*(volatile const int *)status & kBadLayout) return;
+    if (gate && !*(volatile const int *)gate) return;       // the shared-matrix form took the call
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int E = T.E, L1 = T.L1;
     unsigned char *base = smem + (size_t)w * wbytes;
@@ -223,26 +256,8 @@ __global__ void __launch_bounds__(128, MINB)
             }
         }
         __syncwarp();
-        amp_phase<R>(E, lane, [&](int e) { return cbuf[e]; }, amp, pha);
-        __syncwarp();
-        const double rf = g.reff * kBohr, wdeg = P.deg[p], s2 = P.sigma2 ? P.sigma2[p] : 0.0;
-        unsigned long long *acc_row = racc + (size_t)P.row[p] * NK;
-        for (int k0 = 0; k0 < NK; k0 += 32) {
-            const int k = k0 + lane;
-            if (k < NK) {
-                const int lo = span[2 * k], hi = span[2 * k + 1];
-                double a = 0.0, ph = 0.0;
-                for (int j = lo; j < hi; ++j) {
-                    const double sv = S[(size_t)k * E + j];
-                    a += sv * amp[j];
-                    ph += sv * pha[j];
-                }
-                const double qk = q[k];
-                const double damp = s2 != 0.0 ? exp(-2.0 * s2 * qk * qk) : 1.0;   // exact 1 without sigma^2
-                const double v = wdeg * a * sin_arg<R>(ph + 2.0 * qk * rf) * damp;
-                if (!fixed_add(acc_row + k, (size_t)P.nrows * NK, v)) atomicOr(status, kBadRange);
-            }
-        }
+        const double rf = g.reff * kBohr;
+        path_terms<R>(P, p, E, NK, lane, q, S, span, [&](int e) { return cbuf[e]; }, amp, pha, rf, racc, status);
         if (lane == 0 && reff_save) reff_save[p] = rf;
         __syncwarp();
     }
@@ -260,70 +275,25 @@ inline fg_status grid_for(KernelT kern, int threads, size_t smem, int num_sms, i
     return FG_OK;
 }
 
+// The one-kernel form over pd's paths; gate: it returns at once unless *gate is set (null: always runs).
 template <typename R, int EDGE>
-fg_status Launch<R, EDGE>::cchi(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const void *coords,
-                                int coords_f64, const int64_t *ipots, void *cchi, void *reff, int *bad, int warps,
-                                cudaStream_t st)
+fg_status launch_fused(const StageView &sv, const Tables<R> &T, const PathsDev &pd, int NK, const double *q,
+                       const double *S, const int *span, unsigned long long *racc, void *cchi_save, double *reff_save,
+                       unsigned long long *counter, int *status, const FusedShape &shape, const int *gate,
+                       cudaStream_t st)
 {
     using K = Kinds<EDGE>;
-    const int MM = nleg == 2 ? K::MMSS : K::MMMS;
-    const size_t wb = warp_bytes<R>(sv.L1, nleg - 1, MM, sv.E, false);
-    warps = fit_warps(warps, wb, sv.max_smem);
+    const int nsc_max = pd.nleg_max - 1;
+    const size_t wb = warp_bytes<R>(sv.L1, nsc_max, K::MM, sv.E, true, shape.stage_t);
+    const int warps = fit_warps(shape.warps > 4 ? 4 : shape.warps, wb, sv.max_smem);
     const int threads = warps * 32;
-    const size_t smem = wb * warps;
+    auto kern = shape.regs_alt ? k_fused<R, EDGE, FusedMinBlocks<R>::alt> : k_fused<R, EDGE, FusedMinBlocks<R>::def>;
     int blocks = 0;
-    if (coords_f64) {
-        auto kern = k_cchi<R, EDGE, double>;
-        if (fg_status rc = grid_for(kern, threads, smem, sv.num_sms, B, blocks)) return rc;
-        timer_begin(st);
-        kern<<<blocks, threads, smem, st>>>(T, static_cast<const double *>(coords), ipots, B, nleg,
-                                            static_cast<C2<R> *>(cchi), static_cast<R *>(reff), bad, wb);
-    } else {
-        auto kern = k_cchi<R, EDGE, float>;
-        if (fg_status rc = grid_for(kern, threads, smem, sv.num_sms, B, blocks)) return rc;
-        timer_begin(st);
-        kern<<<blocks, threads, smem, st>>>(T, static_cast<const float *>(coords), ipots, B, nleg,
-                                            static_cast<C2<R> *>(cchi), static_cast<R *>(reff), bad, wb);
-    }
-    timer_end(st);
+    if (fg_status rc = grid_for(kern, threads, wb * warps, sv.num_sms, pd.n, blocks)) return rc;
+    kern<<<blocks, threads, wb * warps, st>>>(T, pd, NK, q, S, span, racc, static_cast<C2<R> *>(cchi_save), reff_save,
+                                              counter, status, nsc_max, wb, shape.stage_t ? 1 : 0, gate);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
-}
-
-template <typename R, int EDGE>
-fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const fg_paths *P, int NK, const double *q,
-                                 const double *S, const int *span, double *rows, void *cchi_save, double *reff_save,
-                                 unsigned char *ws, const FusedShape &shape, cudaStream_t st,
-                                 unsigned long long *words)
-{
-    using K = Kinds<EDGE>;
-    unsigned long long *counter = reinterpret_cast<unsigned long long *>(ws);
-    int *status = reinterpret_cast<int *>(ws + kStatusOffset);
-    unsigned long long *racc = words ? words : reinterpret_cast<unsigned long long *>(ws + kCounterBytes);
-    if (words) {
-        FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes, st));
-        FG_CUDA(cudaMemsetAsync(words, 0, (size_t)2 * P->nrows * NK * sizeof(unsigned long long), st));
-    } else {
-        FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes + row_sum_bytes(P->nrows, NK), st));
-    }
-    if (fg_status rc = launch_validate(P, sv.nph1, status, st)) return rc;
-    if (P->n > 0) {
-        const int nsc_max = P->nleg_max - 1;
-        const size_t wb = warp_bytes<R>(sv.L1, nsc_max, K::MM, sv.E, true, shape.stage_t);
-        const int warps = fit_warps(shape.warps > 4 ? 4 : shape.warps, wb, sv.max_smem);
-        const int threads = warps * 32;
-        auto kern = shape.regs_alt ? k_fused<R, EDGE, FusedMinBlocks<R>::alt> : k_fused<R, EDGE, FusedMinBlocks<R>::def>;
-        int blocks = 0;
-        if (fg_status rc = grid_for(kern, threads, wb * warps, sv.num_sms, P->n, blocks)) return rc;
-        PathsDev pd{P->n, P->nleg_max, P->nrows, P->coords, P->ipots, P->nleg, P->deg, P->sigma2, P->order, P->row};
-        timer_begin(st);
-        kern<<<blocks, threads, wb * warps, st>>>(T, pd, NK, q, S, span, racc, static_cast<C2<R> *>(cchi_save),
-                                                  reff_save, counter, status, nsc_max, wb, shape.stage_t ? 1 : 0);
-        timer_end(st);
-        FG_CUDA(cudaGetLastError());
-    }
-    if (!rows) return FG_OK;
-    return launch_row_finish(P->nrows, NK, racc, rows, status, st);
 }
 
 template <typename R>

@@ -22,6 +22,7 @@ constexpr int kGparStride = 32;         // per path in the fused backward's work
 struct StageView {
     int E, L1, nph1, num_sms, ilinit;
     int max_smem;   // opt-in shared memory per block (bytes)
+    int iorder;
 };
 
 // Warps per block that fit the per-warp shared memory (at least 1; the launch reports a block that does not fit)
@@ -45,12 +46,13 @@ struct FusedShape {
 template <typename R, int EDGE> struct Launch {
     static fg_status cchi(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const void *coords,
                           int coords_f64, const int64_t *ipots, void *cchi, void *reff, int *bad, int warps,
-                          cudaStream_t st);
+                          unsigned char *ws, size_t ws_bytes, cudaStream_t st);
     // rows null: the exact sums are left in words (2 x nrows x NK, see fg_chi_reduce_words) instead of finished
     static fg_status fused(const StageView &sv, const Tables<R> &T, const fg_paths *P, int NK, const double *q,
                            const double *S, const int *span, double *rows, void *cchi_save, double *reff_save,
                            unsigned char *ws, const FusedShape &shape, cudaStream_t st,
-                           unsigned long long *words = nullptr);
+                           unsigned long long *words = nullptr, unsigned char *share_ws = nullptr,
+                           size_t share_bytes = 0);
     static fg_status cchi_bwd(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const void *coords,
                               int coords_f64, const int64_t *ipots, const void *grad_cchi, const void *grad_reff,
                               void *grad_coords, unsigned char *ws, int warps, cudaStream_t st);
@@ -112,6 +114,50 @@ fg_status describe_paths_warp(int64_t B, int32_t nleg, const int32_t *seq, const
                               const int64_t *absorbers, const fg_pf_tables *T, const uint8_t *keep, float *coords,
                               int64_t *ipots, int64_t *atoms, float *rtot, float *xport, int64_t *key, float *c1,
                               int64_t *ip1, cudaStream_t st);
+
+// ---- the path signal with shared scattering matrices (fg_shared.cuh) -------------------------------------------------
+struct __align__(16) ShareKey { unsigned long long x, y, z, w; };   // leg, next leg, beta (FP64 bits), potential
+constexpr int kShareMin = 2;                               // least scatterers per class that make the form worth taking
+constexpr int64_t kShareSub = 1 << 18;                     // paths per sub-batch (bounds the workspace)
+constexpr int64_t kShareWorth = 1 << 15;                   // (path, 32 energies) items worth looking for classes
+constexpr int64_t kShareSmall = 8192;                      // (path, 32 energies) items of a small call
+constexpr size_t kShareMatrixBytes = (size_t)1 << 30;      // the classes' matrices: 2e5 classes, 32 energies, FP32
+struct ShareHead {                      // counters of one sub-batch, in the workspace head
+    int classes, two, general, pad;     // classes, two-leg paths, 1: the one-kernel form evaluates this sub-batch
+    long long scatterers;               // scatterers of paths of three and more legs
+};
+constexpr size_t kShareHeadOffset = 128;
+// A sub-batch's classes and the arrays they are found with.
+struct ShareIdx {
+    int64_t n;                   // paths of the sub-batch
+    int stride, nsc_max;         // leg dimension of coords and ipots, scatterers per path at most
+    const int *nlegs;            // null: every path has nleg_uniform legs
+    int nleg_uniform;
+    const int *order;            // null: 0..n-1
+    ShareKey *key;               // n * nsc_max keys
+    int *slot_of;                // n * nsc_max hash slots
+    unsigned *hash;              // owners (scatterer index, 0xffffffff: empty), hmask + 1 of them
+    unsigned hmask;
+    int *cls;                    // the class of an occupied slot
+    unsigned *owner;             // the scatterer that represents a class, cls_cap of them
+    int64_t cls_cap;
+    ShareHead *head;
+    const int *status;           // may be null
+    __device__ __forceinline__ int legs(int64_t p) const { return nlegs ? nlegs[p] : nleg_uniform; }
+    __device__ __forceinline__ bool refused() const { return status && (*(volatile const int *)status & kBadLayout); }
+};
+fg_status launch_share_insert(const ShareIdx &s, cudaStream_t st);
+
+// Sizes and offsets of the shared form's workspace for calls of n paths of up to nleg_max legs; sub: paths per
+// sub-batch (0: the form does not apply).
+struct SharePlan {
+    int64_t sub = 0, cls_cap = 0;
+    int nsc_max = 0, chunks = 0, passes = 0, split = 1, force = 0;
+    unsigned hcap = 0;
+    size_t rec = 0, key = 0, slot = 0, hash = 0, cls = 0, owner = 0, two = 0, tab = 0, F = 0, f_bytes = 0, sig = 0,
+           total = 0;
+};
+SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit);
 
 // Events around the main kernel of a call when kernel timing is on (fg_set_kernel_timing)
 void timer_begin(cudaStream_t st);

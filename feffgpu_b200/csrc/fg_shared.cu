@@ -1,0 +1,102 @@
+// fg_shared.cu -- classes of equal scatterers (fg_shared.cuh) and the sizes of their workspace.
+#include <algorithm>
+
+#include "fg_forward.cuh"
+#include "fg_launch.h"
+
+namespace fg {
+namespace {
+__device__ __forceinline__ unsigned key_hash(const ShareKey &k)
+{
+    // each word's bits spread by an odd multiplier, folded (the finaliser of MurmurHash3, Appleby, public domain)
+    unsigned long long h = k.x * 0x9e3779b97f4a7c15ull ^ (k.y * 0xc2b2ae3d27d4eb4full + k.w) ^ (k.z * 0x165667b19e3779f9ull);
+    h ^= h >> 33; h *= 0xff51afd7ed558ccdull;
+    h ^= h >> 33; h *= 0xc4ceb9fe1a85ec53ull;
+    return (unsigned)(h ^ (h >> 33));
+}
+
+// A thread per scatterer: linear probing; a slot belongs to the first scatterer that claimed it, and every scatterer
+// whose key equals the owner's bit for bit is of its class.  The table has at least twice as many slots as scatterers.
+__global__ void __launch_bounds__(256) k_share_insert(ShareIdx s)
+{
+    if (s.refused()) return;
+    const int64_t total = s.n * s.nsc_max;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = t / s.nsc_max;
+        const int nleg = s.legs(s.order ? s.order[i] : i);
+        const bool live = nleg > 2 && (int)(t % s.nsc_max) < nleg - 1;
+        const unsigned votes = __ballot_sync(__activemask(), live);
+        if (!live) continue;
+        if ((threadIdx.x & 31) == __ffs(votes) - 1) atomicAdd((unsigned long long *)&s.head->scatterers, (unsigned long long)__popc(votes));
+        const ShareKey k = s.key[t];
+        unsigned h = key_hash(k) & s.hmask;
+        for (unsigned probe = 0; probe <= s.hmask; ++probe, h = (h + 1) & s.hmask) {
+            const unsigned was = atomicCAS(s.hash + h, 0xffffffffu, (unsigned)t);
+            if (was == 0xffffffffu) {
+                const int c = atomicAdd(&s.head->classes, 1);
+                s.cls[h] = c;
+                if (c < s.cls_cap) s.owner[c] = (unsigned)t;
+                break;
+            }
+            const ShareKey o = s.key[was];
+            if (o.x == k.x && o.y == k.y && o.z == k.z && o.w == k.w) break;
+        }
+        s.slot_of[t] = (int)h;
+    }
+}
+}  // namespace
+
+fg_status launch_share_insert(const ShareIdx &s, cudaStream_t st)
+{
+    const int64_t total = s.n * s.nsc_max;
+    k_share_insert<<<(int)std::min<int64_t>((total + 255) / 256, 148 * 8), 256, 0, st>>>(s);
+    FG_CUDA(cudaGetLastError());
+    return FG_OK;
+}
+
+SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit)
+{
+    SharePlan p;
+    if (iorder > 2 || n < 1) return p;
+    // Lists of up to three legs share nothing (every scatterer has the absorber on one side and the path's only other
+    // atom on the other), so they take this form only where few paths leave the chip idle and it spreads their energies
+    // over warps: many energies, or the fifteen-column single scattering of L and M edges (897 paths, L3, 59 energies:
+    // 342 -> 245 us; at the K edge on 60 energies the extra launches cost more than the spreading gains: 421 -> 474 us).
+    // Longer paths take it wherever the call is worth the launches that find the classes (about 40 us): at two chunks
+    // of energies and 4,438 paths of up to four legs, 1.27 scatterers per class, looking for them cost 5 %.
+    const int chunks = (E + 31) / 32;
+    const bool small = n * chunks <= kShareSmall && (chunks >= 4 || ilinit > 1);
+    if (!small && (nleg_max < 4 || (chunks < 4 && n * chunks <= kShareWorth))) return p;
+    const size_t real = fp64 ? 8 : 4;
+    p.sub = std::min<int64_t>(n, kShareSub);
+    p.nsc_max = nleg_max - 1;
+    p.chunks = chunks;
+    const int64_t scat = p.sub * p.nsc_max;
+    const size_t per = 20 * 2 * real * 32;          // one class, one chunk: 20 canonical entries (orders 0-2)
+    const size_t all = (size_t)scat * p.chunks * per;
+    p.f_bytes = std::min(all, kShareMatrixBytes);
+    p.cls_cap = std::min<int64_t>(scat, (int64_t)(p.f_bytes / per));
+    const int fit = (int)std::min<size_t>(p.chunks, p.f_bytes / ((size_t)scat * per));   // chunks per pass at worst
+    p.passes = fit ? (p.chunks + fit - 1) / fit : p.chunks;
+    p.force = small && fit == p.chunks;
+    // small calls spread a path's energies over warps; large ones load its record once per pass
+    p.split = p.sub < 148 * 12 ? chunks : 1;
+    p.hcap = 64;
+    while ((int64_t)p.hcap < 2 * scat) p.hcap *= 2;
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += align_up(bytes, 256); return o; };
+    p.rec = take((size_t)p.sub * align_up(fp64 ? sizeof(WarpPath<double>) : sizeof(WarpPath<float>), 16));
+    p.key = take((size_t)scat * sizeof(ShareKey));
+    p.slot = take((size_t)scat * 4);
+    p.hash = take((size_t)p.hcap * 4);
+    p.cls = take((size_t)p.hcap * 4);
+    p.owner = take((size_t)p.cls_cap * 4);
+    p.two = take((size_t)p.sub * 4);
+    p.tab = take((size_t)p.cls_cap * (L1 + 1) * dstride(2) * real);
+    p.F = take(p.f_bytes);
+    p.sig = take((size_t)p.sub * E * 2 * real);
+    p.total = at;
+    return p;
+}
+
+}  // namespace fg

@@ -139,8 +139,11 @@ class GPUPathStage:
         ipots = ipots.contiguous()
         out = torch.empty(B, self.E, device=self.device, dtype=self.cdtype)
         reff = torch.empty(B, device=self.device, dtype=self.rdtype)
-        _lib.check(self._lib.fg_cchi(self._h, self.prec, B, nleg, coords.data_ptr(), int(coords.dtype == torch.float64),
-                                     ipots.data_ptr(), out.data_ptr(), reff.data_ptr(), None, _stream(self.device)))
+        ws_n = int(self._lib.fg_cchi_workspace(self._h, B, nleg))
+        ws = torch.empty(ws_n, device=self.device, dtype=torch.uint8) if ws_n else None
+        _lib.check(self._lib.fg_cchi_ws(self._h, self.prec, B, nleg, coords.data_ptr(),
+                                        int(coords.dtype == torch.float64), ipots.data_ptr(), out.data_ptr(),
+                                        reff.data_ptr(), None, _ptr(ws), ws_n, _stream(self.device)))
         return out, reff
 
     def _cchi_backward(self, coords, ipots, g_cchi, g_reff):
@@ -387,7 +390,8 @@ class GPUPathStage:
         NK = q.shape[0]
         ps = self._paths_struct(batch, coords, sigma2)
         words = torch.empty(2, batch.nrows, NK, device=self.device, dtype=torch.int64)
-        ws = batch.workspace(256)
+        ws_n = int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK))
+        ws = torch.empty(max(ws_n, 256), device=self.device, dtype=torch.uint8)
         cchi = reff = None
         if save:
             cchi = torch.empty(batch.n, self.E, device=self.device,
@@ -395,7 +399,7 @@ class GPUPathStage:
             reff = torch.empty(batch.n, device=self.device, dtype=torch.float64)
         _lib.check(self._lib.fg_chi_reduce_words(self._h, prec, C.byref(ps), NK, q.data_ptr(), S.data_ptr(),
                                                  self._span(S).data_ptr(), words.data_ptr(), _ptr(cchi), _ptr(reff),
-                                                 ws.data_ptr(), 256, _stream(self.device)))
+                                                 ws.data_ptr(), ws.numel(), _stream(self.device)))
         return words, cchi, reff
 
     def _chi_reduce_forward(self, batch, coords, sigma2, q, S, prec, save: bool):
@@ -404,7 +408,7 @@ class GPUPathStage:
         ps = self._paths_struct(batch, coords, sigma2)
         rows = torch.empty(batch.nrows, NK, device=self.device, dtype=torch.float64)
         ws_n = int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK))
-        ws = batch.workspace(ws_n)
+        ws = torch.empty(max(ws_n, 1), device=self.device, dtype=torch.uint8)
         cchi = reff = None
         if save:
             cchi = torch.empty(batch.n, self.E, device=self.device,

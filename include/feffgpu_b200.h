@@ -92,6 +92,13 @@ FG_API const char *fg_last_error(void);
  * (a device int32, left untouched when every index is valid). */
 FG_API fg_status fg_cchi(const fg_stage *stage, fg_precision prec, int64_t B, int32_t nleg, const void *coords,
                   int32_t coords_f64, const int64_t *ipots, void *cchi, void *reff, int32_t *bad_ipot, void *stream);
+/* The same call with device scratch: with workspace_bytes >= fg_cchi_workspace(...) (0: it would not be used) equal
+ * scatterers of the paths are evaluated once and small calls spread their energies over the GPU; with less, as fg_cchi.
+ * The workspace is free again when the call's work on `stream` is done. */
+FG_API size_t fg_cchi_workspace(const fg_stage *stage, int64_t B, int32_t nleg);
+FG_API fg_status fg_cchi_ws(const fg_stage *stage, fg_precision prec, int64_t B, int32_t nleg, const void *coords,
+                  int32_t coords_f64, const int64_t *ipots, void *cchi, void *reff, int32_t *bad_ipot,
+                  void *workspace, size_t workspace_bytes, void *stream);
 
 /* Adjoint of fg_cchi: grad_coords (B, nleg, 3) = d(loss)/d(coords) from grad_cchi (B, E) complex with PyTorch's
  * convention d(loss)/d(Re) + i d(loss)/d(Im), and grad_reff (B) (may be NULL).  grad_coords has the precision's
@@ -134,8 +141,10 @@ typedef struct fg_paths {
  * stream capture it returns without waiting (a graph replay with such an input gives NaN rows).  Host pointers and
  * sizes are checked before any launch. */
 
-/* Workspace of the fused calls: a work-queue counter and status word, and the rows' exact sums (2 x nrows x NK 64-bit
- * words; no per-path storage). */
+/* Workspace of the fused calls: a work-queue counter and status word, the rows' exact sums (2 x nrows x NK 64-bit
+ * words) and, for batches with paths of four and more legs and for small ones, the arrays with which equal scatterers
+ * of the paths are evaluated once (up to about 3 GB, whatever the number of paths).  A call given only the first two
+ * (256 + 16 nrows NK bytes, rounded up to 256) evaluates every scatterer on its own; the rows are the same. */
 FG_API size_t fg_chi_reduce_workspace(const fg_stage *stage, const fg_paths *paths, int32_t NK);
 
 /* rows (nrows, NK) FP64 = sum over paths p of deg_p exp(-2 sigma2_p q^2) chi_p(q), chi_p from cchi and chi_fine
@@ -155,7 +164,8 @@ FG_API fg_status fg_chi_reduce(const fg_stage *stage, fg_precision prec, const f
  * 2^64) and words[nrows * NK + r * NK + k] the low word (the next 32 bits of every term, summed).  Words of partial
  * sums add exactly as 64-bit integers, so summing them over several GPUs (an integer all-reduce) and then calling
  * fg_rows_from_words gives rows bit for bit equal to one call over all the paths, whatever the number of GPUs or
- * the split.  The workspace needs only its 256-byte head.  No reference counterpart. */
+ * the split.  The workspace needs only its 256-byte head; one of fg_chi_reduce_workspace(...) bytes lets equal
+ * scatterers be evaluated once.  No reference counterpart. */
 FG_API fg_status fg_chi_reduce_words(const fg_stage *stage, fg_precision prec, const fg_paths *paths, int32_t NK,
                                      const double *q, const double *S, const int32_t *span, uint64_t *words,
                                      void *cchi_save, double *reff_save, void *workspace, size_t workspace_bytes,
@@ -168,7 +178,7 @@ FG_API fg_status fg_rows_from_words(int64_t nrows, int32_t NK, const uint64_t *w
  * control (a simulation code that reserves the whole device for its own pool at start-up) and so cannot provide
  * the workspace fg_chi_reduce asks for.  Instead of a caller workspace it uses an array compiled into the library,
  * FG_NOALLOC_SCRATCH_BYTES (32 MiB) on every GPU that loads the library, held until the process exits; a batch
- * whose fg_chi_reduce_workspace exceeds that (more than about 5,200 rows at 401 k points, whatever the number of
+ * whose row sums exceed that (more than about 5,200 rows at 401 k points, whatever the number of
  * paths) is rejected with FG_ERR_VALUE (split it by rows).  It allocates
  * nothing: no cudaMalloc, no cudaFree, no allocating library call.  The first call with a given stage looks up the
  * array's device address with the stage's device current and keeps it in the stage; make that first call before any

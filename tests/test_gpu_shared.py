@@ -1,0 +1,122 @@
+"""The shared-matrix form of the fused stage and of the drop-in signal (csrc/fg_shared.cuh) against the one-kernel form,
+which a call given only the head and the row sums as workspace (fg_chi_reduce) or none (fg_cchi) takes: the same
+operations in the same order per value, so the tolerances are a few roundings of one value (FP32 1e-6 and FP64 1e-13 of
+the largest), over leg counts 2..9, revisits, sizes around the small-call rule, two sub-batches, and lists without any
+equal scatterers."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from tests.fixtures import phase
+
+pytestmark = pytest.mark.gpu
+DTYPES = [torch.complex64, torch.complex128]
+TOL = {torch.complex64: 1e-6, torch.complex128: 1e-13}
+
+
+def _list(nph, counts, atoms, seed=0):
+    """Paths over few atoms (their scatterers repeat) as PathBatch groups; consecutive atoms differ, revisits allowed."""
+    rng = np.random.default_rng(seed)
+    pts = np.concatenate([np.zeros((1, 3)), rng.uniform(-4.0, 4.0, (atoms, 3))])
+    pot = np.concatenate([[0], rng.integers(1, nph + 1, atoms)])
+    groups = []
+    for nleg, B in counts.items():
+        seq = np.zeros((B, nleg), int)
+        for j in range(1, nleg):
+            last = j == nleg - 1
+            lo = 1 if j == 1 or last else 0
+            pick = rng.integers(lo, atoms + 1, B)
+            while (bad := (pick == seq[:, j - 1])).any():
+                pick[bad] = rng.integers(lo, atoms + 1, int(bad.sum()))
+            seq[:, j] = pick
+        groups.append((pts[seq], pot[seq], rng.uniform(1, 3, B), rng.integers(0, 3, B)))
+    return groups
+
+
+def _rows(st, b, q, S, shared, words=False):
+    from feffgpu_b200 import _lib
+    span = st._span(S)
+    ps = st._paths_struct(b, b.coords, None)
+    NK = int(q.shape[0])
+    full = int(st._lib.fg_chi_reduce_workspace(st._h, C.byref(ps), NK))
+    least = 256 + (16 * b.nrows * NK + 255) // 256 * 256
+    ws = torch.empty(full if shared else least, dtype=torch.uint8, device="cuda")
+    rows = torch.empty(b.nrows, NK, dtype=torch.float64, device="cuda")
+    cc = torch.empty(b.n, st.E, dtype=st.cdtype, device="cuda")
+    rf = torch.empty(b.n, dtype=torch.float64, device="cuda")
+    _lib.check(st._lib.fg_chi_reduce(st._h, st.prec, C.byref(ps), NK, q.data_ptr(), S.data_ptr(), span.data_ptr(),
+                                     rows.data_ptr(), cc.data_ptr(), rf.data_ptr(), ws.data_ptr(), ws.numel(),
+                                     torch.cuda.current_stream().cuda_stream))
+    return rows, cc, rf, full > least
+
+
+def _same(a, b, tol):
+    assert torch.isfinite(torch.view_as_real(b) if b.is_complex() else b).all()
+    assert (a - b).abs().max() <= tol * b.abs().max()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", ["cfg2_phase", "case_A014", "case_A009"])
+@pytest.mark.parametrize("nk", [0, 161])
+@pytest.mark.parametrize("counts", [{4: 1}, {2: 7, 3: 33, 4: 5}, {9: 40, 8: 3, 2: 1}, {6: 3000, 5: 2000, 3: 11}],
+                         ids=["one", "few", "long", "many"])
+def test_shared_form_equals_one_kernel_form(dtype, case, nk, counts):
+    from feffgpu_b200 import GPUPathStage, PathBatch
+    from feffgpu_b200.pad import resample_phase
+    P = resample_phase(phase(case), np.linspace(0.0, 20.0, nk)) if nk else phase(case)
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    b = PathBatch(_list(P.nph, counts, 7), nrows=3, device="cuda")
+    q = torch.arange(1, 402, dtype=torch.float64, device="cuda") * 0.05
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    got, cc, rf, offered = _rows(st, b, q, S, True)
+    ref, cr, rr, _ = _rows(st, b, q, S, False)
+    assert offered == (nk > 0 or (b.n < 4000 and st.ilinit > 1))       # share_plan's rule at 2, 3 and 6 chunks
+    _same(cc, cr, TOL[dtype])
+    _same(got, ref, TOL[dtype])
+    assert torch.equal(rf, rr)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_shared_form_over_two_sub_batches_and_without_sharing(dtype):
+    """More paths than one sub-batch holds (2^18); and as many paths with no two scatterers alike, which the call leaves
+    to the one-kernel form after it has counted them."""
+    from feffgpu_b200 import GPUPathStage, PathBatch
+    P = phase("case_A014")
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    q = torch.arange(1, 21, dtype=torch.float64, device="cuda")
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    groups = _list(P.nph, {4: (1 << 18) - 3, 3: 9, 2: 4}, 6, seed=1)
+    b = PathBatch(groups, nrows=3, device="cuda")
+    got, cc, _, offered = _rows(st, b, q, S, True)
+    ref, cr, _, _ = _rows(st, b, q, S, False)
+    assert offered
+    _same(cc, cr, TOL[dtype])
+    _same(got, ref, TOL[dtype])
+    rng = np.random.default_rng(2)
+    own = [(c + np.where(np.arange(c.shape[1])[None, :, None] > 0, rng.normal(0, 0.05, c.shape), 0.0), i, d, r)
+           for c, i, d, r in ((c[:9000], i[:9000], d[:9000], r[:9000]) for c, i, d, r in groups)]
+    b = PathBatch(own, nrows=3, device="cuda")
+    got, cc, _, _ = _rows(st, b, q, S, True)
+    ref, cr, _, _ = _rows(st, b, q, S, False)
+    _same(cc, cr, TOL[dtype])
+    _same(got, ref, TOL[dtype])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nleg,B", [(2, 5), (3, 1), (4, 700), (7, 9000), (9, 31)])
+def test_drop_in_signal_with_and_without_scratch(dtype, nleg, B):
+    from feffgpu_b200 import GPUPathStage, _lib
+    P = phase("case_A014")
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    c, ip, _, _ = _list(P.nph, {nleg: B}, 6, seed=3)[0]
+    c = torch.tensor(c, device="cuda", dtype=st.rdtype)
+    ip = torch.tensor(ip, device="cuda")
+    got, rf = st.cchi(c, ip)
+    ref = torch.empty_like(got)
+    rr = torch.empty_like(rf)
+    _lib.check(st._lib.fg_cchi(st._h, st.prec, B, nleg, c.data_ptr(), int(dtype == torch.complex128), ip.data_ptr(),
+                               ref.data_ptr(), rr.data_ptr(), None, torch.cuda.current_stream().cuda_stream))
+    _same(got, ref, TOL[dtype])
+    assert torch.equal(rf, rr)

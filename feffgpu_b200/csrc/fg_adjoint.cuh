@@ -18,11 +18,60 @@
 #pragma once
 #include <type_traits>
 
-#include "fg_shared.cuh"
+#include "fg_share.h"
 
 namespace fg {
 
 // ------------------------------------------------------------------------------------------------ setup
+// Canonical entry r of one scatterer's rotation table D(beta) and of d/dbeta D: columns r of out and outd.
+template <typename R>
+__device__ __forceinline__ void rotation_column_adj(R *out, R *outd, const Tables<R> &T, double b, int MM, int DS, int r)
+{
+    const int L1 = T.L1;
+    int m1, m2;
+    canon_mn(MM, r, m1, m2);
+    const double c = cos(b), s = sin(b), c2 = cos(0.5 * b), s2 = sin(0.5 * b);
+    out += r;
+    outd += r;
+    const double *xf = T.xfac + (m1 + 3) * 7 + (m2 + 3);
+    double dm1 = 0.0, d0 = 0.0, em1 = 0.0, e0 = 0.0;   // d and d/dbeta at l-2, l-1
+    const int lseed = min(L1, 4);
+    for (int l = 0; l < lseed; ++l) {             // l <= 3: Wigner's explicit sum
+        const double dl = wigner_small(l, m1, m2, c2, s2, seed_table(T));
+        const double el = wigner_small_dbeta(l, m1, m2, c2, s2, seed_table(T));
+        const double x = xf[(size_t)(l + 1) * 49];
+        out[(size_t)(l + 1) * DS] = (R)(dl * x);
+        outd[(size_t)(l + 1) * DS] = (R)(el * x);
+        dm1 = d0; d0 = dl;
+        em1 = e0; e0 = el;
+    }
+    // the three-term recursion, unrolled so that the coefficient loads issue ahead of the dependent steps
+#pragma unroll 4
+    for (int l = lseed; l < L1; ++l) {
+        const double *q = T.rc + (((size_t)(l - 1) * 7 + (m1 + 3)) * 7 + (m2 + 3)) * 3;
+        const double f = fma(q[0], c, -q[1]);
+        const double dl = fma(f, d0, -q[2] * dm1);
+        const double el = fma(f, e0, fma(-q[0] * s, d0, -q[2] * em1));
+        const double x = xf[(size_t)(l + 1) * 49];
+        out[(size_t)(l + 1) * DS] = (R)(dl * x);
+        outd[(size_t)(l + 1) * DS] = (R)(el * x);
+        dm1 = d0; d0 = dl;
+        em1 = e0; e0 = el;
+    }
+}
+
+// d/dbeta of the termination's rotation matrices d^{l_t}(beta_nleg)
+template <typename R>
+__device__ __forceinline__ void term_dbeta(const WarpPath<R> &g, R (*dterm_db)[49], const Tables<R> &T, int nleg, int lane)
+{
+    for (int task = lane; task < T.nterm * 49; task += 32) {
+        const int t = task / 49, m1 = (task % 49) / 7 - 3, m2 = task % 7 - 3;
+        const double b = g.beta[nleg];
+        dterm_db[t][task % 49] = (R)wigner_small_dbeta(T.term_l[t], m1, m2, cos(0.5 * b), sin(0.5 * b),
+                                                        seed_table(T));
+    }
+}
+
 // Rotation tables D^(k) and their derivatives d/dbeta D^(k) for k = 1..nsc (one recursion for both; path_setup
 // then skips its own pass) and the termination's d/dbeta d^{l_t}(beta_nleg).
 template <typename R>
@@ -32,45 +81,10 @@ __device__ void adj_setup(const WarpPath<R> &g, R *dh, R *dhd, R (*dterm_db)[49]
     const int nsc = nleg - 1;
     const int NC = ncanon(MM), DS = dstride(MM), L1 = T.L1;
     for (int task = lane; task < nsc * NC; task += 32) {
-        const int k = task / NC + 1, r = task % NC;
-        int m1, m2;
-        canon_mn(MM, r, m1, m2);
-        const double b = g.beta[k];
-        const double c = cos(b), s = sin(b), c2 = cos(0.5 * b), s2 = sin(0.5 * b);
-        const size_t o = (size_t)(k - 1) * (L1 + 1) * DS + r;
-        R *out = dh + o, *outd = dhd + o;
-        const double *xf = T.xfac + (m1 + 3) * 7 + (m2 + 3);
-        double dm1 = 0.0, d0 = 0.0, em1 = 0.0, e0 = 0.0;   // d and d/dbeta at l-2, l-1
-        const int lseed = min(L1, 4);
-        for (int l = 0; l < lseed; ++l) {             // l <= 3: Wigner's explicit sum
-            const double dl = wigner_small(l, m1, m2, c2, s2, seed_table(T));
-            const double el = wigner_small_dbeta(l, m1, m2, c2, s2, seed_table(T));
-            const double x = xf[(size_t)(l + 1) * 49];
-            out[(size_t)(l + 1) * DS] = (R)(dl * x);
-            outd[(size_t)(l + 1) * DS] = (R)(el * x);
-            dm1 = d0; d0 = dl;
-            em1 = e0; e0 = el;
-        }
-        // the three-term recursion, unrolled so that the coefficient loads issue ahead of the dependent steps
-#pragma unroll 4
-        for (int l = lseed; l < L1; ++l) {
-            const double *q = T.rc + (((size_t)(l - 1) * 7 + (m1 + 3)) * 7 + (m2 + 3)) * 3;
-            const double f = fma(q[0], c, -q[1]);
-            const double dl = fma(f, d0, -q[2] * dm1);
-            const double el = fma(f, e0, fma(-q[0] * s, d0, -q[2] * em1));
-            const double x = xf[(size_t)(l + 1) * 49];
-            out[(size_t)(l + 1) * DS] = (R)(dl * x);
-            outd[(size_t)(l + 1) * DS] = (R)(el * x);
-            dm1 = d0; d0 = dl;
-            em1 = e0; e0 = el;
-        }
+        const size_t o = (size_t)(task / NC) * (L1 + 1) * DS;
+        rotation_column_adj<R>(dh + o, dhd + o, T, g.beta[task / NC + 1], MM, DS, task % NC);
     }
-    for (int task = lane; task < T.nterm * 49; task += 32) {
-        const int t = task / 49, m1 = (task % 49) / 7 - 3, m2 = task % 7 - 3;
-        const double b = g.beta[nleg];
-        dterm_db[t][task % 49] = (R)wigner_small_dbeta(T.term_l[t], m1, m2, cos(0.5 * b), sin(0.5 * b),
-                                                        seed_table(T));
-    }
+    term_dbeta<R>(g, dterm_db, T, nleg, lane);
 }
 
 // ------------------------------------------------------------------------------------------------ termination
@@ -990,11 +1004,12 @@ __global__ void __launch_bounds__(128) k_adjoint(Tables<R> T, const CT *__restri
                                                   const double *__restrict__ greff_d, const R *__restrict__ greff_r,
                                                   R *__restrict__ gout_r, double *__restrict__ gout_d,
                                                   unsigned long long *counter, int *status, int nsc_max, size_t wbytes,
-                                                  double *__restrict__ gpar_out)
+                                                  double *__restrict__ gpar_out, const int *gate)
 {
     using K = Kinds<EDGE>;
     extern __shared__ __align__(16) unsigned char smem[];
     if (*(volatile const int *)status & kBadLayout) return;     // a batch that k_validate refused
+    if (gate && !*(volatile const int *)gate) return;           // the shared-matrix form took the call
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int E = T.E, L1 = T.L1;
     unsigned char *base = smem + (size_t)w * wbytes;
@@ -1072,17 +1087,19 @@ __global__ void __launch_bounds__(128) k_adjoint(Tables<R> T, const CT *__restri
 template <typename CT>
 __global__ void __launch_bounds__(128) k_coord_grad(const CT *__restrict__ coords, int stride,
                                                      const int *__restrict__ nlegs, int nleg_uniform, int64_t B,
-                                                     const double *__restrict__ gpar, double *__restrict__ gout,
-                                                     const int *status)
+                                                     const int *__restrict__ order, const double *__restrict__ gpar,
+                                                     double *__restrict__ gout, const int *status, const int *gate)
 {
     __shared__ double s_xyz[4][kMaxLeg][3], s_gpar[4][3 * (kMaxLeg + 1)], s_cg[4][9 * kMaxLeg];
     if (*(volatile const int *)status & kBadLayout) return;     // a batch that k_validate refused
+    if (gate && !*(volatile const int *)gate) return;           // the shared-matrix form took the call
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int64_t p = (int64_t)blockIdx.x * 4 + w; p < B; p += (int64_t)gridDim.x * 4) {
+    for (int64_t i = (int64_t)blockIdx.x * 4 + w; i < B; i += (int64_t)gridDim.x * 4) {
+        const int64_t p = order ? order[i] : i;
         const int nleg = nlegs ? nlegs[p] : nleg_uniform;
         const double *gp = gpar + p * kGparStride;
-        for (int i = lane; i < nleg * 3; i += 32) s_xyz[w][i / 3][i % 3] = (double)coords[p * stride * 3 + i] / kBohr;
-        for (int i = lane; i < 3 * (kMaxLeg + 1); i += 32) s_gpar[w][i] = gp[i];
+        for (int t = lane; t < nleg * 3; t += 32) s_xyz[w][t / 3][t % 3] = (double)coords[p * stride * 3 + t] / kBohr;
+        for (int t = lane; t < 3 * (kMaxLeg + 1); t += 32) s_gpar[w][t] = gp[t];
         const int frame = (int)gp[3 * (kMaxLeg + 1)];
         __syncwarp();
         if (frame) {
@@ -1204,7 +1221,7 @@ fg_status launch_adjoint(const StageView &sv, const Tables<R> &T, const CT *coor
                          const int *nlegs, int nleg_uniform, int nsc_max, int64_t B, const int *order,
                          const C2<R> *gbar, const double *greff_d, const R *greff_r, R *gout_r, double *gout_d,
                          unsigned long long *counter, int *status, int warps, cudaStream_t st,
-                         double *gpar_out = nullptr)
+                         double *gpar_out = nullptr, const int *gate = nullptr)
 {
     using K = Kinds<EDGE>;
     const size_t wb = adj_warp_bytes<R>(sv.L1, nsc_max, K::MM);
@@ -1221,10 +1238,10 @@ fg_status launch_adjoint(const StageView &sv, const Tables<R> &T, const CT *coor
         }
     int blocks = 0;
     if (fg_status rc = grid_for(kern, threads, wb * warps, sv.num_sms, B, blocks)) return rc;
-    timer_begin(st);
+    if (!gate) timer_begin(st);
     kern<<<blocks, threads, wb * warps, st>>>(T, coords, ipots, stride, nlegs, nleg_uniform, B, order, gbar, greff_d,
-                                              greff_r, gout_r, gout_d, counter, status, nsc_max, wb, gpar_out);
-    timer_end(st);
+                                              greff_r, gout_r, gout_d, counter, status, nsc_max, wb, gpar_out, gate);
+    if (!gate) timer_end(st);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
@@ -1248,31 +1265,67 @@ fg_status launch_fine_adjoint(const StageView &sv, int64_t B, int NK, int mode, 
     return FG_OK;
 }
 
-template <typename R, int EDGE>
-fg_status Launch<R, EDGE>::cchi_bwd(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const void *coords,
-                                    int coords_f64, const int64_t *ipots, const void *grad_cchi, const void *grad_reff,
-                                    void *grad_coords, unsigned char *ws, int warps, cudaStream_t st)
+template <typename R, int EDGE, typename CT>
+fg_status cchi_bwd_call(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const CT *coords,
+                        const int64_t *ipots, const C2<R> *gb, const R *gr, R *out, unsigned char *ws, size_t ws_bytes,
+                        int warps, cudaStream_t st)
 {
     unsigned long long *counter = reinterpret_cast<unsigned long long *>(ws);
     int *status = reinterpret_cast<int *>(ws + kStatusOffset);
+    FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes, st));
+    if constexpr (EDGE <= 3) {
+        const SharePlan pl = share_plan(B, nleg, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit, true);
+        if (pl.sub && ws_bytes >= kCounterBytes + pl.total) {
+            unsigned char *sw = ws + kCounterBytes;
+            ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
+            Share<R> s = share_view<R, EDGE>(pl, sw, head, status, sv.L1);
+            s.stride = s.nleg_uniform = nleg;
+            for (int64_t t0 = 0; t0 < B; t0 += pl.sub) {
+                s.n = std::min<int64_t>(pl.sub, B - t0);
+                const CT *c = coords + t0 * nleg * 3;
+                const int64_t *ip = ipots + t0 * nleg;
+                const C2<R> *gt = gb + t0 * sv.E;
+                const R *grt = gr ? gr + t0 : nullptr;
+                R *ot = out + t0 * nleg * 3;
+                if (fg_status rc = ShareLaunch<R, EDGE>::template adjoint<CT>(sv, T, pl, s, sw, c, ip, status, gt, nullptr, grt, nullptr,
+                                                              ot, st))
+                    return rc;
+                if (!pl.force) {
+                    if (t0) FG_CUDA(cudaMemsetAsync(counter, 0, sizeof(*counter), st));
+                    if (fg_status rc = launch_adjoint<R, EDGE, CT>(sv, T, c, ip, nleg, nullptr, nleg, nleg - 1, s.n, nullptr,
+                                                                   gt, nullptr, grt, ot, nullptr, counter, status, warps,
+                                                                   st, nullptr, &head->general))
+                        return rc;
+                }
+            }
+            return FG_OK;
+        }
+    }
+    return launch_adjoint<R, EDGE, CT>(sv, T, coords, ipots, nleg, nullptr, nleg, nleg - 1, B, nullptr, gb, nullptr, gr, out,
+                                       nullptr, counter, status, warps, st);
+}
+
+template <typename R, int EDGE>
+fg_status Launch<R, EDGE>::cchi_bwd(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const void *coords,
+                                    int coords_f64, const int64_t *ipots, const void *grad_cchi, const void *grad_reff,
+                                    void *grad_coords, unsigned char *ws, size_t ws_bytes, int warps, cudaStream_t st)
+{
     const C2<R> *gb = static_cast<const C2<R> *>(grad_cchi);
     const R *gr = static_cast<const R *>(grad_reff);
-    FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes, st));
+    R *out = static_cast<R *>(grad_coords);
     if (coords_f64)
-        return launch_adjoint<R, EDGE, double>(sv, T, static_cast<const double *>(coords), ipots, nleg, nullptr, nleg,
-                                               nleg - 1, B, nullptr, gb, nullptr, gr, static_cast<R *>(grad_coords),
-                                               nullptr, counter, status, warps, st);
-    return launch_adjoint<R, EDGE, float>(sv, T, static_cast<const float *>(coords), ipots, nleg, nullptr, nleg,
-                                          nleg - 1, B, nullptr, gb, nullptr, gr, static_cast<R *>(grad_coords),
-                                          nullptr, counter, status, warps, st);
+        return cchi_bwd_call<R, EDGE>(sv, T, B, nleg, static_cast<const double *>(coords), ipots, gb, gr, out, ws, ws_bytes,
+                                      warps, st);
+    return cchi_bwd_call<R, EDGE>(sv, T, B, nleg, static_cast<const float *>(coords), ipots, gb, gr, out, ws, ws_bytes,
+                                  warps, st);
 }
 
 template <typename R, int EDGE>
 fg_status Launch<R, EDGE>::fused_bwd(const StageView &sv, const Tables<R> &T, const fg_paths *P, int NK,
                                      const double *q, const double *S, const int *span, const int *tspan,
                                      const double *grad_rows, const void *cchi_saved, const double *reff_saved,
-                                     double *grad_coords, double *grad_sigma2, unsigned char *ws, int warps,
-                                     cudaStream_t st)
+                                     double *grad_coords, double *grad_sigma2, unsigned char *ws,
+                                     size_t ws_bytes, int warps, cudaStream_t st)
 {
     unsigned long long *counter = reinterpret_cast<unsigned long long *>(ws);
     int *status = reinterpret_cast<int *>(ws + kStatusOffset);
@@ -1287,14 +1340,39 @@ fg_status Launch<R, EDGE>::fused_bwd(const StageView &sv, const Tables<R> &T, co
                                               span, tspan, nullptr, grad_rows, P->row, P->deg, P->sigma2,
                                               gbar, nullptr, greff, grad_sigma2, status, st))
         return rc;
-    if (fg_status rc = launch_adjoint<R, EDGE, double>(sv, T, P->coords, P->ipots, P->nleg_max, P->nleg, 0,
-                                                       P->nleg_max - 1, P->n, P->order, gbar, greff, nullptr, nullptr,
-                                                       grad_coords, counter, status, warps, st, gpar))
-        return rc;
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((P->n + 3) / 4, (int64_t)sv.num_sms * 16));
-    k_coord_grad<double><<<blocks, 128, 0, st>>>(P->coords, P->nleg_max, P->nleg, 0, P->n, gpar, grad_coords, status);
-    FG_CUDA(cudaGetLastError());
-    return FG_OK;
+    // the paths of order[t0 ..] in the one-kernel form (gate: only where the shared form left them)
+    auto general = [&](int64_t t0, int64_t n, const int *gate) -> fg_status {
+        if (t0) FG_CUDA(cudaMemsetAsync(counter, 0, sizeof(*counter), st));
+        if (fg_status rc = launch_adjoint<R, EDGE, double>(sv, T, P->coords, P->ipots, P->nleg_max, P->nleg, 0,
+                                                           P->nleg_max - 1, n, P->order + t0, gbar, greff, nullptr, nullptr,
+                                                           grad_coords, counter, status, warps, st, gpar, gate))
+            return rc;
+        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 3) / 4, (int64_t)sv.num_sms * 16));
+        k_coord_grad<double><<<blocks, 128, 0, st>>>(P->coords, P->nleg_max, P->nleg, 0, n, P->order + t0, gpar,
+                                                     grad_coords, status, gate);
+        FG_CUDA(cudaGetLastError());
+        return FG_OK;
+    };
+    const size_t used = fused_bwd_workspace(P, NK, sv.E);
+    const SharePlan pl = share_plan(P->n, P->nleg_max, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit, true);
+    if constexpr (EDGE <= 3)
+        if (pl.sub && ws_bytes >= used + pl.total) {
+            ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
+            Share<R> s = share_view<R, EDGE>(pl, ws + used, head, status, sv.L1);
+            s.stride = P->nleg_max;
+            s.nlegs = P->nleg;
+            for (int64_t t0 = 0; t0 < P->n; t0 += pl.sub) {
+                s.n = std::min<int64_t>(pl.sub, P->n - t0);
+                s.order = P->order + t0;
+                if (fg_status rc = ShareLaunch<R, EDGE>::template adjoint<double>(sv, T, pl, s, ws + used, P->coords, P->ipots, status, gbar,
+                                                                  greff, nullptr, grad_coords, nullptr, st))
+                    return rc;
+                if (!pl.force)
+                    if (fg_status rc = general(t0, s.n, &head->general)) return rc;
+            }
+            return FG_OK;
+        }
+    return general(0, P->n, nullptr);
 }
 
 template <typename R>

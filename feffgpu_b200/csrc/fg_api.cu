@@ -435,10 +435,10 @@ template <class F> fg_status by_kind(const fg_stage *s, fg_precision prec, F &&f
 }
 
 // Bytes of the shared form's workspace in the larger of the two precisions (0 where it does not apply)
-size_t share_bytes(const fg_stage *s, int64_t n, int nleg_max)
+size_t share_bytes(const fg_stage *s, int64_t n, int nleg_max, bool adjoint = false)
 {
-    return std::max(share_plan(n, nleg_max, s->E, s->L1, false, s->iorder, s->ilinit).total,
-                    share_plan(n, nleg_max, s->E, s->L1, true, s->iorder, s->ilinit).total);
+    return std::max(share_plan(n, nleg_max, s->E, s->L1, false, s->iorder, s->ilinit, adjoint).total,
+                    share_plan(n, nleg_max, s->E, s->L1, true, s->iorder, s->ilinit, adjoint).total);
 }
 
 // Host-side checks of a batch's sizes and pointers; k_validate checks the contents (indices) on the device and
@@ -493,7 +493,7 @@ extern "C" fg_status fg_cchi(const fg_stage *s, fg_precision prec, int64_t B, in
 extern "C" size_t fg_cchi_backward_workspace(const fg_stage *s, int64_t B, int32_t nleg)
 {
     if (!s || B < 0 || nleg < 2 || nleg > kMaxLeg) return 0;
-    return cchi_bwd_workspace(B, nleg);
+    return cchi_bwd_workspace(B, nleg) + share_bytes(s, B, nleg, true);
 }
 
 extern "C" fg_status fg_cchi_backward(const fg_stage *s, fg_precision prec, int64_t B, int32_t nleg,
@@ -515,7 +515,7 @@ extern "C" fg_status fg_cchi_backward(const fg_stage *s, fg_precision prec, int6
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return by_kind(s, prec, [&](auto L, const auto &T) {
         return decltype(L)::cchi_bwd(sv, T, B, nleg, coords, coords_f64, ipots, grad_cchi, grad_reff, grad_coords,
-                                     static_cast<unsigned char *>(workspace), bwd_warps(s), st);
+                                     static_cast<unsigned char *>(workspace), workspace_bytes, bwd_warps(s), st);
     });
 }
 
@@ -626,7 +626,7 @@ extern "C" fg_status fg_rows_from_words(int64_t nrows, int32_t NK, const uint64_
 extern "C" size_t fg_chi_reduce_backward_workspace(const fg_stage *s, const fg_paths *P, int32_t NK)
 {
     if (!s || !P || NK < 0) return 0;
-    return fused_bwd_workspace(P, NK, s->E);
+    return fused_bwd_workspace(P, NK, s->E) + share_bytes(s, P->n, P->nleg_max, true);
 }
 
 extern "C" fg_status fg_chi_reduce_backward(const fg_stage *s, fg_precision prec, const fg_paths *P, int32_t NK,
@@ -651,7 +651,7 @@ extern "C" fg_status fg_chi_reduce_backward(const fg_stage *s, fg_precision prec
     if (fg_status rc = by_kind(s, prec, [&](auto L, const auto &T) {
             return decltype(L)::fused_bwd(sv, T, P, NK, q, S, span, tspan, grad_rows, cchi_saved, reff_saved,
                                           grad_coords, grad_sigma2, static_cast<unsigned char *>(workspace),
-                                          bwd_warps(s), st);
+                                          workspace_bytes, bwd_warps(s), st);
         }))
         return rc;
     return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st);

@@ -26,6 +26,12 @@ template <typename R> struct WarpPath {
     R dterm[2][49];                // d^{l_t}_{m1 m2}(beta_nleg), [m1+3][m2+3]
 };
 
+// What the adjoint's record of a path adds: d/dbeta of dterm and the frame it is differentiated in.
+template <typename R> struct AdjExtra {
+    R dterm_db[2][49];
+    int frame;
+};
+
 template <typename R, int MM> __host__ __device__ constexpr size_t dh_floats(int L1, int nsc)
 {
     return (size_t)nsc * (L1 + 1) * dstride(MM);

@@ -55,12 +55,12 @@ template <typename R, int EDGE> struct Launch {
                            size_t share_bytes = 0);
     static fg_status cchi_bwd(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const void *coords,
                               int coords_f64, const int64_t *ipots, const void *grad_cchi, const void *grad_reff,
-                              void *grad_coords, unsigned char *ws, int warps, cudaStream_t st);
+                              void *grad_coords, unsigned char *ws, size_t ws_bytes, int warps, cudaStream_t st);
     static fg_status fused_bwd(const StageView &sv, const Tables<R> &T, const fg_paths *P, int NK, const double *q,
                                const double *S, const int *span, const int *tspan, const double *grad_rows,
                                const void *cchi_saved,
                                const double *reff_saved, double *grad_coords, double *grad_sigma2, unsigned char *ws,
-                               int warps, cudaStream_t st);
+                               size_t ws_bytes, int warps, cudaStream_t st);
 };
 
 // Precision-only launches (no lambda-set dependence).
@@ -118,6 +118,7 @@ fg_status describe_paths_warp(int64_t B, int32_t nleg, const int32_t *seq, const
 // ---- the path signal with shared scattering matrices (fg_shared.cuh) -------------------------------------------------
 struct __align__(16) ShareKey { unsigned long long x, y, z, w; };   // leg, next leg, beta (FP64 bits), potential
 constexpr int kShareMin = 2;                               // least scatterers per class that make the form worth taking
+constexpr int64_t kShareItems = 1 << 16;                   // (path, part of its energies) items that fill the chip
 constexpr int64_t kShareSub = 1 << 18;                     // paths per sub-batch (bounds the workspace)
 constexpr int64_t kShareWorth = 1 << 15;                   // (path, 32 energies) items worth looking for classes
 constexpr int64_t kShareSmall = 8192;                      // (path, 32 energies) items of a small call
@@ -152,12 +153,14 @@ fg_status launch_share_insert(const ShareIdx &s, cudaStream_t st);
 // sub-batch (0: the form does not apply).
 struct SharePlan {
     int64_t sub = 0, cls_cap = 0;
-    int nsc_max = 0, chunks = 0, passes = 0, split = 1, force = 0;
+    int nsc_max = 0, chunks = 0, passes = 0, split = 1, force = 0, mats = 1;
     unsigned hcap = 0;
     size_t rec = 0, key = 0, slot = 0, hash = 0, cls = 0, owner = 0, two = 0, tab = 0, F = 0, f_bytes = 0, sig = 0,
-           total = 0;
+           gpar = 0, total = 0;
 };
-SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit);
+// adjoint: the plan of the backward calls (a class keeps its matrix and three derivatives, paths their parameter
+// gradients instead of signals)
+SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit, bool adjoint = false);
 
 // Events around the main kernel of a call when kernel timing is on (fg_set_kernel_timing)
 void timer_begin(cudaStream_t st);

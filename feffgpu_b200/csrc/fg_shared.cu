@@ -54,16 +54,17 @@ fg_status launch_share_insert(const ShareIdx &s, cudaStream_t st)
     return FG_OK;
 }
 
-SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit)
+SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit, bool adjoint)
 {
     SharePlan p;
     if (iorder > 2 || n < 1) return p;
     // Lists of up to three legs share nothing (every scatterer has the absorber on one side and the path's only other
     // atom on the other), so they take this form only where few paths leave the chip idle and it spreads their energies
     // over warps: many energies, or the fifteen-column single scattering of L and M edges (897 paths, L3, 59 energies:
-    // 342 -> 245 us; at the K edge on 60 energies the extra launches cost more than the spreading gains: 421 -> 474 us).
-    // Longer paths take it wherever the call is worth the launches that find the classes (about 40 us): at two chunks
-    // of energies and 4,438 paths of up to four legs, 1.27 scatterers per class, looking for them cost 5 %.
+    // 342 -> 245 us; at the K edge on 60 energies the extra launches cost what the spreading gains: 396 paths forward
+    // 421 -> 474 us, backward of 396 and 4,438 paths 445 -> 472 and 1355 -> 1420 us).  Longer paths take it wherever
+    // the call is worth the launches that find the classes (about 40 us): at two chunks of energies and 4,438 paths of
+    // up to four legs, 1.27 scatterers per class, looking for them cost 5 %.
     const int chunks = (E + 31) / 32;
     const bool small = n * chunks <= kShareSmall && (chunks >= 4 || ilinit > 1);
     if (!small && (nleg_max < 4 || (chunks < 4 && n * chunks <= kShareWorth))) return p;
@@ -72,29 +73,34 @@ SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iord
     p.nsc_max = nleg_max - 1;
     p.chunks = chunks;
     const int64_t scat = p.sub * p.nsc_max;
-    const size_t per = 20 * 2 * real * 32;          // one class, one chunk: 20 canonical entries (orders 0-2)
+    p.mats = adjoint ? 4 : 1;
+    const size_t per = p.mats * 20 * 2 * real * 32;          // one class, one chunk: 20 canonical entries (orders 0-2)
     const size_t all = (size_t)scat * p.chunks * per;
-    p.f_bytes = std::min(all, kShareMatrixBytes);
+    p.f_bytes = std::min(all, adjoint ? 2 * kShareMatrixBytes : kShareMatrixBytes);
     p.cls_cap = std::min<int64_t>(scat, (int64_t)(p.f_bytes / per));
     const int fit = (int)std::min<size_t>(p.chunks, p.f_bytes / ((size_t)scat * per));   // chunks per pass at worst
     p.passes = fit ? (p.chunks + fit - 1) / fit : p.chunks;
     p.force = small && fit == p.chunks;
-    // small calls spread a path's energies over warps; large ones load its record once per pass
-    p.split = p.sub < 148 * 12 ? chunks : 1;
+    // a path's energies are spread over warps until the items fill the chip many times over (10,007 paths x 13 chunks,
+    // backward: k_share_chain_adj 4.0 ms unsplit, the last of its six waves nearly empty)
+    p.split = (int)std::min<int64_t>(chunks, (kShareItems + p.sub - 1) / p.sub);
     p.hcap = 64;
     while ((int64_t)p.hcap < 2 * scat) p.hcap *= 2;
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += align_up(bytes, 256); return o; };
-    p.rec = take((size_t)p.sub * align_up(fp64 ? sizeof(WarpPath<double>) : sizeof(WarpPath<float>), 16));
+    const size_t rec = align_up(fp64 ? sizeof(WarpPath<double>) : sizeof(WarpPath<float>), 16);
+    const size_t ext = align_up(fp64 ? sizeof(AdjExtra<double>) : sizeof(AdjExtra<float>), 16);
+    p.rec = take((size_t)p.sub * (adjoint ? rec + ext : rec));
     p.key = take((size_t)scat * sizeof(ShareKey));
     p.slot = take((size_t)scat * 4);
     p.hash = take((size_t)p.hcap * 4);
     p.cls = take((size_t)p.hcap * 4);
     p.owner = take((size_t)p.cls_cap * 4);
     p.two = take((size_t)p.sub * 4);
-    p.tab = take((size_t)p.cls_cap * (L1 + 1) * dstride(2) * real);
+    p.tab = take((size_t)p.cls_cap * (L1 + 1) * dstride(2) * real * (adjoint ? 2 : 1));
     p.F = take(p.f_bytes);
-    p.sig = take((size_t)p.sub * E * 2 * real);
+    if (adjoint) p.gpar = take((size_t)p.split * p.sub * kGparStride * sizeof(double));
+    else p.sig = take((size_t)p.sub * E * 2 * real);
     p.total = at;
     return p;
 }

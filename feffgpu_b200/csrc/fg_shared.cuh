@@ -9,7 +9,7 @@
 //   k_share_geom    a warp per path: geometry, Euler phases, termination rotations (the path's record), the keys
 //   k_share_insert  a thread per scatterer: classes from a hash table of the keys (exact comparison)
 //   k_share_tables  a thread per (class, rotation-table entry): D of every class
-//   k_share_f       a warp per (class, 32 energies): the canonical entries of F~; two-leg paths' signals beside them
+//   k_share_f       a warp per (class, 32 energies): F~ in its two flip blocks; two-leg paths' signals beside them
 //   k_share_chain   a warp per (path, 32 energies): chain product, termination, cfac
 //   k_share_fine    a warp per path (fused calls): fine grid and exact row sums
 //
@@ -21,25 +21,9 @@
 // of up to seven legs, FP64 form 14.3 -> 5.65 ms.  What bounds it: the chain product's 144 complex multiply-adds per
 // scatterer and energy and the 160 bytes (FP32) of matrix it reads for them, 4.3 TB/s from L2 and HBM.
 #pragma once
-#include "fg_kernels.cuh"
+#include "fg_adjoint.cuh"
 
 namespace fg {
-
-// The workspace as the kernels of one sub-batch see it.
-template <typename R> struct Share : ShareIdx {
-    unsigned char *rec;          // n records of rec_bytes (WarpPath<R>)
-    size_t rec_bytes;
-    int *two;                    // two-leg paths of the sub-batch (at most n)
-    R *tab;                      // cls_cap rotation tables of tab_len entries
-    int tab_len;
-    unsigned char *F;            // the matrices: f_bytes
-    size_t f_bytes;
-    int chunks;                  // chunks of 32 energies
-    int force;                   // this form is taken whatever the sharing (small calls)
-    int by_path;                 // signals are stored by path (else by position in the sub-batch)
-    __device__ __forceinline__ int64_t path(int64_t i) const { return order ? order[i] : i; }
-    __device__ __forceinline__ int64_t row(int64_t i) const { return by_path ? path(i) : i; }
-};
 
 // bytes of one class's matrices over one chunk
 template <typename R, int KIND> __host__ __device__ constexpr size_t f_chunk_bytes()
@@ -54,11 +38,11 @@ template <typename R, int KIND> __device__ __forceinline__ int share_chunks(cons
 {
     const int64_t U = s.head->classes, S = s.head->scatterers;
     if (U > s.cls_cap || (!s.force && U * kShareMin > S)) return 0;
-    const size_t per = (size_t)max(U, (int64_t)1) * f_chunk_bytes<R, KIND>();
+    const size_t per = (size_t)max(U, (int64_t)1) * s.mats * f_chunk_bytes<R, KIND>();
     return (int)min((size_t)s.chunks, s.f_bytes / per);
 }
 
-// A matrix's canonical entries, two complex FP32 (one FP64) per 16-byte word, words lane-contiguous.
+// A matrix's entries, two complex FP32 (one FP64) per 16-byte word, words lane-contiguous.
 template <typename R, int NE> __device__ __forceinline__ void store_f(unsigned char *at, int lane, const C2<R> (&f)[NE])
 {
     if constexpr (sizeof(R) == 4) {
@@ -89,9 +73,167 @@ template <typename R, int NE> __device__ __forceinline__ void load_f(const unsig
     }
 }
 
+// ------------------------------------------------------------------------------------------------ flip basis
+// F~ commutes with the signed flip (S v)_m = (-1)^m v_(-m), so in the basis u_m = v_m + (-1)^m v_(-m) (and v_0 of each
+// n), w_m = v_m - (-1)^m v_(-m) it is two blocks: 4 x 4 over u = (0,0), (0,1), 1, 2 and 2 x 2 over w = 1, 2.  The classes
+// keep the 20 block entries, formed once per class, and a chain step costs 80 complex multiply-adds instead of 144; the
+// Euler phase e^{-i eta m} mixes u_m and w_m by cos and -i sin.  (In k_fused, which forms every matrix in the registers
+// of its chain, the same basis cost more registers than it saved work.)
+template <int KIND> struct Flip {
+    static constexpr LamTab L = lamtab(KIND);
+    static_assert(L.N == 6 && L.MM == 2, "the six-entry sets of orders 0-2");
+    static constexpr int NE0 = L.N0 == 4 ? 3 : 4, NO0 = L.N0 == 4 ? 1 : 2;   // u and w entries within the final state
+    // (m, n) of u entry i; w entry i: m = i + 1
+    static __host__ __device__ constexpr int em(int i) { return i < 2 ? 0 : i - 1; }
+    static __host__ __device__ constexpr int en(int i) { return i == 1; }
+    // position of (m, n) in the lambda set
+    static __host__ __device__ constexpr int at(int m, int n)
+    {
+        const LamTab t = lamtab(KIND);
+        for (int i = 0; i < 6; ++i)
+            if (t.m[i] == m && t.n[i] == n) return i;
+        return 0;
+    }
+};
+
+// The block entries (u block row-major, then w block) from the canonical entries
+template <typename R, int KIND> __device__ __forceinline__ void to_blocks(const C2<R> (&acc)[20], C2<R> (&f)[20])
+{
+    constexpr LamTab L = lamtab(KIND);
+    constexpr RepTab<KIND, L.N, L.N> RT{};
+    using B = Flip<KIND>;
+    auto F = [&](int a, int b) { return RT.sg[a][b] > 0 ? acc[RT.rep[a][b]] : cscl(acc[RT.rep[a][b]], R(-1)); };
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int a = B::at(B::em(i), B::en(i)), b = B::at(B::em(j), B::en(j));
+            C2<R> v = F(a, b);
+            if (B::em(j)) {
+                if (B::em(i)) {
+                    const C2<R> x = F(a, B::at(-B::em(j), 0));
+                    v = (B::em(j) & 1) ? csub(v, x) : cadd(v, x);
+                }
+            } else if (B::em(i)) {
+                v = cscl(v, R(2));
+            }
+            f[4 * i + j] = v;
+        }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int a = B::at(i + 1, 0);
+            const C2<R> v = F(a, B::at(j + 1, 0)), x = F(a, B::at(-j - 1, 0));
+            f[16 + 2 * i + j] = j == 0 ? cadd(v, x) : csub(v, x);
+        }
+}
+
+// (u, w) turned by the Euler phase e^{-i eta m}, given as ph = e^{-i eta m}: (c u - i s w, c w - i s u)
+template <typename R> __device__ __forceinline__ void turn(C2<R> ph, C2<R> &u, C2<R> &w)
+{
+    const R c = ph.x, s = -ph.y;
+    const C2<R> a = u, b = w;
+    u = C2<R>{fma(c, a.x, s * b.y), fma(c, a.y, -s * b.x)};
+    w = C2<R>{fma(c, b.x, s * a.y), fma(c, b.y, -s * a.x)};
+}
+
+// One column (u entries x[0..3], w entries x[4..5]) times the blocks, then the phase; rows: only the first NE0 u and NO0
+// w entries are formed (what the termination reads)
+template <typename R, int KIND>
+__device__ __forceinline__ void block_step(const C2<R> (&f)[20], C2<R> e1, C2<R> e2, bool all, C2<R> (&x)[6])
+{
+    using B = Flip<KIND>;
+    C2<R> y[6];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        y[i] = cz<R>();
+        if (all || i < B::NE0)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[i] = cfma(f[4 * i + j], x[j], y[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        y[4 + i] = cz<R>();
+        if (all || i < B::NO0)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) y[4 + i] = cfma(f[16 + 2 * i + j], x[4 + j], y[4 + i]);
+    }
+    turn(e1, y[2], y[4]);
+    turn(e2, y[3], y[5]);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) x[i] = y[i];
+}
+
+// The first matrix's column c of the N0 (u columns, then w columns): a block column, then the phase
+template <typename R, int KIND>
+__device__ __forceinline__ void block_first(const C2<R> (&f)[20], C2<R> e1, C2<R> e2, int c, C2<R> (&x)[6])
+{
+    using B = Flip<KIND>;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) x[i] = cz<R>();
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (j < B::NE0 && c == j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = f[4 * i + j];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+        if (j < B::NO0 && c == B::NE0 + j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) x[4 + i] = f[16 + 2 * i + j];
+    turn(e1, x[2], x[4]);
+    turn(e2, x[3], x[5]);
+}
+
+// The chain product back in the lambda set's entries, Q[b][a] for a, b < N0, from its columns P(c)[i]
+template <typename R, int KIND, class PF>
+__device__ __forceinline__ void from_blocks(const PF &P, C2<R> (&Q)[lamtab(KIND).N0][lamtab(KIND).N0])
+{
+    constexpr LamTab L = lamtab(KIND);
+    using B = Flip<KIND>;
+#pragma unroll
+    for (int a = 0; a < L.N0; ++a) {
+        const int am = L.m[a] < 0 ? -L.m[a] : L.m[a];
+        // the column of entry a: u_am (+-) w_am
+        C2<R> x[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            if (am == 0) {
+                x[i] = P(L.n[a], i);
+            } else {
+                const C2<R> u = P(am + 1, i), w = P(B::NE0 + am - 1, i);
+                if (L.m[a] > 0) x[i] = cadd(u, w);
+                else x[i] = (am & 1) ? csub(w, u) : csub(u, w);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < L.N0; ++b) {
+            const int bm = L.m[b] < 0 ? -L.m[b] : L.m[b];
+            if (bm == 0) Q[b][a] = x[L.n[b]];
+            else if (L.m[b] > 0) Q[b][a] = cscl(cadd(x[bm + 1], x[3 + bm]), R(0.5));
+            else Q[b][a] = cscl((bm & 1) ? csub(x[3 + bm], x[bm + 1]) : csub(x[bm + 1], x[3 + bm]), R(0.5));
+        }
+    }
+}
+
 __device__ __forceinline__ void copy16(void *dst, const void *src, size_t bytes, int lane)
 {
     for (size_t i = lane; i < bytes / 16; i += 32) static_cast<uint4 *>(dst)[i] = static_cast<const uint4 *>(src)[i];
+}
+
+// The keys of path i's scatterers, or its entry in the list of two-leg paths
+template <typename R>
+__device__ __forceinline__ void share_keys(const Share<R> &s, const WarpPath<R> &g, int64_t i, int nleg, int lane)
+{
+    if (nleg == 2) {
+        if (lane == 0) s.two[atomicAdd(&s.head->two, 1)] = (int)i;
+    } else if (lane >= 1 && lane < nleg) {
+        s.key[i * s.nsc_max + lane - 1] = ShareKey{(unsigned long long)__double_as_longlong(g.ri[lane]),
+                                                   (unsigned long long)__double_as_longlong(g.ri[lane + 1]),
+                                                   (unsigned long long)__double_as_longlong(g.beta[lane]),
+                                                   (unsigned long long)g.ip[lane]};
+    }
 }
 
 // Records, keys and the list of two-leg paths (a batch that k_validate refused is left alone).
@@ -109,16 +251,7 @@ __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, con
         path_setup<R, CT>(g, nullptr, T, coords + p * s.stride * 3, ipots + p * s.stride, nleg, lane, status,
                           nleg == 2 ? MM_ss : MM_ms, false);
         copy16(s.rec + i * s.rec_bytes, &g, s.rec_bytes, lane);
-        if (nleg == 2) {
-            if (lane == 0) s.two[atomicAdd(&s.head->two, 1)] = (int)i;
-        } else if (lane >= 1 && lane < nleg) {
-            ShareKey k;
-            k.x = (unsigned long long)__double_as_longlong(g.ri[lane]);
-            k.y = (unsigned long long)__double_as_longlong(g.ri[lane + 1]);
-            k.z = (unsigned long long)__double_as_longlong(g.beta[lane]);
-            k.w = (unsigned long long)g.ip[lane];
-            s.key[i * s.nsc_max + lane - 1] = k;
-        }
+        share_keys(s, g, i, nleg, lane);
         __syncwarp();
     }
 }
@@ -187,7 +320,9 @@ __global__ void __launch_bounds__(128) k_share_f(Tables<R> T, Share<R> s, int pa
                         zfac(cscl(ck, (R)__longlong_as_double((long long)key.y))),
                         zfac(cscl(ck, (R)__longlong_as_double((long long)key.x))));
                     mask_lambda<R, KIND, L.N, L.N>(acc, T.nlam);
-                    store_f<R, RT.n>(s.F + (c * G + (it - n_two) % ng) * f_chunk_bytes<R, KIND>(), lane, acc);
+                    C2<R> f[20];
+                    to_blocks<R, KIND>(acc, f);
+                    store_f<R, 20>(s.F + (c * G + (it - n_two) % ng) * f_chunk_bytes<R, KIND>(), lane, f);
                 }
             }
         }
@@ -204,8 +339,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 2)
     using K = Kinds<EDGE>;
     constexpr int KIND = K::MS;
     constexpr LamTab L = lamtab(KIND);
-    constexpr int N = L.N, N0 = L.N0, MM = L.MM;
-    constexpr RepTab<KIND, N, N> RT{};
+    constexpr int N0 = L.N0;
     if (s.refused()) return;
     const int G = share_chunks<R, KIND>(s), g0 = pass * G;
     if (!G || g0 >= s.chunks) return;
@@ -230,34 +364,22 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 2)
                 out[o + e] = cz<R>();
                 continue;
             }
-            C2<R> P[N][N0];
+            C2<R> P[N0][6];                                  // columns, in the flip basis
             for (int k = 1; k <= nsc; ++k) {
-                C2<R> f[RT.n];
-                load_f<R, RT.n>(s.F + ((int64_t)cls_sh[w][k - 1] * G + gc) * f_chunk_bytes<R, KIND>(), lane, f);
-                C2<R> ph[2 * MM + 1];
-                phase_powers<R, MM>(g.phs[k + 1], ph);
+                C2<R> f[20];
+                load_f<R, 20>(s.F + ((int64_t)cls_sh[w][k - 1] * G + gc) * f_chunk_bytes<R, KIND>(), lane, f);
+                const C2<R> e1 = g.phs[k + 1], e2 = cmul(e1, e1);
+                if (k == 1) {
 #pragma unroll
-                for (int b = 0; b < N0; ++b) {
-                    C2<R> col[N];
+                    for (int c = 0; c < N0; ++c) block_first<R, KIND>(f, e1, e2, c, P[c]);
+                } else {
 #pragma unroll
-                    for (int a = 0; a < N; ++a) {
-                        C2<R> v = cz<R>();
-                        if (k == 1) {
-                            v = RT.sg[a][b] > 0 ? f[RT.rep[a][b]] : cscl(f[RT.rep[a][b]], R(-1));
-                        } else if (sizeof(R) == 8 || a < N0 || k < nsc) {   // the termination reads rows < N0 only
-#pragma unroll
-                            for (int c = 0; c < N; ++c) {
-                                const C2<R> fv = f[RT.rep[a][c]];
-                                v = RT.sg[a][c] > 0 ? cfma(fv, P[c][b], v) : cfms(fv, P[c][b], v);
-                            }
-                        }
-                        col[a] = cmul(ph[L.m[a] + MM], v);
-                    }
-#pragma unroll
-                    for (int a = 0; a < N; ++a) P[a][b] = col[a];
+                    for (int c = 0; c < N0; ++c) block_step<R, KIND>(f, e1, e2, k < nsc, P[c]);
                 }
             }
-            const C2<R> ptrac = termination<R, KIND>(g, T, e, nleg, ck, [&](int b, int a) { return P[b][a]; });
+            C2<R> Q[N0][N0];
+            from_blocks<R, KIND>([&](int c, int i) { return P[c][i]; }, Q);
+            const C2<R> ptrac = termination<R, KIND>(g, T, e, nleg, ck, [&](int b, int a) { return Q[b][a]; });
             out[o + e] = cmul(ptrac, cfac(g, T, e, nleg, ck));
         }
         __syncwarp();
@@ -296,27 +418,8 @@ template <typename R, int KIND> __global__ void k_share_reff(Share<R> s, R *__re
 
 // ------------------------------------------------------------------------------------------------ launches
 template <typename R, int EDGE>
-Share<R> share_view(const SharePlan &pl, unsigned char *ws, ShareHead *head, const int *status, int L1)
-{
-    Share<R> s{};
-    s.rec = ws + pl.rec; s.rec_bytes = geo_bytes<R>();
-    s.key = reinterpret_cast<ShareKey *>(ws + pl.key);
-    s.slot_of = reinterpret_cast<int *>(ws + pl.slot);
-    s.hash = reinterpret_cast<unsigned *>(ws + pl.hash); s.hmask = pl.hcap - 1;
-    s.cls = reinterpret_cast<int *>(ws + pl.cls);
-    s.owner = reinterpret_cast<unsigned *>(ws + pl.owner); s.cls_cap = pl.cls_cap;
-    s.two = reinterpret_cast<int *>(ws + pl.two);
-    s.tab = reinterpret_cast<R *>(ws + pl.tab); s.tab_len = (L1 + 1) * dstride(lamtab(Kinds<EDGE>::MS).MM);
-    s.F = ws + pl.F; s.f_bytes = pl.f_bytes;
-    s.chunks = pl.chunks; s.force = pl.force; s.nsc_max = pl.nsc_max;
-    s.head = head; s.status = status;
-    return s;
-}
-
-// The sub-batch's classes and the signals of its paths in out (n, E); where the form is not taken, head->general is set
-// and out is left alone.  coords, ipots, nlegs: whole arrays (order picks the sub-batch) or the sub-batch's own.
-template <typename R, int EDGE, typename CT>
-fg_status share_signals(const StageView &sv, const Tables<R> &T, const SharePlan &pl, Share<R> &s, const CT *coords,
+template <typename CT>
+fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T, const SharePlan &pl, Share<R> &s, const CT *coords,
                         const int64_t *ipots, int *status, C2<R> *out, cudaStream_t st)
 {
     using K = Kinds<EDGE>;
@@ -349,123 +452,580 @@ fg_status share_signals(const StageView &sv, const Tables<R> &T, const SharePlan
     return FG_OK;
 }
 
-// The one-kernel form of the drop-in call; gate as in launch_fused.
-template <typename R, int EDGE, typename CT>
-fg_status launch_cchi(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const CT *coords,
-                      const int64_t *ipots, C2<R> *cchi, R *reff, int *bad, int warps, const int *gate, cudaStream_t st)
+template <typename R, int EDGE>
+fg_status ShareLaunch<R, EDGE>::fine(const StageView &sv, const Share<R> &s, const PathsDev &pd, int NK, const double *q,
+                                     const double *S, const int *span, const C2<R> *sig, unsigned long long *racc,
+                                     double *reff_save, int *status, cudaStream_t st)
 {
-    using K = Kinds<EDGE>;
-    const size_t wb = warp_bytes<R>(sv.L1, nleg - 1, nleg == 2 ? K::MMSS : K::MMMS, sv.E, false);
-    warps = fit_warps(warps, wb, sv.max_smem);
+    auto kern = k_share_fine<R, Kinds<EDGE>::MS>;
+    const size_t wb = 2 * align_up((size_t)sv.E * sizeof(double), 16);
+    const int warps = fit_warps(4, wb, sv.max_smem);
     int blocks = 0;
-    auto kern = k_cchi<R, EDGE, CT>;
-    if (fg_status rc = grid_for(kern, warps * 32, wb * warps, sv.num_sms, B, blocks)) return rc;
-    kern<<<blocks, warps * 32, wb * warps, st>>>(T, coords, ipots, B, nleg, cchi, reff, bad, wb, gate);
+    if (fg_status rc = grid_for(kern, 32 * warps, wb * warps, sv.num_sms, s.n, blocks)) return rc;
+    kern<<<blocks, 32 * warps, wb * warps, st>>>(s, pd, sv.E, NK, q, S, span, sig, racc, reff_save, status, wb);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
 
-template <typename R, int EDGE, typename CT>
-fg_status cchi_call(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const CT *coords,
-                    const int64_t *ipots, C2<R> *cchi, R *reff, int *bad, int warps, unsigned char *ws, size_t ws_bytes,
-                    cudaStream_t st)
+template <typename R, int EDGE> fg_status ShareLaunch<R, EDGE>::reff(const Share<R> &s, R *out, cudaStream_t st)
 {
-    const SharePlan pl = ws ? share_plan(B, nleg, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit) : SharePlan{};
-    if constexpr (EDGE <= 3)
-        if (pl.sub && ws_bytes >= kCounterBytes + pl.total) {
-            ShareHead *head = reinterpret_cast<ShareHead *>(ws);
-            Share<R> s = share_view<R, EDGE>(pl, ws + kCounterBytes, head, nullptr, sv.L1);
-            s.stride = s.nleg_uniform = nleg;
-            for (int64_t t0 = 0; t0 < B; t0 += pl.sub) {
-                s.n = std::min<int64_t>(pl.sub, B - t0);
-                const CT *c = coords + t0 * nleg * 3;
-                const int64_t *ip = ipots + t0 * nleg;
-                C2<R> *out = cchi + t0 * sv.E;
-                if (fg_status rc = share_signals<R, EDGE, CT>(sv, T, pl, s, c, ip, bad, out, st)) return rc;
-                k_share_reff<R, Kinds<EDGE>::MS><<<(int)std::min<int64_t>((s.n + 255) / 256, 148 * 4), 256, 0, st>>>(s, reff + t0);
-                FG_CUDA(cudaGetLastError());
-                if (!pl.force)
-                    if (fg_status rc = launch_cchi<R, EDGE, CT>(sv, T, s.n, nleg, c, ip, out, reff + t0, bad, warps,
-                                                                &head->general, st))
-                        return rc;
-            }
-            return FG_OK;
-        }
-    timer_begin(st);
-    if (fg_status rc = launch_cchi<R, EDGE, CT>(sv, T, B, nleg, coords, ipots, cchi, reff, bad, warps, nullptr, st)) return rc;
-    timer_end(st);
+    k_share_reff<R, Kinds<EDGE>::MS><<<(int)std::min<int64_t>((s.n + 255) / 256, 148 * 4), 256, 0, st>>>(s, out);
+    FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
 
-template <typename R, int EDGE>
-fg_status Launch<R, EDGE>::cchi(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const void *coords,
-                                int coords_f64, const int64_t *ipots, void *cchi, void *reff, int *bad, int warps,
-                                unsigned char *ws, size_t ws_bytes, cudaStream_t st)
+// ------------------------------------------------------------------------------------------------ shared matrices
+// The adjoint with shared scattering matrices (fg_shared.cuh): a class keeps, per energy, F~ and its derivatives along
+// beta and the lengths of its two legs, so that a path's sweep 2 contracts its orbit weights with them instead of
+// running the partial waves again: 60 complex multiply-adds and 480 bytes per scatterer and energy (FP32) against
+// about 25 x 60 multiply-adds.
+//
+//   k_share_geom_adj    a warp per path: the record with the frame and d/dbeta of the termination, the keys
+//   k_share_tables_adj  a thread per (class, entry): D and D'
+//   k_share_f_adj       two warps per (class, 32 energies): (F~, dF~/dbeta) and (dF~/drho_in, dF~/drho_out)
+//   k_share_chain_adj   a warp per (path, energies): energy_ms_adj's sweeps with the matrices read
+//   k_share_two_adj     a warp per (two-leg path, energies)
+//   k_share_coord_grad  a warp per path: parameter gradients summed in a fixed order, carried to the coordinates
+template <typename R> __device__ __forceinline__ AdjExtra<R> &adj_extra(unsigned char *rec)
 {
-    C2<R> *c = static_cast<C2<R> *>(cchi);
-    R *rf = static_cast<R *>(reff);
-    if (coords_f64)
-        return cchi_call<R, EDGE>(sv, T, B, nleg, static_cast<const double *>(coords), ipots, c, rf, bad, warps, ws, ws_bytes, st);
-    return cchi_call<R, EDGE>(sv, T, B, nleg, static_cast<const float *>(coords), ipots, c, rf, bad, warps, ws, ws_bytes, st);
+    return *reinterpret_cast<AdjExtra<R> *>(rec + geo_bytes<R>());
+}
+
+template <typename R, typename CT>
+__global__ void __launch_bounds__(128) k_share_geom_adj(Tables<R> T, Share<R> s, const CT *__restrict__ coords,
+                                                        const int64_t *__restrict__ ipots, int *status, int MM_ss,
+                                                        int MM_ms)
+{
+    if (*(volatile const int *)status & kBadLayout) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned char *base = smem + (size_t)w * s.rec_bytes;
+    WarpPath<R> &g = *reinterpret_cast<WarpPath<R> *>(base);
+    for (int64_t i = (int64_t)blockIdx.x * 4 + w; i < s.n; i += (int64_t)gridDim.x * 4) {
+        const int64_t p = s.path(i);
+        const int nleg = s.legs(p);
+        path_setup<R, CT>(g, nullptr, T, coords + p * s.stride * 3, ipots + p * s.stride, nleg, lane, status,
+                          nleg == 2 ? MM_ss : MM_ms, false);
+        term_dbeta<R>(g, adj_extra<R>(base).dterm_db, T, nleg, lane);
+        const int frame = choose_frame<R>(g, nleg, lane);
+        if (frame) reframe_path<R>(g, nleg, lane, frame);
+        if (lane == 0) adj_extra<R>(base).frame = frame;
+        __syncwarp();
+        copy16(s.rec + i * s.rec_bytes, base, s.rec_bytes, lane);
+        share_keys(s, g, i, nleg, lane);
+        __syncwarp();
+    }
+}
+
+template <typename R, int KIND> __global__ void __launch_bounds__(128) k_share_tables_adj(Tables<R> T, Share<R> s)
+{
+    constexpr int MM = lamtab(KIND).MM, NC = ncanon(MM), DS = dstride(MM);
+    if (s.refused()) return;
+    if (!share_chunks<R, KIND>(s)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) s.head->general = 1;       // the one-kernel form that follows runs
+        return;
+    }
+    const int64_t tasks = (int64_t)s.head->classes * NC;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < tasks; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t c = i / NC;
+        R *t = s.tab + c * 2 * s.tab_len;
+        rotation_column_adj<R>(t, t + s.tab_len, T, __longlong_as_double((long long)s.key[s.owner[c]].z), MM, DS,
+                               (int)(i % NC));
+    }
+}
+
+// F~ (accumulate_f's operations) and dF~/dbeta of one class and energy, from its two rotation tables
+template <typename R, int KIND>
+__device__ __forceinline__ void accumulate_f_beta(C2<R> (&acc)[RepTab<KIND, lamtab(KIND).N, lamtab(KIND).N>().n],
+                                                  C2<R> (&accb)[RepTab<KIND, lamtab(KIND).N, lamtab(KIND).N>().n],
+                                                  const R *dh, const R *dhd, const C2<R> *tlk, int E, int ilx,
+                                                  C2<R> z_in, C2<R> z_out)
+{
+    constexpr LamTab L = lamtab(KIND);
+    constexpr RepTab<KIND, L.N, L.N> RT{};
+    constexpr int DS = dstride(L.MM), NCAN = ncanon(L.MM), CI = L.CI, CO = L.CO;
+#pragma unroll
+    for (int r = 0; r < RT.n; ++r) acc[r] = accb[r] = cz<R>();
+    C2<R> pi[CI + 1], ci[CI + 1], po[CO + 1], co[CO + 1];
+#pragma unroll
+    for (int j = 0; j <= CI; ++j) pi[j] = ci[j] = cz<R>();
+#pragma unroll
+    for (int j = 0; j <= CO; ++j) po[j] = co[j] = cz<R>();
+    pi[1] = ci[1] = po[1] = co[1] = C2<R>{R(1), R(0)};
+    C2<R> t1 = tlk[E];
+    for (int il = 1; il <= ilx; ++il) {
+        const C2<R> t = t1;
+        if (il < ilx) t1 = tlk[(size_t)(il + 1) * E];
+        R d[NCAN], dd[NCAN];
+        load_row<R, NCAN>(dh + (size_t)il * DS, d);
+        load_row<R, NCAN>(dhd + (size_t)il * DS, dd);
+        C2<R> tco[CO + 1];
+#pragma unroll
+        for (int j = 1; j <= CO; ++j) tco[j] = pmul(t, co[j]);
+#pragma unroll
+        for (int r = 0; r < RT.n; ++r) {
+            const C2<R> u = pmul(ci[RT.ci[r]], tco[RT.co[r]]);
+            acc[r] = pfmr(u, d[RT.d[r]], acc[r]);
+            accb[r] = pfmr(u, dd[RT.d[r]], accb[r]);
+        }
+        const R w = R(2 * il - 1);
+        const C2<R> wi = cscl(z_in, w), wo = cscl(z_out, w);
+        C2<R> ni[CI + 1], no[CO + 1];
+        ni[1] = cfms(wi, ci[1], pi[1]);
+#pragma unroll
+        for (int j = 2; j <= CI; ++j) ni[j] = cfms(wi, cadd(ci[j], ci[j - 1]), pi[j]);
+        no[1] = cfms(wo, co[1], po[1]);
+#pragma unroll
+        for (int j = 2; j <= CO; ++j) no[j] = cfms(wo, cadd(co[j], co[j - 1]), po[j]);
+#pragma unroll
+        for (int j = 1; j <= CI; ++j) { pi[j] = ci[j]; ci[j] = ni[j]; }
+#pragma unroll
+        for (int j = 1; j <= CO; ++j) { po[j] = co[j]; co[j] = no[j]; }
+    }
+}
+
+// dF~/drho_in and dF~/drho_out of one class and energy (the spherical waves' derivatives as in contract_f_adj)
+template <typename R, int KIND>
+__device__ __forceinline__ void accumulate_f_rho(C2<R> (&ai)[RepTab<KIND, lamtab(KIND).N, lamtab(KIND).N>().n],
+                                                 C2<R> (&ao)[RepTab<KIND, lamtab(KIND).N, lamtab(KIND).N>().n],
+                                                 const R *dh, const C2<R> *tlk, int E, int ilx, C2<R> z_in, C2<R> z_out)
+{
+    constexpr LamTab L = lamtab(KIND);
+    constexpr RepTab<KIND, L.N, L.N> RT{};
+    constexpr int DS = dstride(L.MM), NCAN = ncanon(L.MM), CI = L.CI, CO = L.CO;
+#pragma unroll
+    for (int r = 0; r < RT.n; ++r) ai[r] = ao[r] = cz<R>();
+    C2<R> pi[CI + 2], ci[CI + 2], po[CO + 2], co[CO + 2];
+#pragma unroll
+    for (int j = 0; j <= CI + 1; ++j) pi[j] = ci[j] = cz<R>();
+#pragma unroll
+    for (int j = 0; j <= CO + 1; ++j) po[j] = co[j] = cz<R>();
+    pi[1] = ci[1] = po[1] = co[1] = C2<R>{R(1), R(0)};
+    C2<R> t1 = tlk[E];
+    for (int il = 1; il <= ilx; ++il) {
+        const C2<R> t = t1;
+        if (il < ilx) t1 = tlk[(size_t)(il + 1) * E];
+        R d[NCAN];
+        load_row<R, NCAN>(dh + (size_t)il * DS, d);
+        C2<R> tco[CO + 1], tdco[CO + 1], dci[CI + 1];
+#pragma unroll
+        for (int j = 1; j <= CO; ++j) {
+            tco[j] = pmul(t, co[j]);
+            tdco[j] = pmul(t, mi_z(z_out, pfmr(co[j], R(j - 1), cscl(co[j + 1], R(j)))));
+        }
+#pragma unroll
+        for (int j = 1; j <= CI; ++j) dci[j] = mi_z(z_in, pfmr(ci[j], R(j - 1), cscl(ci[j + 1], R(j))));
+#pragma unroll
+        for (int r = 0; r < RT.n; ++r) {
+            ai[r] = pfmr(pmul(dci[RT.ci[r]], tco[RT.co[r]]), d[RT.d[r]], ai[r]);
+            ao[r] = pfmr(pmul(ci[RT.ci[r]], tdco[RT.co[r]]), d[RT.d[r]], ao[r]);
+        }
+        const R w = R(2 * il - 1);
+        const C2<R> wi = cscl(z_in, w), wo = cscl(z_out, w);
+        C2<R> ni[CI + 2], no[CO + 2];
+#pragma unroll
+        for (int j = 1; j <= CI + 1; ++j) ni[j] = pfms(wi, j > 1 ? padd(ci[j], ci[j - 1]) : ci[j], pi[j]);
+#pragma unroll
+        for (int j = 1; j <= CO + 1; ++j) no[j] = pfms(wo, j > 1 ? padd(co[j], co[j - 1]) : co[j], po[j]);
+#pragma unroll
+        for (int j = 1; j <= CI + 1; ++j) { pi[j] = ci[j]; ci[j] = ni[j]; }
+#pragma unroll
+        for (int j = 1; j <= CO + 1; ++j) { po[j] = co[j]; co[j] = no[j]; }
+    }
+}
+
+// Items (class, chunk of the pass, half): the class's four matrices over the chunk lie one after the other (F~, beta,
+// rho_in, rho_out).  Entries outside a lower lambda order's set are stored as zeros, derivatives too, so a path's
+// weights need no masking.
+template <typename R, int EDGE>
+__global__ void __launch_bounds__(128) k_share_f_adj(Tables<R> T, Share<R> s, int pass, size_t wbytes)
+{
+    using K = Kinds<EDGE>;
+    constexpr int KIND = K::MS;
+    constexpr LamTab L = lamtab(KIND);
+    constexpr RepTab<KIND, L.N, L.N> RT{};
+    const int G = s.refused() ? 0 : share_chunks<R, KIND>(s), g0 = pass * G;
+    const int ng = min(G, s.chunks - g0), E = T.E;          // <= 0: nothing to do
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    R *dh = reinterpret_cast<R *>(smem + (size_t)w * wbytes);
+    const int64_t items = ng > 0 ? (int64_t)s.head->classes * ng * 2 : 0;
+    for (int64_t it = (int64_t)blockIdx.x * nw + w; it < items; it += (int64_t)gridDim.x * nw) {
+        const int half = (int)(it & 1), gc = (int)((it >> 1) % ng);
+        const int64_t c = (it >> 1) / ng;
+        const int e = first_chunk(E) + 32 * (g0 + gc) + lane;
+        copy16(dh, s.tab + c * 2 * s.tab_len, (size_t)s.tab_len * sizeof(R) * (half ? 1 : 2), lane);
+        const ShareKey key = s.key[s.owner[c]];
+        __syncwarp();
+        if (e >= 0 && e < E) {
+            const C2<R> ck = T.ck[e];
+            if (fabs((double)ck.x) + fabs((double)ck.y) > 1e-16) {
+                const int ip = (int)key.w;
+                const C2<R> *tl = T.tl + (size_t)ip * (T.L1 + 1) * E + e;
+                const int ilx = T.lmax[ip * E + e] + 1;
+                const C2<R> z_in = zfac(cscl(ck, (R)__longlong_as_double((long long)key.y)));
+                const C2<R> z_out = zfac(cscl(ck, (R)__longlong_as_double((long long)key.x)));
+                C2<R> a[RT.n], b[RT.n];
+                if (half) accumulate_f_rho<R, KIND>(a, b, dh, tl, E, ilx, z_in, z_out);
+                else accumulate_f_beta<R, KIND>(a, b, dh, dh + s.tab_len, tl, E, ilx, z_in, z_out);
+                mask_lambda<R, KIND, L.N, L.N>(a, T.nlam);
+                mask_lambda<R, KIND, L.N, L.N>(b, T.nlam);
+                unsigned char *at = s.F + ((c * G + gc) * 4 + 2 * half) * f_chunk_bytes<R, KIND>();
+                C2<R> f[20];
+                to_blocks<R, KIND>(a, f);
+                store_f<R, 20>(at, lane, f);
+                to_blocks<R, KIND>(b, f);
+                store_f<R, 20>(at + f_chunk_bytes<R, KIND>(), lane, f);
+            }
+        }
+        __syncwarp();
+    }
+    // the kernel that this one may run beside (k_share_two_adj) has ended before this one does
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+// g + sum of w[r] f[r] over a stored matrix's canonical entries
+template <typename R, int NE>
+__device__ __forceinline__ C2<R> dot_f(const unsigned char *at, int lane, const C2<R> (&w)[NE])
+{
+    C2<R> f[NE], g0 = cz<R>(), g1 = cz<R>();
+    load_f<R, NE>(at, lane, f);
+#pragma unroll
+    for (int r = 0; r < NE; r += 2) {
+        g0 = pfma(w[r], f[r], g0);
+        g1 = pfma(w[r + 1], f[r + 1], g1);
+    }
+    return cadd(g0, g1);
+}
+
+// One energy of a path of three and more legs: energy_ms_adj with its matrices and their derivatives read (cls: the
+// path's classes, at(c): where class c's four matrices of this chunk lie).
+template <typename R, int KIND, class AT>
+__device__ __forceinline__ void shared_energy_adj(const WarpPath<R> &g, const R (*dterm_db)[49], const Tables<R> &T, int e,
+                                                  int nleg, int lane, C2<R> gbar, const AT &at, ParGrad &pg)
+{
+    constexpr LamTab L = lamtab(KIND);
+    constexpr int N0 = L.N0;
+    using B = Flip<KIND>;
+    constexpr size_t FB = f_chunk_bytes<R, KIND>();
+    const int nsc = nleg - 1;
+    const C2<R> ck = T.ck[e];
+    if (fabs((double)ck.x) + fabs((double)ck.y) <= 1e-16) return;
+    auto add_re = [](double &acc, C2<R> s, C2<R> v) { acc += (double)s.x * v.x - (double)s.y * v.y; };
+    const C2<R> cf = cfac(g, T, e, nleg, ck);
+    const C2<R> sd = cmul(C2<R>{gbar.x, -gbar.y}, cf);      // s = conj(gbar) cfac: dL = Re(s dptrac)
+    const C2<R> sck = cmul(sd, ck);
+    // everything in the flip basis: P_k by columns (k = 0: the N0 unit columns), R_k by rows
+    C2<R> Pst[kMaxLeg][N0][6];
+    C2<R> Rst[N0][6];
+#pragma unroll
+    for (int c = 0; c < N0; ++c)
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+            Pst[0][c][i] = (c < B::NE0 ? i == c : i == 4 + c - B::NE0) ? C2<R>{R(1), R(0)} : cz<R>();
+    for (int k = 1; k <= nsc; ++k) {
+        C2<R> f[20];
+        load_f<R, 20>(at(k), lane, f);
+        const C2<R> e1 = g.phs[k + 1], e2 = cmul(e1, e1);
+#pragma unroll 1
+        for (int c = 0; c < N0; ++c) {
+            C2<R> x[6];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) x[i] = Pst[k - 1][c][i];
+            block_step<R, KIND>(f, e1, e2, true, x);
+#pragma unroll
+            for (int i = 0; i < 6; ++i) Pst[k][c][i] = x[i];
+        }
+    }
+    {
+        TermLegs<R, KIND> tl;
+        term_legs<R, KIND>(g, T, e, nleg, ck, tl);
+        C2<R> ge1 = cz<R>(), gbn = cz<R>(), gr1 = cz<R>(), grn = cz<R>();
+        C2<R> Q[N0][N0], Tm[N0][N0];
+        from_blocks<R, KIND>([&](int c, int i) { return Pst[nsc][c][i]; }, Q);
+        const C2<R> ptrac = term_adj<R, KIND>(g, dterm_db, T, e, tl, [&](int b, int a) { return Q[b][a]; }, ge1, gbn, gr1,
+                                              grn, &Tm[0][0], N0);
+        add_re(pg.eta[1], sd, ge1);
+        add_re(pg.beta[nleg], sd, gbn);
+        add_re(pg.ri[1], sck, gr1);
+        add_re(pg.ri[nleg], sck, grn);
+        cfac_grad(g, T, e, nleg, gbar, cmul(ptrac, cf), pg);
+        // R_nsc = [T 0] in the flip basis: rows u, w of T, then its columns halved back
+        auto mix = [](C2<R> p, C2<R> m, int am, bool w) {      // p +- (-1)^am m
+            return ((am & 1) != 0) != w ? csub(p, m) : cadd(p, m);
+        };
+#pragma unroll
+        for (int c = 0; c < N0; ++c) {
+            const bool cw = c >= B::NE0;
+            const int cm = cw ? c - B::NE0 + 1 : B::em(c), cn = cw ? 0 : B::en(c);
+            C2<R> row[N0];
+#pragma unroll
+            for (int b = 0; b < N0; ++b)
+                row[b] = cm == 0 ? Tm[B::at(0, cn)][b] : mix(Tm[B::at(cm, 0)][b], Tm[B::at(-cm, 0)][b], cm, cw);
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                const bool iw = i >= 4;
+                const int im = iw ? i - 3 : B::em(i), in = iw ? 0 : B::en(i);
+                C2<R> v = cz<R>();
+                if (iw ? i - 4 < B::NO0 : i < B::NE0)
+                    v = im == 0 ? row[B::at(0, in)] : cscl(mix(row[B::at(im, 0)], row[B::at(-im, 0)], im, iw), R(0.5));
+                Rst[c][i] = v;
+            }
+        }
+    }
+    for (int k = nsc; k >= 1; --k) {
+        const C2<R> e1 = g.phs[k + 1], e2 = cmul(e1, e1);
+        // weights of F~_k's block entries, (P_(k-1) R_k Phi)[j][i], and the Euler angle's derivative
+        // -i sum_m m (P_k R_k)(m, m), which in this basis pairs u_m with w_m
+        C2<R> Wh[20], tm = cz<R>();
+#pragma unroll
+        for (int r = 0; r < 20; ++r) Wh[r] = cz<R>();
+#pragma unroll 1
+        for (int c = 0; c < N0; ++c) {
+            C2<R> p[6], rr[6];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) { p[i] = Pst[k - 1][c][i]; rr[i] = Rst[c][i]; }
+            tm = pfma(rr[2], Pst[k][c][4], pfma(rr[4], Pst[k][c][2], tm));
+            tm = pfma(cscl(rr[3], R(2)), Pst[k][c][5], pfma(cscl(rr[5], R(2)), Pst[k][c][3], tm));
+            turn(e1, rr[2], rr[4]);
+            turn(e2, rr[3], rr[5]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) Wh[4 * i + j] = pfma(p[j], rr[i], Wh[4 * i + j]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) Wh[16 + 2 * i + j] = pfma(p[4 + j], rr[4 + i], Wh[16 + 2 * i + j]);
+        }
+        add_re(pg.eta[k + 1], sd, C2<R>{tm.y, -tm.x});   // -i tm
+        const unsigned char *m = at(k);
+        add_re(pg.beta[k], sd, dot_f<R, 20>(m + FB, lane, Wh));
+        add_re(pg.ri[k + 1], sck, dot_f<R, 20>(m + 2 * FB, lane, Wh));
+        add_re(pg.ri[k], sck, dot_f<R, 20>(m + 3 * FB, lane, Wh));
+        if (k > 1) {
+            // R_(k-1) = R_k Phi F~_k, one row at a time
+            C2<R> f[20];
+            load_f<R, 20>(m, lane, f);
+#pragma unroll 1
+            for (int c = 0; c < N0; ++c) {
+                C2<R> rr[6];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) rr[i] = Rst[c][i];
+                turn(e1, rr[2], rr[4]);
+                turn(e2, rr[3], rr[5]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    C2<R> v = cz<R>();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v = pfma(rr[i], f[4 * i + j], v);
+                    Rst[c][j] = v;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    Rst[c][4 + j] = pfma(rr[5], f[18 + j], pfma(rr[4], f[16 + j], cz<R>()));
+            }
+        }
+    }
+}
+
+// The parameter gradients of one item summed over the warp's energies into the path's entry of its part (gpar), added
+// to what earlier passes left there.
+__device__ __forceinline__ void store_par(double *o, const ParGrad &pg, int nleg, int lane, bool first)
+{
+    for (int j = 1; j <= nleg; ++j) {
+        double v[3] = {pg.ri[j], pg.beta[j], pg.eta[j]};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int h = 16; h > 0; h >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], h);
+        }
+        if (lane < 3) {
+            const double x = lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]);
+            double &at = o[lane * (kMaxLeg + 1) + j];
+            at = first ? x : at + x;
+        }
+    }
 }
 
 template <typename R, int EDGE>
-fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const fg_paths *P, int NK, const double *q,
-                                 const double *S, const int *span, double *rows, void *cchi_save, double *reff_save,
-                                 unsigned char *ws, const FusedShape &shape, cudaStream_t st,
-                                 unsigned long long *words, unsigned char *share_ws, size_t share_bytes)
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 2) k_share_chain_adj(Tables<R> T, Share<R> s, int pass, int split,
+                                                         const C2<R> *__restrict__ gbar, double *__restrict__ gpar)
 {
     using K = Kinds<EDGE>;
-    unsigned long long *counter = reinterpret_cast<unsigned long long *>(ws);
-    int *status = reinterpret_cast<int *>(ws + kStatusOffset);
-    unsigned long long *racc = words ? words : reinterpret_cast<unsigned long long *>(ws + kCounterBytes);
-    if (words) {
-        FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes, st));
-        FG_CUDA(cudaMemsetAsync(words, 0, (size_t)2 * P->nrows * NK * sizeof(unsigned long long), st));
-    } else {
-        FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes + row_sum_bytes(P->nrows, NK), st));
-    }
-    if (fg_status rc = launch_validate(P, sv.nph1, status, st)) return rc;
-    const SharePlan pl = P->n > 0 ? share_plan(P->n, P->nleg_max, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit) : SharePlan{};
-    if (pl.sub && share_ws && share_bytes >= pl.total) {
-        if constexpr (EDGE <= 3) {
-            ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
-            Share<R> s = share_view<R, EDGE>(pl, share_ws, head, status, sv.L1);
-            s.stride = P->nleg_max;
-            s.nlegs = P->nleg;
-            s.by_path = cchi_save != nullptr;
-            C2<R> *sig = cchi_save ? static_cast<C2<R> *>(cchi_save) : reinterpret_cast<C2<R> *>(share_ws + pl.sig);
-            auto kern = k_share_fine<R, K::MS>;
-            const size_t wb = 2 * align_up((size_t)sv.E * sizeof(double), 16);
-            const int warps = fit_warps(4, wb, sv.max_smem);
-            for (int64_t t0 = 0; t0 < P->n; t0 += pl.sub) {
-                s.n = std::min<int64_t>(pl.sub, P->n - t0);
-                s.order = P->order + t0;
-                if (fg_status rc = share_signals<R, EDGE, double>(sv, T, pl, s, P->coords, P->ipots, status, sig, st))
-                    return rc;
-                const PathsDev pd{s.n, P->nleg_max, P->nrows, P->coords, P->ipots, P->nleg, P->deg, P->sigma2, s.order, P->row};
-                int blocks = 0;
-                if (fg_status rc = grid_for(kern, 32 * warps, wb * warps, sv.num_sms, s.n, blocks)) return rc;
-                kern<<<blocks, 32 * warps, wb * warps, st>>>(s, pd, sv.E, NK, q, S, span, sig, racc, reff_save, status, wb);
-                FG_CUDA(cudaGetLastError());
-                if (!pl.force) {
-                    if (t0) FG_CUDA(cudaMemsetAsync(counter, 0, sizeof(*counter), st));
-                    if (fg_status rc = launch_fused<R, EDGE>(sv, T, pd, NK, q, S, span, racc, cchi_save, reff_save, counter,
-                                                             status, shape, &head->general, st))
-                        return rc;
-                }
-            }
+    constexpr int KIND = K::MS;
+    if (s.refused()) return;
+    const int G = share_chunks<R, KIND>(s), g0 = pass * G;
+    if (!G || g0 >= s.chunks) return;
+    const int ng = min(G, s.chunks - g0), E = T.E;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int cls_sh[4][kMaxLeg];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned char *base = smem + (size_t)w * s.rec_bytes;
+    const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(base);
+    for (int64_t it = (int64_t)blockIdx.x * 4 + w; it < s.n * split; it += (int64_t)gridDim.x * 4) {
+        const int64_t i = it / split, p = s.path(i);
+        const int nleg = s.legs(p);
+        if (nleg == 2) continue;
+        copy16(base, s.rec + i * s.rec_bytes, s.rec_bytes, lane);
+        if (lane < nleg - 1) cls_sh[w][lane] = s.cls[s.slot_of[i * s.nsc_max + lane]];
+        __syncwarp();
+        ParGrad pg;
+        for (int j = 0; j <= kMaxLeg; ++j) pg.ri[j] = pg.beta[j] = pg.eta[j] = 0.0;
+        for (int gc = (int)(it % split); gc < ng; gc += split) {
+            const int e = first_chunk(E) + 32 * (g0 + gc) + lane;
+            if (e >= 0 && e < E)
+                shared_energy_adj<R, KIND>(
+                    g, adj_extra<R>(base).dterm_db, T, e, nleg, lane, gbar[p * E + e],
+                    [&](int k) { return s.F + ((int64_t)cls_sh[w][k - 1] * G + gc) * 4 * f_chunk_bytes<R, KIND>(); }, pg);
+            __syncwarp();
         }
-    } else if (P->n > 0) {
-        const PathsDev pd{P->n, P->nleg_max, P->nrows, P->coords, P->ipots, P->nleg, P->deg, P->sigma2, P->order, P->row};
-        timer_begin(st);
-        if (fg_status rc = launch_fused<R, EDGE>(sv, T, pd, NK, q, S, span, racc, cchi_save, reff_save, counter, status,
-                                                 shape, nullptr, st))
-            return rc;
-        timer_end(st);
+        store_par(gpar + ((it % split) * s.n + i) * kGparStride, pg, nleg, lane, pass == 0);
+        __syncwarp();
     }
-    if (!rows) return FG_OK;
-    return launch_row_finish(P->nrows, NK, racc, rows, status, st);
+}
+
+// Two-leg paths, all their energies in one launch
+template <typename R, int EDGE>
+__global__ void __launch_bounds__(128) k_share_two_adj(Tables<R> T, Share<R> s, int split,
+                                                       const C2<R> *__restrict__ gbar, double *__restrict__ gpar,
+                                                       size_t wbytes)
+{
+    using K = Kinds<EDGE>;
+    if (s.refused() || !share_chunks<R, K::MS>(s)) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    // k_share_f_adj, which needs nothing of this kernel, may start beside it (its launch allows it)
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, E = T.E;
+    unsigned char *base = smem + (size_t)w * wbytes;
+    const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(base);
+    R *dh = reinterpret_cast<R *>(base + s.rec_bytes), *dhd = dh + (size_t)(T.L1 + 1) * dstride(K::MMSS);
+    for (int64_t it = (int64_t)blockIdx.x * nw + w; it < (int64_t)s.head->two * split; it += (int64_t)gridDim.x * nw) {
+        const int64_t i = s.two[it / split], p = s.path(i);
+        copy16(base, s.rec + i * s.rec_bytes, s.rec_bytes, lane);
+        __syncwarp();
+        for (int r = lane; r < ncanon(K::MMSS); r += 32)
+            rotation_column_adj<R>(dh, dhd, T, g.beta[1], K::MMSS, dstride(K::MMSS), r);
+        __syncwarp();
+        ParGrad pg;
+        for (int j = 0; j <= kMaxLeg; ++j) pg.ri[j] = pg.beta[j] = pg.eta[j] = 0.0;
+        for (int gc = (int)(it % split); gc < s.chunks; gc += split) {
+            const int e = first_chunk(E) + 32 * gc + lane;
+            if (e >= 0 && e < E)
+                path_energy_adj<R, EDGE>(g, dh, dhd, adj_extra<R>(base).dterm_db, T, e, 2, gbar[p * E + e], pg);
+            __syncwarp();
+        }
+        store_par(gpar + ((it % split) * s.n + i) * kGparStride, pg, 2, lane, true);
+        __syncwarp();
+    }
+}
+
+// The paths' parameter gradients (their parts summed in order) carried to the coordinates, as k_adjoint and
+// k_coord_grad do it; the atoms come from the record, already in the path's frame.
+template <typename R, int KIND>
+__global__ void __launch_bounds__(128) k_share_coord_grad(Share<R> s, int split, const double *__restrict__ gpar,
+                                                          const double *__restrict__ greff_d,
+                                                          const R *__restrict__ greff_r, double *__restrict__ gout_d,
+                                                          R *__restrict__ gout_r)
+{
+    __shared__ double s_gpar[4][3 * (kMaxLeg + 1)], s_cg[4][9 * kMaxLeg];
+    if (s.refused() || !share_chunks<R, KIND>(s)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int64_t i = (int64_t)blockIdx.x * 4 + w; i < s.n; i += (int64_t)gridDim.x * 4) {
+        const int64_t p = s.path(i);
+        const int nleg = s.legs(p);
+        const unsigned char *rec = s.rec + i * s.rec_bytes;
+        const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(rec);
+        const int frame = reinterpret_cast<const AdjExtra<R> *>(rec + geo_bytes<R>())->frame;
+        const double gr = greff_d ? greff_d[p] : (greff_r ? (double)greff_r[p] : 0.0);
+        for (int t = lane; t < 3 * (kMaxLeg + 1); t += 32) {
+            const int j = t % (kMaxLeg + 1);
+            double v = 0.0;
+            if (j >= 1 && j <= nleg) {
+                for (int q = 0; q < split; ++q) v += gpar[((int64_t)q * s.n + i) * kGparStride + t];
+                if (t < kMaxLeg + 1) v += gr * kBohr * 0.5;          // reff (A) = BOHR sum ri (bohr) / 2
+            }
+            s_gpar[w][t] = v;
+        }
+        __syncwarp();
+        double gc = coord_grad(g.xyz, s_gpar[w], s_cg[w], nleg, lane);
+        if (frame) gc = unframe_grad(gc, lane, frame);
+        if (lane < 3 * s.stride) {
+            const int64_t o = p * s.stride * 3 + lane;
+            const double v = lane < 3 * nleg ? gc : 0.0;
+            if (gout_d) gout_d[o] = v;
+            else gout_r[o] = (R)v;
+        }
+        __syncwarp();
+    }
+}
+
+// One sub-batch's coordinate gradients in the shared form; head->general is set and nothing written where it is not
+// taken.  coords, ipots, gbar, greff and the outputs are indexed by path.
+template <typename R, int EDGE>
+template <typename CT>
+fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T, const SharePlan &pl, Share<R> &s, unsigned char *ws,
+                        const CT *coords, const int64_t *ipots, int *status, const C2<R> *gbar, const double *greff_d,
+                        const R *greff_r, double *gout_d, R *gout_r, cudaStream_t st)
+{
+    using K = Kinds<EDGE>;
+    constexpr int KIND = K::MS;
+    double *gpar = reinterpret_cast<double *>(ws + pl.gpar);
+    s.rec_bytes = geo_bytes<R>() + align_up(sizeof(AdjExtra<R>), 16);
+    FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
+    FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
+    const int pb = (int)std::min<int64_t>((s.n + 3) / 4, (int64_t)sv.num_sms * 16);
+    k_share_geom_adj<R, CT><<<pb, 128, 4 * s.rec_bytes, st>>>(T, s, coords, ipots, status, K::MMSS, K::MMMS);
+    FG_CUDA(cudaGetLastError());
+    if (fg_status rc = launch_share_insert(s, st)) return rc;
+    const int64_t tasks = std::min<int64_t>(s.n * s.nsc_max, s.cls_cap) * ncanon(K::MMMS);
+    k_share_tables_adj<R, KIND><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
+    FG_CUDA(cudaGetLastError());
+    auto kf = k_share_f_adj<R, EDGE>;
+    auto kc = k_share_chain_adj<R, EDGE>;
+    auto k2 = k_share_two_adj<R, EDGE>;
+    const size_t wf = align_up(2 * (size_t)s.tab_len * sizeof(R), 16);
+    const size_t w2 = s.rec_bytes + align_up(2 * (size_t)(sv.L1 + 1) * dstride(K::MMSS) * sizeof(R), 16);
+    const int nf = fit_warps(4, wf, sv.max_smem), n2 = fit_warps(4, w2, sv.max_smem), split = pl.split;
+    int bf = 0, bc = 0, b2 = 0;
+    if (fg_status rc = grid_for(kf, 32 * nf, wf * nf, sv.num_sms, s.n * s.nsc_max * pl.chunks * 2, bf)) return rc;
+    if (fg_status rc = grid_for(kc, 128, 4 * s.rec_bytes, sv.num_sms, s.n * split, bc)) return rc;
+    if (fg_status rc = grid_for(k2, 32 * n2, w2 * n2, sv.num_sms, s.n * split, b2)) return rc;
+    timer_begin(st);
+    k2<<<b2, 32 * n2, w2 * n2, st>>>(T, s, split, gbar, gpar, w2);
+    for (int pass = 0; pass < pl.passes; ++pass) {
+        if (pass == 0) {                                     // beside the two-leg paths' kernel, not after it
+            cudaLaunchAttribute beside{};
+            beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            beside.val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = bf; cfg.blockDim = 32 * nf; cfg.dynamicSmemBytes = wf * nf; cfg.stream = st;
+            cfg.attrs = &beside; cfg.numAttrs = 1;
+            FG_CUDA(cudaLaunchKernelEx(&cfg, kf, T, s, pass, wf));
+        } else {
+            kf<<<bf, 32 * nf, wf * nf, st>>>(T, s, pass, wf);
+        }
+        kc<<<bc, 128, 4 * s.rec_bytes, st>>>(T, s, pass, split, gbar, gpar);
+    }
+    timer_end(st);
+    k_share_coord_grad<R, KIND><<<pb, 128, 0, st>>>(s, split, gpar, greff_d, greff_r, gout_d, gout_r);
+    FG_CUDA(cudaGetLastError());
+    return FG_OK;
 }
 
 }  // namespace fg
+
+#define FG_SHARE_INSTANCE(R, EDGE)                                                                                     \
+    template struct fg::ShareLaunch<R, EDGE>;                                                                         \
+    template fg_status fg::ShareLaunch<R, EDGE>::signals<float>(                                                      \
+        const StageView &, const Tables<R> &, const SharePlan &, Share<R> &, const float *, const int64_t *, int *,   \
+        C2<R> *, cudaStream_t);                                                                                       \
+    template fg_status fg::ShareLaunch<R, EDGE>::signals<double>(                                                     \
+        const StageView &, const Tables<R> &, const SharePlan &, Share<R> &, const double *, const int64_t *, int *,  \
+        C2<R> *, cudaStream_t);                                                                                       \
+    template fg_status fg::ShareLaunch<R, EDGE>::adjoint<float>(                                                      \
+        const StageView &, const Tables<R> &, const SharePlan &, Share<R> &, unsigned char *, const float *,          \
+        const int64_t *, int *, const C2<R> *, const double *, const R *, double *, R *, cudaStream_t);               \
+    template fg_status fg::ShareLaunch<R, EDGE>::adjoint<double>(                                                     \
+        const StageView &, const Tables<R> &, const SharePlan &, Share<R> &, unsigned char *, const double *,         \
+        const int64_t *, int *, const C2<R> *, const double *, const R *, double *, R *, cudaStream_t);

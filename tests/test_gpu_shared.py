@@ -19,7 +19,11 @@ TOL = {torch.complex64: 1e-6, torch.complex128: 1e-13}
 def _list(nph, counts, atoms, seed=0):
     """Paths over few atoms (their scatterers repeat) as PathBatch groups; consecutive atoms differ, revisits allowed."""
     rng = np.random.default_rng(seed)
-    pts = np.concatenate([np.zeros((1, 3)), rng.uniform(-4.0, 4.0, (atoms, 3))])
+    pts = np.zeros((1, 3))
+    while len(pts) <= atoms:                         # no two atoms closer than 1.8 A, as in matter
+        x = rng.uniform(-4.0, 4.0, 3)
+        if np.linalg.norm(pts - x, axis=1).min() > 1.8:
+            pts = np.concatenate([pts, x[None]])
     pot = np.concatenate([[0], rng.integers(1, nph + 1, atoms)])
     groups = []
     for nleg, B in counts.items():
@@ -120,3 +124,70 @@ def test_drop_in_signal_with_and_without_scratch(dtype, nleg, B):
                                ref.data_ptr(), rr.data_ptr(), None, torch.cuda.current_stream().cuda_stream))
     _same(got, ref, TOL[dtype])
     assert torch.equal(rf, rr)
+
+
+def _grads(st, b, q, S, shared, g, s2):
+    """Fused backward's (grad_coords, grad_sigma2) from the one-kernel form's saved signals."""
+    from feffgpu_b200 import _lib
+    span, tspan = st._span(S), st._span(S, True)
+    NK = int(q.shape[0])
+    ps = st._paths_struct(b, b.coords, s2)
+    _, cc, rf, _ = _rows(st, b, q, S, False)
+    full = int(st._lib.fg_chi_reduce_backward_workspace(st._h, C.byref(ps), NK))
+    up = lambda v: (v + 255) // 256 * 256  # noqa: E731
+    least = 256 + up(b.n * st.E * 16) + up(b.n * 8) + up(b.n * 256)
+    ws = torch.empty(full if shared else least, dtype=torch.uint8, device="cuda")
+    gc = torch.empty_like(b.coords)
+    gs = torch.empty(b.n, dtype=torch.float64, device="cuda")
+    _lib.check(st._lib.fg_chi_reduce_backward(st._h, st.prec, C.byref(ps), NK, q.data_ptr(), S.data_ptr(),
+                                              span.data_ptr(), tspan.data_ptr(), g.data_ptr(), cc.data_ptr(),
+                                              rf.data_ptr(), gc.data_ptr(), gs.data_ptr(), ws.data_ptr(), ws.numel(),
+                                              torch.cuda.current_stream().cuda_stream))
+    return gc, gs, full > least
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case,iorder", [("cfg2_phase", 2), ("case_A014", 2), ("case_A009", 2), ("cfg2_phase", 1),
+                                         ("case_A014", 0)])
+@pytest.mark.parametrize("counts", [{3: 1}, {2: 7, 3: 33, 4: 5}, {9: 40, 8: 3, 2: 1}, {6: 1500, 5: 500, 2: 9}],
+                         ids=["one", "few", "long", "many"])
+def test_shared_adjoint_equals_one_kernel_adjoint(dtype, case, iorder, counts):
+    """The gradients of both forms: the shared one sums a class's derivative over the partial waves before a path's
+    weights meet it, the other the weighted terms, so they agree to the rounding of such sums (of order 100 terms: 1e-5
+    of the largest component in the mixed form, 1e-11 in FP64)."""
+    from feffgpu_b200 import GPUPathStage, PathBatch
+    from feffgpu_b200.pad import resample_phase
+    P = resample_phase(phase(case), np.linspace(0.0, 20.0, 131))
+    st = GPUPathStage(P, device="cuda", dtype=dtype, iorder=iorder)
+    b = PathBatch(_list(P.nph, counts, 7, seed=4), nrows=3, device="cuda")
+    q = torch.arange(1, 202, dtype=torch.float64, device="cuda") * 0.1
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    gen = torch.Generator("cuda").manual_seed(5)
+    g = torch.randn(3, 201, dtype=torch.float64, device="cuda", generator=gen)
+    s2 = 0.001 + 0.004 * torch.rand(b.n, dtype=torch.float64, device="cuda", generator=gen)
+    got, gs, offered = _grads(st, b, q, S, True, g, s2)
+    ref, rs, _ = _grads(st, b, q, S, False, g, s2)
+    assert offered
+    _same(got, ref, {torch.complex64: 1e-5, torch.complex128: 1e-11}[dtype])
+    assert torch.equal(gs, rs)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nleg,B", [(2, 5), (3, 1), (4, 700), (7, 5000)])
+def test_drop_in_adjoint_with_and_without_scratch(dtype, nleg, B):
+    from feffgpu_b200 import GPUPathStage, _lib
+    P = phase("case_A014")
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    c, ip, _, _ = _list(P.nph, {nleg: B}, 6, seed=6)[0]
+    c = torch.tensor(c, device="cuda", dtype=st.rdtype)
+    ip = torch.tensor(ip, device="cuda")
+    gen = torch.Generator("cuda").manual_seed(7)
+    g = torch.randn(B, st.E, 2, dtype=st.rdtype, device="cuda", generator=gen)
+    gr = torch.randn(B, dtype=st.rdtype, device="cuda", generator=gen)
+    got = st._cchi_backward(c, ip, torch.view_as_complex(g), gr)
+    ref = torch.empty_like(got)
+    ws = torch.empty(256, dtype=torch.uint8, device="cuda")
+    _lib.check(st._lib.fg_cchi_backward(st._h, st.prec, B, nleg, c.data_ptr(), int(dtype == torch.complex128),
+                                        ip.data_ptr(), g.data_ptr(), gr.data_ptr(), ref.data_ptr(), ws.data_ptr(), 256,
+                                        torch.cuda.current_stream().cuda_stream))
+    _same(got, ref, {torch.complex64: 1e-5, torch.complex128: 1e-11}[dtype])

@@ -17,6 +17,7 @@ import time
 import numpy as np
 import torch
 
+from . import _lib
 from .batch import PathBatch
 from .cell import as_cell, cell_words
 
@@ -28,9 +29,9 @@ class MinImage:
 
     def __init__(self, box, device):
         self.cell = as_cell(box)
-        self.words = None
+        self.words = self.cell18 = None
         if isinstance(self.cell, np.ndarray):
-            w = torch.as_tensor(cell_words(self.cell, np.float64), device=device)
+            w = self.cell18 = torch.as_tensor(cell_words(self.cell, np.float64), device=device).contiguous()
             self.words = (w[:9].reshape(3, 3), w[9:].reshape(3, 3))
 
     def __call__(self, rel: torch.Tensor) -> torch.Tensor:
@@ -57,6 +58,9 @@ class PathModel:
         for g in groups:
             a = torch.as_tensor(np.asarray(g[0]), dtype=torch.long)
             B, n = a.shape
+            if a.numel() and (int(a.min()) < -len(pos) or int(a.max()) >= len(pos)):
+                raise IndexError(f"atom index outside the {len(pos)} positions")
+            a = torch.where(a < 0, a + len(pos), a)
             rel = self.min_image(pos[a.to(dev)] - pos[a[:, :1].to(dev)]).cpu().numpy()
             bgroups.append((rel, g[1], g[2] if len(g) > 2 else None, g[3] if len(g) > 3 else None))
             pad = torch.cat([a, a[:, :1].expand(B, nleg_max - n)], 1)
@@ -64,7 +68,15 @@ class PathModel:
         self.batch = PathBatch(bgroups, nrows=nrows, device=dev)
         self.atoms = torch.cat(atoms).to(dev)
         legs = torch.arange(nleg_max, device=dev)
-        self.mask = (legs[None, :] < self.batch.nleg[:, None].long()).to(torch.float64)[:, :, None]
+        live = legs[None, :] < self.batch.nleg[:, None].long()
+        self.mask = live.to(torch.float64)[:, :, None]
+        # for every atom the path slots that hold it (fg_path_scatter), in path order
+        self.natoms = int(pos.shape[0])
+        slots = torch.nonzero(live.reshape(-1)).squeeze(1)
+        at = self.atoms.reshape(-1)[slots]
+        self.entry = slots[torch.sort(at, stable=True).indices].to(torch.int32)
+        self.entry_off = torch.zeros(self.natoms + 1, device=dev, dtype=torch.int64)
+        self.entry_off[1:] = torch.cumsum(torch.bincount(at, minlength=self.natoms), 0)[:self.natoms]
 
     def coords(self, pos: torch.Tensor) -> torch.Tensor:
         """(n, nleg_max, 3) relative coordinates of every path at positions pos (N, 3), differentiable."""
@@ -72,7 +84,36 @@ class PathModel:
         return self.min_image(rel) * self.mask
 
     def rows(self, pos: torch.Tensor, q: torch.Tensor, S: torch.Tensor, sigma2=None) -> torch.Tensor:
-        return self.stage.chi_reduce(self.batch, q, S, coords=self.coords(pos), sigma2=sigma2)
+        # FP64 positions on the stage's device go through the gather kernel and its fixed-order adjoint (fg_path_gather,
+        # fg_path_scatter), anything else through coords
+        fast = (torch.is_tensor(pos) and pos.device == self.stage.device and pos.dtype == torch.float64 and
+                tuple(pos.shape) == (self.natoms, 3) and self.batch.n * self.batch.nleg_max < 1 << 31)
+        coords = _Gather.apply(pos, self) if fast else self.coords(pos)
+        return self.stage.chi_reduce(self.batch, q, S, coords=coords, sigma2=sigma2)
+
+
+class _Gather(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, pos, model):
+        b, mi = model.batch, model.min_image
+        x = pos.detach().contiguous()
+        out = torch.empty(b.n, b.nleg_max, 3, device=x.device, dtype=torch.float64)
+        box = float(mi.cell) if mi.cell is not None and mi.cell18 is None else -1.0
+        _lib.check(_lib.load().fg_path_gather(b.n, b.nleg_max, x.data_ptr(), model.atoms.data_ptr(), b.nleg.data_ptr(),
+                                              box, None if mi.cell18 is None else mi.cell18.data_ptr(),
+                                              out.data_ptr(), torch.cuda.current_stream(x.device).cuda_stream))
+        ctx.model = model
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        m = ctx.model
+        g = g.contiguous()
+        out = torch.empty(m.natoms, 3, device=g.device, dtype=torch.float64)
+        _lib.check(_lib.load().fg_path_scatter(m.natoms, m.batch.nleg_max, m.entry_off.data_ptr(), m.entry.data_ptr(),
+                                               m.batch.nleg.data_ptr(), g.data_ptr(), out.data_ptr(),
+                                               torch.cuda.current_stream(g.device).cuda_stream))
+        return out, None
 
 
 def finder_groups(finder, positions, box, absorbers, ipot_of, weight=None):

@@ -341,6 +341,17 @@ FG_API fg_status fg_path_geometry_backward(int64_t B, int32_t nleg, const double
                                            const double *grad_beta, const double *grad_eta, double *grad_coords,
                                            void *stream);
 
+/* Coordinates (n, nleg_max, 3) FP64 of paths held as atom indices atoms (n, nleg_max), absorber first, at positions pos
+ * (N, 3) FP64: relative to the absorber under the minimum image (box: a cubic length, not positive for none; cell: the
+ * cell's rows and its inverse, 18 doubles, or NULL), zero at slots past nleg[p] (exafs/forward.py:664-725).  The indices
+ * are the caller's to keep within the positions. */
+FG_API fg_status fg_path_gather(int64_t n, int32_t nleg_max, const double *pos, const int64_t *atoms,
+                                const int32_t *nleg, double box, const double *cell, double *coords, void *stream);
+/* Its adjoint: grad_pos (natoms, 3) from grad_coords (n, nleg_max, 3).  off (natoms + 1) and entry: for every atom the
+ * slots p * nleg_max + j, j < nleg[p], that hold it; sums in a fixed order. */
+FG_API fg_status fg_path_scatter(int64_t natoms, int32_t nleg_max, const int64_t *off, const int32_t *entry,
+                                 const int32_t *nleg, const double *grad_coords, double *grad_pos, void *stream);
+
 /* ---------------------------------------------------------------------------------------------- R-space misfit
  * The loss of the refinement (src/feffgpu/exafs/transform.py:104-145): per row b of rows (B, NK) FP64,
  * R[b] = inv_norm * sum_m |(F x_b)_m - target_m|^2 with F (NR, NK) the windowed, k-weighted FFT restricted to the R

@@ -435,10 +435,10 @@ template <class F> fg_status by_kind(const fg_stage *s, fg_precision prec, F &&f
 }
 
 // Bytes of the shared form's workspace in the larger of the two precisions (0 where it does not apply)
-size_t share_bytes(const fg_stage *s, int64_t n, int nleg_max, bool adjoint = false)
+size_t share_bytes(const fg_stage *s, int64_t n, int nleg_max, bool adjoint = false, int NK = 0)
 {
-    return std::max(share_plan(n, nleg_max, s->E, s->L1, false, s->iorder, s->ilinit, adjoint).total,
-                    share_plan(n, nleg_max, s->E, s->L1, true, s->iorder, s->ilinit, adjoint).total);
+    return std::max(share_plan(n, nleg_max, s->E, s->L1, false, s->iorder, s->ilinit, adjoint, NK).total,
+                    share_plan(n, nleg_max, s->E, s->L1, true, s->iorder, s->ilinit, adjoint, NK).total);
 }
 
 // Host-side checks of a batch's sizes and pointers; k_validate checks the contents (indices) on the device and
@@ -558,7 +558,7 @@ extern "C" fg_status fg_chi_fine_backward(const fg_stage *s, fg_precision prec, 
 extern "C" size_t fg_chi_reduce_workspace(const fg_stage *s, const fg_paths *P, int32_t NK)
 {
     if (!s || !P || NK < 0) return 0;
-    return fused_workspace(P, NK) + share_bytes(s, P->n, P->nleg_max);
+    return fused_workspace(P, NK) + share_bytes(s, P->n, P->nleg_max, false, NK);
 }
 
 extern "C" fg_status fg_chi_reduce(const fg_stage *s, fg_precision prec, const fg_paths *P, int32_t NK,

@@ -30,16 +30,24 @@ constexpr int kBadRange = 4;    // a weighted path term not finite or beyond the
 // so the rows do not depend on the order in which paths finish, the launch shape or the GPU.  (Measured on B200:
 // 45.80 ms against 45.99 for per-path terms in memory summed in a fixed order afterwards on the 189,419-path benchmark
 // batch, 137.5 against 149.1 ms on the 4.2e6-path MD batch, and no workspace beyond the rows.)
-// Adds v to the fixed-point sum whose two words are a[0] and a[stride]; false (nothing added) if v is not finite or
-// |v| >= 2^31.
-__device__ __forceinline__ bool fixed_add(unsigned long long *a, size_t stride, double v)
+// Adds v to the fixed-point sum (hi, lo); false (nothing added) if v is not finite or |v| >= 2^31.
+__device__ __forceinline__ bool fixed_words(double v, unsigned long long &hi, unsigned long long &lo)
 {
     if (!(fabs(v) < 2147483648.0)) return false;
     const double x = v * 4294967296.0;                  // exact: v * 2^32, |x| < 2^63
-    const double hi = floor(x);
-    const double lo = rint((x - hi) * 4294967296.0);    // the next 32 bits, 0 <= lo <= 2^32; rounding below 2^-64
-    atomicAdd(a, (unsigned long long)(long long)hi);
-    atomicAdd(a + stride, (unsigned long long)lo);
+    const double h = floor(x);
+    const double l = rint((x - h) * 4294967296.0);      // the next 32 bits, 0 <= l <= 2^32; rounding below 2^-64
+    hi += (unsigned long long)(long long)h;
+    lo += (unsigned long long)l;
+    return true;
+}
+// The same for a sum in memory whose two words are a[0] and a[stride].
+__device__ __forceinline__ bool fixed_add(unsigned long long *a, size_t stride, double v)
+{
+    unsigned long long hi = 0, lo = 0;
+    if (!fixed_words(v, hi, lo)) return false;
+    atomicAdd(a, hi);
+    atomicAdd(a + stride, lo);
     return true;
 }
 

@@ -412,6 +412,62 @@ __device__ C2<R> energy_ms(const WarpPath<R> &g, const R *dh, const Tables<R> &T
     const C2<R> ptrac = termination<R, KIND>(g, T, e, nleg, ck, [&](int b, int a) { return P[b][a]; });
     return cmul(ptrac, cfac(g, T, e, nleg, ck));
 }
+// Three legs alone (k_stage_energies): with only a first and a last matrix in the kernel, each is accumulated as far as
+// it is read, the first one's columns and the last one's rows within the final state (14 of 20 canonical entries each at
+// the K edge, and one spherical-wave column less in the last), value for value as energy_ms forms them.
+template <typename R, int KIND>
+__device__ C2<R> energy_ms3(const WarpPath<R> &g, const R *dh, const Tables<R> &T, int e)
+{
+    constexpr LamTab L = lamtab(KIND);
+    constexpr int N = L.N, N0 = L.N0, MM = L.MM, DS = dstride(MM), UNR = sizeof(R) == 4 ? 2 : 1;
+    const int E = T.E;
+    const size_t tlip = (size_t)(T.L1 + 1) * E;
+    const C2<R> ck = T.ck[e];
+    if (fabs((double)ck.x) + fabs((double)ck.y) <= 1e-16) return cz<R>();
+    const C2<R> z2 = zfac(cscl(ck, (R)g.ri[2]));
+    C2<R> P[N][N0];
+    {
+        constexpr RepTab<KIND, N, N0> RT{};
+        C2<R> acc[RT.n];
+        const int ip = g.ip[1];
+        accumulate_f<R, KIND, N, N0, UNR>(acc, dh, T.tl + ip * tlip + e, E, T.lmax[ip * E + e] + 1, z2,
+                                          zfac(cscl(ck, (R)g.ri[1])));
+        mask_lambda<R, KIND, N, N0>(acc, T.nlam);
+        C2<R> ph[2 * MM + 1];
+        phase_powers<R, MM>(g.phs[2], ph);
+#pragma unroll
+        for (int a = 0; a < N; ++a)
+#pragma unroll
+            for (int b = 0; b < N0; ++b) {
+                const C2<R> v = acc[RT.rep[a][b]];
+                P[a][b] = cmul(ph[L.m[a] + MM], RT.sg[a][b] > 0 ? v : cscl(v, R(-1)));
+            }
+    }
+    constexpr RepTab<KIND, N0, N> RT{};
+    C2<R> acc[RT.n];
+    const int ip = g.ip[2];
+    accumulate_f<R, KIND, N0, N, UNR>(acc, dh + (size_t)(T.L1 + 1) * DS, T.tl + ip * tlip + e, E, T.lmax[ip * E + e] + 1,
+                                      zfac(cscl(ck, (R)g.ri[3])), z2);
+    mask_lambda<R, KIND, N0, N>(acc, T.nlam);
+    C2<R> ph[2 * MM + 1];
+    phase_powers<R, MM>(g.phs[3], ph);
+    C2<R> Q[N0][N0];
+#pragma unroll
+    for (int a = 0; a < N0; ++a)
+#pragma unroll
+        for (int b = 0; b < N0; ++b) {
+            C2<R> s = cz<R>();
+#pragma unroll
+            for (int c = 0; c < N; ++c) {
+                const C2<R> f = acc[RT.rep[a][c]];
+                s = RT.sg[a][c] > 0 ? cfma(f, P[c][b], s) : cfms(f, P[c][b], s);
+            }
+            Q[a][b] = cmul(ph[L.m[a] + MM], s);
+        }
+    const C2<R> ptrac = termination<R, KIND>(g, T, e, 3, ck, [&](int b, int a) { return Q[b][a]; });
+    return cmul(ptrac, cfac(g, T, e, 3, ck));
+}
+
 // Single scattering (nleg = 2), K edge: the six-entry set, flip-symmetric accumulation.
 template <typename R, int KIND>
 __device__ C2<R> energy_ss_sym(const WarpPath<R> &g, const R *dh, const Tables<R> &T, int e)

@@ -121,6 +121,8 @@ constexpr int kShareMin = 2;                               // least scatterers p
 constexpr int64_t kShareItems = 1 << 16;                   // (path, part of its energies) items that fill the chip
 constexpr int64_t kShareSub = 1 << 18;                     // paths per sub-batch (bounds the workspace)
 constexpr int64_t kShareWorth = 1 << 15;                   // (path, 32 energies) items worth looking for classes
+constexpr int64_t kStageWorth = 1 << 12;                   // (path, 32 energies) items from which the staged form pays
+constexpr int64_t kStageSub = 1 << 15;                     // paths per sub-batch of the staged form (its tables stay in L2)
 constexpr int64_t kShareSmall = 8192;                      // (path, 32 energies) items of a small call
 constexpr size_t kShareMatrixBytes = (size_t)1 << 30;      // the classes' matrices: 2e5 classes, 32 energies, FP32
 struct ShareHead {                      // counters of one sub-batch, in the workspace head
@@ -135,7 +137,7 @@ struct ShareIdx {
     const int *nlegs;            // null: every path has nleg_uniform legs
     int nleg_uniform;
     const int *order;            // null: 0..n-1
-    ShareKey *key;               // n * nsc_max keys
+    ShareKey *key;               // n * nsc_max keys (null: the staged form, which looks for no classes)
     int *slot_of;                // n * nsc_max hash slots
     unsigned *hash;              // owners (scatterer index, 0xffffffff: empty), hmask + 1 of them
     unsigned hmask;
@@ -153,14 +155,14 @@ fg_status launch_share_insert(const ShareIdx &s, cudaStream_t st);
 // sub-batch (0: the form does not apply).
 struct SharePlan {
     int64_t sub = 0, cls_cap = 0;
-    int nsc_max = 0, chunks = 0, passes = 0, split = 1, force = 0, mats = 1;
+    int nsc_max = 0, chunks = 0, passes = 0, split = 1, force = 0, mats = 1, staged = 0;
     unsigned hcap = 0;
     size_t rec = 0, key = 0, slot = 0, hash = 0, cls = 0, owner = 0, two = 0, tab = 0, F = 0, f_bytes = 0, sig = 0,
-           gpar = 0, total = 0;
+           gpar = 0, pts = 0, total = 0;
 };
 // adjoint: the plan of the backward calls (a class keeps its matrix and three derivatives, paths their parameter
 // gradients instead of signals)
-SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit, bool adjoint = false);
+SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit, bool adjoint = false, int NK = 0);
 
 // Events around the main kernel of a call when kernel timing is on (fg_set_kernel_timing)
 void timer_begin(cudaStream_t st);

@@ -27,13 +27,13 @@ Share<R> share_view(const SharePlan &pl, unsigned char *ws, ShareHead *head, con
 {
     Share<R> s{};
     s.rec = ws + pl.rec; s.rec_bytes = geo_bytes<R>();
-    s.key = reinterpret_cast<ShareKey *>(ws + pl.key);
+    s.key = pl.staged ? nullptr : reinterpret_cast<ShareKey *>(ws + pl.key);
     s.slot_of = reinterpret_cast<int *>(ws + pl.slot);
     s.hash = reinterpret_cast<unsigned *>(ws + pl.hash); s.hmask = pl.hcap - 1;
     s.cls = reinterpret_cast<int *>(ws + pl.cls);
     s.owner = reinterpret_cast<unsigned *>(ws + pl.owner); s.cls_cap = pl.cls_cap;
     s.two = reinterpret_cast<int *>(ws + pl.two);
-    s.tab = reinterpret_cast<R *>(ws + pl.tab); s.tab_len = (L1 + 1) * dstride(lamtab(Kinds<EDGE>::MS).MM);
+    s.tab = reinterpret_cast<R *>(ws + pl.tab); s.tab_len = (L1 + 1) * dstride(pl.staged ? Kinds<EDGE>::MM : lamtab(Kinds<EDGE>::MS).MM);
     s.F = ws + pl.F; s.f_bytes = pl.f_bytes;
     s.chunks = pl.chunks; s.mats = pl.mats; s.force = pl.force; s.nsc_max = pl.nsc_max;
     s.head = head; s.status = status;
@@ -47,8 +47,8 @@ template <typename R, int EDGE> struct ShareLaunch {
     static fg_status signals(const StageView &sv, const Tables<R> &T, const SharePlan &pl, Share<R> &s, const CT *coords,
                              const int64_t *ipots, int *status, C2<R> *out, cudaStream_t st);
     static fg_status fine(const StageView &sv, const Share<R> &s, const PathsDev &pd, int NK, const double *q,
-                          const double *S, const int *span, const C2<R> *sig, unsigned long long *racc,
-                          double *reff_save, int *status, cudaStream_t st);
+                          const double *S, const int *span, unsigned char *pts, bool first, const C2<R> *sig,
+                          unsigned long long *racc, double *reff_save, int *status, cudaStream_t st);
     static fg_status reff(const Share<R> &s, R *out, cudaStream_t st);
     template <typename CT>
     static fg_status adjoint(const StageView &sv, const Tables<R> &T, const SharePlan &pl, Share<R> &s, unsigned char *ws,
@@ -132,7 +132,7 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
         FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes + row_sum_bytes(P->nrows, NK), st));
     }
     if (fg_status rc = launch_validate(P, sv.nph1, status, st)) return rc;
-    const SharePlan pl = P->n > 0 ? share_plan(P->n, P->nleg_max, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit) : SharePlan{};
+    const SharePlan pl = P->n > 0 ? share_plan(P->n, P->nleg_max, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit, false, NK) : SharePlan{};
     if (pl.sub && share_ws && share_bytes >= pl.total) {
         if constexpr (EDGE <= 3) {
             ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
@@ -148,7 +148,8 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
                                                                                   sig, st))
                     return rc;
                 const PathsDev pd{s.n, P->nleg_max, P->nrows, P->coords, P->ipots, P->nleg, P->deg, P->sigma2, s.order, P->row};
-                if (fg_status rc = ShareLaunch<R, EDGE>::fine(sv, s, pd, NK, q, S, span, sig, racc, reff_save, status, st))
+                if (fg_status rc = ShareLaunch<R, EDGE>::fine(sv, s, pd, NK, q, S, span, share_ws + pl.pts, t0 == 0, sig, racc,
+                                                              reff_save, status, st))
                     return rc;
                 if (!pl.force) {
                     if (t0) FG_CUDA(cudaMemsetAsync(counter, 0, sizeof(*counter), st));

@@ -54,7 +54,7 @@ fg_status launch_share_insert(const ShareIdx &s, cudaStream_t st)
     return FG_OK;
 }
 
-SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit, bool adjoint)
+SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iorder, int ilinit, bool adjoint, int NK)
 {
     SharePlan p;
     if (iorder > 2 || n < 1) return p;
@@ -67,11 +67,29 @@ SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iord
     // up to four legs, 1.27 scatterers per class, looking for them cost 5 %.
     const int chunks = (E + 31) / 32;
     const bool small = n * chunks <= kShareSmall && (chunks >= 4 || ilinit > 1);
-    if (!small && (nleg_max < 4 || (chunks < 4 && n * chunks <= kShareWorth))) return p;
+    // What is left and large enough takes the staged form (4,438 paths on 60 energies 1.35 -> 1.08 ms a refinement step,
+    // its rows' sums in shared memory then another 0.05; at 396 paths its launches cost what it gains).
+    const bool classes = small || (nleg_max >= 4 && (chunks >= 4 || n * chunks > kShareWorth));
+    p.staged = !adjoint && !classes && n * chunks > kStageWorth;
+    if (!classes && !p.staged) return p;
     const size_t real = fp64 ? 8 : 4;
-    p.sub = std::min<int64_t>(n, kShareSub);
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += align_up(bytes, 256); return o; };
+    const size_t rec = align_up(fp64 ? sizeof(WarpPath<double>) : sizeof(WarpPath<float>), 16);
     p.nsc_max = nleg_max - 1;
     p.chunks = chunks;
+    p.pts = take((size_t)NK * 32);
+    if (p.staged) {
+        p.sub = std::min<int64_t>(n, kStageSub);
+        p.force = p.passes = 1;
+        p.split = (int)std::min<int64_t>(chunks, (kShareItems / 4 + p.sub - 1) / p.sub);
+        p.rec = take((size_t)p.sub * rec);
+        p.tab = take((size_t)p.sub * p.nsc_max * (L1 + 1) * dstride(3) * real);
+        p.sig = take((size_t)p.sub * E * 2 * real);
+        p.total = at;
+        return p;
+    }
+    p.sub = std::min<int64_t>(n, kShareSub);
     const int64_t scat = p.sub * p.nsc_max;
     p.mats = adjoint ? 4 : 1;
     const size_t per = p.mats * 20 * 2 * real * 32;          // one class, one chunk: 20 canonical entries (orders 0-2)
@@ -86,9 +104,6 @@ SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iord
     p.split = (int)std::min<int64_t>(chunks, (kShareItems + p.sub - 1) / p.sub);
     p.hcap = 64;
     while ((int64_t)p.hcap < 2 * scat) p.hcap *= 2;
-    size_t at = 0;
-    auto take = [&](size_t bytes) { const size_t o = at; at += align_up(bytes, 256); return o; };
-    const size_t rec = align_up(fp64 ? sizeof(WarpPath<double>) : sizeof(WarpPath<float>), 16);
     const size_t ext = align_up(fp64 ? sizeof(AdjExtra<double>) : sizeof(AdjExtra<float>), 16);
     p.rec = take((size_t)p.sub * (adjoint ? rec + ext : rec));
     p.key = take((size_t)scat * sizeof(ShareKey));

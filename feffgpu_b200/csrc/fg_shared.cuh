@@ -222,6 +222,12 @@ __device__ __forceinline__ void copy16(void *dst, const void *src, size_t bytes,
     for (size_t i = lane; i < bytes / 16; i += 32) static_cast<uint4 *>(dst)[i] = static_cast<const uint4 *>(src)[i];
 }
 
+template <typename R> __device__ __forceinline__ ShareKey share_key(const WarpPath<R> &g, int k)
+{
+    return ShareKey{(unsigned long long)__double_as_longlong(g.ri[k]), (unsigned long long)__double_as_longlong(g.ri[k + 1]),
+                    (unsigned long long)__double_as_longlong(g.beta[k]), (unsigned long long)g.ip[k]};
+}
+
 // The keys of path i's scatterers, or its entry in the list of two-leg paths
 template <typename R>
 __device__ __forceinline__ void share_keys(const Share<R> &s, const WarpPath<R> &g, int64_t i, int nleg, int lane)
@@ -229,30 +235,88 @@ __device__ __forceinline__ void share_keys(const Share<R> &s, const WarpPath<R> 
     if (nleg == 2) {
         if (lane == 0) s.two[atomicAdd(&s.head->two, 1)] = (int)i;
     } else if (lane >= 1 && lane < nleg) {
-        s.key[i * s.nsc_max + lane - 1] = ShareKey{(unsigned long long)__double_as_longlong(g.ri[lane]),
-                                                   (unsigned long long)__double_as_longlong(g.ri[lane + 1]),
-                                                   (unsigned long long)__double_as_longlong(g.beta[lane]),
-                                                   (unsigned long long)g.ip[lane]};
+        s.key[i * s.nsc_max + lane - 1] = share_key(g, lane);
     }
 }
 
-// Records, keys and the list of two-leg paths (a batch that k_validate refused is left alone).
+// Records, keys and the list of two-leg paths (a batch that k_validate refused is left alone).  A block takes PB paths
+// at a time, a thread per (path, leg) where path_setup has a warp per path with a lane per leg: same operations, most of
+// the lanes busy (128,844 paths of up to eight legs: 134 us, 292 us with a warp per path).
 template <typename R, typename CT>
 __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, const CT *__restrict__ coords,
-                                                    const int64_t *__restrict__ ipots, int *status, int MM_ss, int MM_ms)
+                                                    const int64_t *__restrict__ ipots, int *status, int PB)
 {
     if (status && (*(volatile const int *)status & kBadLayout)) return;
     extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    WarpPath<R> &g = *reinterpret_cast<WarpPath<R> *>(smem + (size_t)w * s.rec_bytes);
-    for (int64_t i = (int64_t)blockIdx.x * 4 + w; i < s.n; i += (int64_t)gridDim.x * 4) {
-        const int64_t p = s.path(i);
-        const int nleg = s.legs(p);
-        path_setup<R, CT>(g, nullptr, T, coords + p * s.stride * 3, ipots + p * s.stride, nleg, lane, status,
-                          nleg == 2 ? MM_ss : MM_ms, false);
-        copy16(s.rec + i * s.rec_bytes, &g, s.rec_bytes, lane);
-        share_keys(s, g, i, nleg, lane);
-        __syncwarp();
+    double *half = reinterpret_cast<double *>(smem + (size_t)PB * s.rec_bytes);      // cos, sin of beta_nleg / 2
+    const int tid = threadIdx.x, nl = s.nsc_max + 1;
+    auto rec = [&](int l) -> WarpPath<R> & { return *reinterpret_cast<WarpPath<R> *>(smem + (size_t)l * s.rec_bytes); };
+    for (int64_t i0 = (int64_t)blockIdx.x * PB; i0 < s.n; i0 += (int64_t)gridDim.x * PB) {
+        const int cnt = (int)min((int64_t)PB, s.n - i0);
+        for (int t = tid; t < cnt * nl * 3; t += 128) {
+            const int l = t / (3 * nl), r = t % (3 * nl);
+            const int64_t p = s.path(i0 + l);
+            if (r < 3 * s.legs(p)) rec(l).xyz[r / 3][r % 3] = (double)coords[p * s.stride * 3 + r] / kBohr;
+        }
+        for (int t = tid; t < cnt * (nl + 1); t += 128) {
+            const int l = t / (nl + 1), j = t % (nl + 1);
+            const int64_t p = s.path(i0 + l);
+            const int nleg = s.legs(p);
+            if (j > nleg) continue;
+            int64_t v = ipots[p * s.stride + (j == nleg ? 0 : j)];
+            if (v < 0 || v >= T.nph1) {
+                if (status) atomicOr(status, kBadIpot);
+                v = v < 0 ? 0 : T.nph1 - 1;
+            }
+            rec(l).ip[j] = (int)v;
+        }
+        __syncthreads();
+        for (int t = tid; t < cnt * nl; t += 128) {
+            const int l = t / nl, j = t % nl + 1, nleg = s.legs(s.path(i0 + l));
+            if (j > nleg) continue;
+            WarpPath<R> &g = rec(l);
+            auto rat = [&](int i, double *o) {
+                const int a = (i == 0 || i == nleg) ? 0 : i;
+                o[0] = g.xyz[a][0]; o[1] = g.xyz[a][1]; o[2] = g.xyz[a][2];
+            };
+            const LegGeom lg = leg_geometry<double>(rat, j, nleg);
+            g.ri[j] = lg.ri; g.beta[j] = lg.beta; g.alpha[j] = lg.alpha; g.gamma[j] = lg.gamma;
+            if (j == nleg) {
+                half[2 * l] = cos(0.5 * lg.beta);
+                half[2 * l + 1] = sin(0.5 * lg.beta);
+            }
+        }
+        __syncthreads();
+        for (int t = tid; t < cnt * nl; t += 128) {
+            const int l = t / nl, j = t % nl + 1, nleg = s.legs(s.path(i0 + l));
+            if (j > nleg) continue;
+            WarpPath<R> &g = rec(l);
+            const double eta = g.alpha[j == 1 ? nleg : j - 1] + g.gamma[j];
+            double sn, cs;
+            sincos(eta, &sn, &cs);
+            g.phs[j] = C2<R>{(R)cs, (R)(-sn)};
+            if (j == 1) {
+                double r = 0.0;
+                for (int q = 1; q <= nleg; ++q) r += g.ri[q];
+                g.reff = 0.5 * r;
+            }
+            if (s.key) {
+                if (nleg == 2) {
+                    if (j == 1) s.two[atomicAdd(&s.head->two, 1)] = (int)(i0 + l);
+                } else if (j < nleg) {
+                    s.key[(i0 + l) * s.nsc_max + j - 1] = share_key(g, j);
+                }
+            }
+        }
+        for (int t = tid; t < cnt * T.nterm * 49; t += 128) {
+            const int l = t / (T.nterm * 49), q = t % (T.nterm * 49), e = q % 49;
+            rec(l).dterm[q / 49][e] = (R)wigner_small(T.term_l[q / 49], e / 7 - 3, e % 7 - 3, half[2 * l], half[2 * l + 1],
+                                                      seed_table(T));
+        }
+        __syncthreads();
+        for (size_t t = tid; t < cnt * s.rec_bytes / 16; t += 128)
+            reinterpret_cast<uint4 *>(s.rec + i0 * s.rec_bytes)[t] = reinterpret_cast<const uint4 *>(smem)[t];
+        __syncthreads();
     }
 }
 
@@ -386,32 +450,196 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 2)
     }
 }
 
-// Fine grid and exact row sums of the fused calls from the paths' signals, as k_fused forms them.
-template <typename R, int KIND>
-__global__ void __launch_bounds__(128) k_share_fine(Share<R> s, PathsDev P, int E, int NK, const double *__restrict__ q,
-                                                    const double *__restrict__ S, const int *__restrict__ span,
-                                                    const C2<R> *__restrict__ cchi, unsigned long long *__restrict__ racc,
-                                                    double *__restrict__ reff_save, int *status, size_t wbytes)
+// ------------------------------------------------------------------------------------------------ staged form
+// Lists of up to three legs (MD trajectories) share nothing, but k_fused spends more than half its time there on what is
+// done once per path -- geometry, rotation tables, the fine grid -- at the eight warps per SM that its energy loop allows.
+// The staged form gives each part a kernel of its own shape: k_share_geom, the tables by a thread per (scatterer, entry)
+// into the workspace, the energies by a warp per path with record and tables copied in, then k_share_fine.  537,000 paths
+// of 2,048 absorbers, 60 energies, 401 points, mixed: 15.0 -> 9.5 ms (energies 5.5, fine grid 1.9, tables 1.1, geometry
+// 0.7 ms); 4,438 paths of up to four legs: 178 -> 140 us.  What bounds it: the energies' FP32 multiply-adds and their
+// fixed latencies at 12 (three legs) and 8 warps per SM.
+template <typename R, int EDGE> __global__ void __launch_bounds__(128) k_stage_tables(Tables<R> T, Share<R> s)
 {
-    if (s.refused() || !share_chunks<R, KIND>(s)) return;
+    using K = Kinds<EDGE>;
+    constexpr int NC = ncanon(K::MM);
+    if (s.refused()) return;
+    const int64_t tasks = s.n * s.nsc_max * NC;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tasks; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t c = t / NC, i = c / s.nsc_max;
+        const int r = (int)(t % NC), k = (int)(c % s.nsc_max) + 1, nleg = s.legs(s.path(i));
+        const int MM = nleg == 2 ? K::MMSS : K::MMMS;
+        if (k >= nleg || r >= ncanon(MM)) continue;
+        const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(s.rec + i * s.rec_bytes);
+        rotation_column<R>(s.tab + c * s.tab_len, T, g.beta[k], MM, dstride(MM), r);
+    }
+}
+
+// SHORT: no path has more than three legs
+template <typename R, int EDGE, bool SHORT>
+__global__ void __launch_bounds__(128, FusedMinBlocks<R>::def) k_stage_energies(Tables<R> T, Share<R> s, int split,
+                                                                                C2<R> *__restrict__ out, size_t wbytes)
+{
+    using K = Kinds<EDGE>;
+    if (s.refused()) return;
     extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double *pha = reinterpret_cast<double *>(smem + (size_t)w * wbytes);
-    double *amp = pha + align_up((size_t)E, 2);
-    for (int64_t i = (int64_t)blockIdx.x * nw + w; i < s.n; i += (int64_t)gridDim.x * nw) {
-        const int64_t p = s.path(i);
-        const C2<R> *c = cchi + (s.by_path ? p : i) * E;
-        const double rf = reinterpret_cast<const WarpPath<R> *>(s.rec + i * s.rec_bytes)->reff * kBohr;
-        path_terms<R>(P, p, E, NK, lane, q, S, span, [&](int e) { return c[e]; }, amp, pha, rf, racc, status);
-        if (lane == 0 && reff_save) reff_save[p] = rf;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, E = T.E;
+    unsigned char *base = smem + (size_t)w * wbytes;
+    const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(base);
+    R *dh = reinterpret_cast<R *>(base + s.rec_bytes);
+    for (int64_t it = (int64_t)blockIdx.x * nw + w; it < s.n * split; it += (int64_t)gridDim.x * nw) {
+        const int64_t i = it / split, o = s.row(i) * E;
+        const int nleg = s.legs(s.path(i)), MM = nleg == 2 ? K::MMSS : K::MMMS;
+        copy16(base, s.rec + i * s.rec_bytes, s.rec_bytes, lane);
+        // the tables of a path's scatterers, one after the other as the energies read them
+        const int len = (T.L1 + 1) * dstride(MM);
+        for (int k = 0; k < nleg - 1; ++k)
+            copy16(dh + k * len, s.tab + (i * s.nsc_max + k) * s.tab_len, (size_t)len * sizeof(R), lane);
         __syncwarp();
+        for (int gc = (int)(it % split); gc < s.chunks; gc += split) {
+            const int e = first_chunk(E) + 32 * gc + lane;
+            if (e < 0 || e >= E) continue;
+            if (nleg > 2) {
+                if constexpr (SHORT) out[o + e] = energy_ms3<R, K::MS>(g, dh, T, e);
+                else out[o + e] = energy_ms<R, K::MS>(g, dh, T, e, nleg);
+            } else {
+                if constexpr (K::SS_SYM) out[o + e] = energy_ss_sym<R, K::SS>(g, dh, T, e);
+                else out[o + e] = energy_ss_col<R, K::SS>(g, dh, T, e);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// A fine-grid point's interpolation: the weights of its first two energies (S rows with more are read from S)
+struct __align__(16) FinePoint {
+    double w0, w1, q;
+    int lo, n;
+};
+static __global__ void k_fine_points(int NK, int E, const double *__restrict__ q, const double *__restrict__ S,
+                              const int *__restrict__ span, FinePoint *__restrict__ out)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= NK) return;
+    FinePoint f;
+    f.lo = span[2 * k];
+    f.n = span[2 * k + 1] - f.lo;
+    f.q = q[k];
+    f.w0 = f.n > 0 ? S[(size_t)k * E + f.lo] : 0.0;
+    f.w1 = f.n > 1 ? S[(size_t)k * E + f.lo + 1] : 0.0;
+    out[k] = f;
+}
+
+// Fine grid and exact row sums of the fused calls from the paths' signals, value for value as k_fused forms them
+// (path_terms).  A warp takes a contiguous range of the sub-batch's paths, PG at a time, so that a fine-grid point's
+// interpolation is read once for all of them.  Integer sums give the same in any order: with ACC the terms of one row are
+// added in the warp's shared memory, and only its sums go to the row's words, those of neighbouring warps first added
+// together -- a row's 401 points take one addition each per block and not per path, which is what a small batch on one row
+// waits for: 4,438 paths on 60 energies 84 -> 25 us; 537,000 paths on 64 rows 2.29 -> 1.94 ms (4.3 ms a warp per path with
+// S read in place).  On 401 energies (128,844 paths, 1.29 ms) the FP64 arc tangents and square roots of the phases bound it.
+template <typename R, int KIND, int PG, bool ACC>
+__global__ void __launch_bounds__(256) k_share_fine(Share<R> s, PathsDev P, int E, int NK, const double *__restrict__ S,
+                                                    const FinePoint *__restrict__ pts, const C2<R> *__restrict__ cchi,
+                                                    unsigned long long *__restrict__ racc,
+                                                    double *__restrict__ reff_save, int *status, int64_t range,
+                                                    size_t wbytes)
+{
+    if (s.refused() || (s.key && !share_chunks<R, KIND>(s))) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int last_row[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, E2 = (E + 1) & ~1;
+    auto words = [&](int v) {
+        return reinterpret_cast<ulonglong2 *>(smem + (size_t)v * wbytes + (size_t)2 * PG * E2 * sizeof(double));
+    };
+    double *pha = reinterpret_cast<double *>(smem + (size_t)w * wbytes), *amp = pha + PG * E2;
+    const size_t stride = (size_t)P.nrows * NK;
+    auto add = [&](int row, int k, unsigned long long hi, unsigned long long lo) {
+        atomicAdd(racc + (size_t)row * NK + k, hi);
+        atomicAdd(racc + (size_t)row * NK + k + stride, lo);
+    };
+    const int64_t lo_i = min(s.n, ((int64_t)blockIdx.x * nw + w) * range), hi_i = min(s.n, lo_i + range);
+    int cur = -1;                                    // the row whose terms the warp's words hold (ACC)
+    for (int64_t i0 = lo_i; i0 < hi_i; i0 += PG) {
+        const int cnt = (int)min((int64_t)PG, hi_i - i0);
+        double rf[PG], wdeg[PG], s2[PG];
+        int row[PG];
+#pragma unroll
+        for (int j = 0; j < PG; ++j) {
+            if (j >= cnt) break;
+            const int64_t p = s.path(i0 + j);
+            const C2<R> *c = cchi + (s.by_path ? p : i0 + j) * E;
+            amp_phase<R>(E, lane, [&](int e) { return c[e]; }, amp + j * E2, pha + j * E2);
+            rf[j] = reinterpret_cast<const WarpPath<R> *>(s.rec + (i0 + j) * s.rec_bytes)->reff * kBohr;
+            wdeg[j] = P.deg[p];
+            s2[j] = P.sigma2 ? P.sigma2[p] : 0.0;
+            row[j] = P.row[p];
+            if (lane == 0 && reff_save) reff_save[p] = rf[j];
+        }
+        __syncwarp();
+        int next = cur;
+        for (int k0 = 0; k0 < NK; k0 += 32) {
+            const int k = k0 + lane;
+            next = cur;
+            if (k < NK) {
+                const FinePoint f = pts[k];
+                unsigned long long hi = 0, lo = 0;
+                if (ACC && cur >= 0) {
+                    const ulonglong2 v = words(w)[k];
+                    hi = v.x;
+                    lo = v.y;
+                }
+#pragma unroll
+                for (int j = 0; j < PG; ++j) {
+                    if (j >= cnt) break;
+                    if (row[j] != next) {            // the sums so far go to their row
+                        if (next >= 0) add(next, k, hi, lo);
+                        hi = lo = 0;
+                        next = row[j];
+                    }
+                    const double *a_ = amp + j * E2 + f.lo, *p_ = pha + j * E2 + f.lo;
+                    double a = 0.0, ph = 0.0;
+                    if (f.n <= 2) {
+                        if (f.n > 0) { a += f.w0 * a_[0]; ph += f.w0 * p_[0]; }
+                        if (f.n > 1) { a += f.w1 * a_[1]; ph += f.w1 * p_[1]; }
+                    } else {
+                        for (int m = 0; m < f.n; ++m) {
+                            const double sv = S[(size_t)k * E + f.lo + m];
+                            a += sv * a_[m];
+                            ph += sv * p_[m];
+                        }
+                    }
+                    const double damp = s2[j] != 0.0 ? exp(-2.0 * s2[j] * f.q * f.q) : 1.0;   // exact 1 without sigma^2
+                    const double v = wdeg[j] * a * sin_arg<R>(ph + 2.0 * f.q * rf[j]) * damp;
+                    if (!fixed_words(v, hi, lo)) atomicOr(status, kBadRange);
+                }
+                if (ACC) words(w)[k] = make_ulonglong2(hi, lo);
+                else add(next, k, hi, lo);
+            }
+        }
+        if (ACC) cur = row[cnt - 1];
+        __syncwarp();
+    }
+    if (!ACC) return;
+    if (lane == 0) last_row[w] = cur;
+    __syncthreads();
+    for (int k = threadIdx.x; k < NK; k += blockDim.x) {
+        unsigned long long hi = 0, lo = 0;
+        for (int v = 0; v < nw; ++v) {
+            if (last_row[v] < 0) continue;
+            const ulonglong2 x = words(v)[k];
+            hi += x.x;
+            lo += x.y;
+            if (v + 1 == nw || last_row[v + 1] != last_row[v]) {
+                add(last_row[v], k, hi, lo);
+                hi = lo = 0;
+            }
+        }
     }
 }
 
 // reff of the drop-in call from the records
 template <typename R, int KIND> __global__ void k_share_reff(Share<R> s, R *__restrict__ reff)
 {
-    if (!share_chunks<R, KIND>(s)) return;
+    if (s.key && !share_chunks<R, KIND>(s)) return;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < s.n; p += (int64_t)gridDim.x * blockDim.x)
         reff[p] = (R)(reinterpret_cast<const WarpPath<R> *>(s.rec + p * s.rec_bytes)->reff * kBohr);
 }
@@ -424,11 +652,33 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
 {
     using K = Kinds<EDGE>;
     constexpr int KIND = K::MS;
-    FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
-    FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
-    const int blocks = (int)std::min<int64_t>((s.n + 3) / 4, (int64_t)sv.num_sms * 16);
-    k_share_geom<R, CT><<<blocks, 128, 4 * s.rec_bytes, st>>>(T, s, coords, ipots, status, K::MMSS, K::MMMS);
+    if (!pl.staged) {
+        FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
+        FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
+    }
+    // paths per block of the geometry: a thread per leg, fewer where the paths do not fill the chip that way
+    const int PB = (int)std::max<int64_t>(1, std::min<int64_t>(128 / (s.nsc_max + 1), s.n / (sv.num_sms * 4)));
+    const size_t gb = PB * (s.rec_bytes + 16);
+    int blocks = 0;
+    auto kg = k_share_geom<R, CT>;
+    if (fg_status rc = grid_for(kg, 128, gb, sv.num_sms, (s.n + PB - 1) / PB * 4, blocks)) return rc;
+    kg<<<blocks, 128, gb, st>>>(T, s, coords, ipots, status, PB);
     FG_CUDA(cudaGetLastError());
+    if (pl.staged) {
+        const int64_t tasks = s.n * s.nsc_max * ncanon(K::MM);
+        k_stage_tables<R, EDGE><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
+        FG_CUDA(cudaGetLastError());
+        auto ke = s.nsc_max <= 2 ? k_stage_energies<R, EDGE, true> : k_stage_energies<R, EDGE, false>;
+        const size_t wb = s.rec_bytes + align_up((size_t)s.nsc_max * s.tab_len * sizeof(R), 16);
+        const int ew = fit_warps(4, wb, sv.max_smem);
+        int eb = 0;
+        if (fg_status rc = grid_for(ke, 32 * ew, wb * ew, sv.num_sms, s.n * pl.split, eb)) return rc;
+        timer_begin(st);
+        ke<<<eb, 32 * ew, wb * ew, st>>>(T, s, pl.split, out, wb);
+        timer_end(st);
+        FG_CUDA(cudaGetLastError());
+        return FG_OK;
+    }
     if (fg_status rc = launch_share_insert(s, st)) return rc;
     const int64_t tasks = std::min<int64_t>(s.n * s.nsc_max, s.cls_cap) * ncanon(K::MMMS);
     k_share_tables<R, KIND><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
@@ -441,11 +691,12 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
     int fb = 0, cb = 0;
     if (fg_status rc = grid_for(kf, 32 * fw, wb * fw, sv.num_sms, s.n * s.nsc_max * pl.chunks, fb)) return rc;
     const int split = pl.split;
-    if (fg_status rc = grid_for(kc, 128, 4 * s.rec_bytes, sv.num_sms, s.n * split, cb)) return rc;
+    const size_t wc = 4 * s.rec_bytes;
+    if (fg_status rc = grid_for(kc, 128, wc, sv.num_sms, s.n * split, cb)) return rc;
     timer_begin(st);
     for (int pass = 0; pass < pl.passes; ++pass) {
         kf<<<fb, 32 * fw, wb * fw, st>>>(T, s, pass, out, wb);
-        kc<<<cb, 128, 4 * s.rec_bytes, st>>>(T, s, pass, split, out);
+        kc<<<cb, 128, wc, st>>>(T, s, pass, split, out);
     }
     timer_end(st);
     FG_CUDA(cudaGetLastError());
@@ -454,15 +705,23 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
 
 template <typename R, int EDGE>
 fg_status ShareLaunch<R, EDGE>::fine(const StageView &sv, const Share<R> &s, const PathsDev &pd, int NK, const double *q,
-                                     const double *S, const int *span, const C2<R> *sig, unsigned long long *racc,
-                                     double *reff_save, int *status, cudaStream_t st)
+                                     const double *S, const int *span, unsigned char *pts, bool first, const C2<R> *sig,
+                                     unsigned long long *racc, double *reff_save, int *status, cudaStream_t st)
 {
-    auto kern = k_share_fine<R, Kinds<EDGE>::MS>;
-    const size_t wb = 2 * align_up((size_t)sv.E * sizeof(double), 16);
-    const int warps = fit_warps(4, wb, sv.max_smem);
+    FinePoint *fp = reinterpret_cast<FinePoint *>(pts);
+    if (first) k_fine_points<<<(NK + 127) / 128, 128, 0, st>>>(NK, sv.E, q, S, span, fp);
+    // Four paths at a time where their amplitudes and phases are small (537,000 paths, 60 energies: 2.3 ms, two at a time
+    // 2.6) and there are paths enough; the rows' sums in shared memory up to 1,024 points.
+    const bool four = sv.E <= 128 && s.n >= (int64_t)sv.num_sms * 64, acc = NK <= 1024;
+    using K = Kinds<EDGE>;
+    auto kern = four ? (acc ? k_share_fine<R, K::MS, 4, true> : k_share_fine<R, K::MS, 4, false>)
+                     : (acc ? k_share_fine<R, K::MS, 1, true> : k_share_fine<R, K::MS, 1, false>);
+    const size_t wb = (size_t)2 * (four ? 4 : 1) * ((sv.E + 1) & ~1) * sizeof(double) + (acc ? (size_t)NK * 16 : 0);
+    const int warps = fit_warps(8, wb, sv.max_smem / 2);
     int blocks = 0;
     if (fg_status rc = grid_for(kern, 32 * warps, wb * warps, sv.num_sms, s.n, blocks)) return rc;
-    kern<<<blocks, 32 * warps, wb * warps, st>>>(s, pd, sv.E, NK, q, S, span, sig, racc, reff_save, status, wb);
+    const int64_t range = (s.n + (int64_t)blocks * warps - 1) / ((int64_t)blocks * warps);
+    kern<<<blocks, 32 * warps, wb * warps, st>>>(s, pd, sv.E, NK, S, fp, sig, racc, reff_save, status, range, wb);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
@@ -863,8 +1122,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 2) k_share_chain_adj
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned char *base = smem + (size_t)w * s.rec_bytes;
     const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(base);
+    // all paths of one part of the energies, then the next: the classes of neighbouring paths over few energies stay in L2
     for (int64_t it = (int64_t)blockIdx.x * 4 + w; it < s.n * split; it += (int64_t)gridDim.x * 4) {
-        const int64_t i = it / split, p = s.path(i);
+        const int part = (int)(it / s.n);
+        const int64_t i = it % s.n, p = s.path(i);
         const int nleg = s.legs(p);
         if (nleg == 2) continue;
         copy16(base, s.rec + i * s.rec_bytes, s.rec_bytes, lane);
@@ -872,15 +1133,16 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 2) k_share_chain_adj
         __syncwarp();
         ParGrad pg;
         for (int j = 0; j <= kMaxLeg; ++j) pg.ri[j] = pg.beta[j] = pg.eta[j] = 0.0;
-        for (int gc = (int)(it % split); gc < ng; gc += split) {
+        for (int gc = part; gc < ng; gc += split) {
             const int e = first_chunk(E) + 32 * (g0 + gc) + lane;
             if (e >= 0 && e < E)
                 shared_energy_adj<R, KIND>(
                     g, adj_extra<R>(base).dterm_db, T, e, nleg, lane, gbar[p * E + e],
-                    [&](int k) { return s.F + ((int64_t)cls_sh[w][k - 1] * G + gc) * 4 * f_chunk_bytes<R, KIND>(); }, pg);
+                    [&](int k) { return s.F + ((int64_t)cls_sh[w][k - 1] * G + gc) * 4 * f_chunk_bytes<R, KIND>(); },
+                    pg);
             __syncwarp();
         }
-        store_par(gpar + ((it % split) * s.n + i) * kGparStride, pg, nleg, lane, pass == 0);
+        store_par(gpar + (part * s.n + i) * kGparStride, pg, nleg, lane, pass == 0);
         __syncwarp();
     }
 }
@@ -989,7 +1251,8 @@ fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T,
     const int nf = fit_warps(4, wf, sv.max_smem), n2 = fit_warps(4, w2, sv.max_smem), split = pl.split;
     int bf = 0, bc = 0, b2 = 0;
     if (fg_status rc = grid_for(kf, 32 * nf, wf * nf, sv.num_sms, s.n * s.nsc_max * pl.chunks * 2, bf)) return rc;
-    if (fg_status rc = grid_for(kc, 128, 4 * s.rec_bytes, sv.num_sms, s.n * split, bc)) return rc;
+    const size_t wc = 4 * s.rec_bytes;
+    if (fg_status rc = grid_for(kc, 128, wc, sv.num_sms, s.n * split, bc)) return rc;
     if (fg_status rc = grid_for(k2, 32 * n2, w2 * n2, sv.num_sms, s.n * split, b2)) return rc;
     timer_begin(st);
     k2<<<b2, 32 * n2, w2 * n2, st>>>(T, s, split, gbar, gpar, w2);
@@ -1005,7 +1268,7 @@ fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T,
         } else {
             kf<<<bf, 32 * nf, wf * nf, st>>>(T, s, pass, wf);
         }
-        kc<<<bc, 128, 4 * s.rec_bytes, st>>>(T, s, pass, split, gbar, gpar);
+        kc<<<bc, 128, wc, st>>>(T, s, pass, split, gbar, gpar);
     }
     timer_end(st);
     k_share_coord_grad<R, KIND><<<pb, 128, 0, st>>>(s, split, gpar, greff_d, greff_r, gout_d, gout_r);

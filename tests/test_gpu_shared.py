@@ -76,10 +76,38 @@ def test_shared_form_equals_one_kernel_form(dtype, case, nk, counts):
     S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
     got, cc, rf, offered = _rows(st, b, q, S, True)
     ref, cr, rr, _ = _rows(st, b, q, S, False)
-    assert offered == (nk > 0 or (b.n < 4000 and st.ilinit > 1))       # share_plan's rule at 2, 3 and 6 chunks
+    # share_plan's rule at 2, 3 and 6 chunks of energies: classes, or the staged form from 4,096 (path, chunk) items
+    assert offered == (nk > 0 or b.n > 4000 or st.ilinit > 1)
     _same(cc, cr, TOL[dtype])
     _same(got, ref, TOL[dtype])
     assert torch.equal(rf, rr)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", ["cfg2_phase", "case_A014", "case_A009"])
+@pytest.mark.parametrize("counts", [{3: 2050}, {2: 4100}, {4: 2300, 3: 7, 2: 3}, {3: 32000, 2: 1001}],
+                         ids=["short", "two", "four", "sub-batches"])
+def test_staged_form_equals_one_kernel_form(dtype, case, counts):
+    """The staged form (many paths on few energies): one sub-batch of 2^15 paths and two, rows that change from path to
+    path, interpolation matrices of two entries a row and of many, more fine-grid points than the shared sums hold."""
+    from feffgpu_b200 import GPUPathStage, PathBatch
+    P = phase(case)
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    b = PathBatch(_list(P.nph, counts, 7, seed=8), nrows=3, device="cuda")
+    q = torch.arange(1, 402, dtype=torch.float64, device="cuda") * 0.05
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    got, cc, rf, offered = _rows(st, b, q, S, True)
+    ref, cr, rr, _ = _rows(st, b, q, S, False)
+    assert offered
+    _same(cc, cr, TOL[dtype])
+    _same(got, ref, TOL[dtype])
+    assert torch.equal(rf, rr)
+    if b.n < 3000:
+        for nk in (35, 1300):
+            qk = torch.linspace(0.5, 15.0, nk, dtype=torch.float64, device="cuda")
+            D = torch.softmax(-(qk[:, None] - torch.linspace(0.5, 15.0, st.E, dtype=torch.float64, device="cuda")) ** 2, 1)
+            D = torch.where(D > 1e-3, D, 0.0).contiguous()
+            _same(_rows(st, b, qk, D, True)[0], _rows(st, b, qk, D, False)[0], TOL[dtype])
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

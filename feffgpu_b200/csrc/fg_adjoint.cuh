@@ -1122,9 +1122,10 @@ __global__ void __launch_bounds__(128) k_coord_grad(const CT *__restrict__ coord
 // Fine-grid adjoint (stage.py:372-388 differentiated): per path, from upstream weights G(q) on the fine grid, the
 // seeds gbar(e) = dL/dRe(cchi) + i dL/dIm(cchi), dL/dreff (A) and, with per-path sigma2, dL/dsigma2.
 // mode 0: G = grad_chi[p][q] (chi_fine's adjoint); mode 1: G = grad_rows[row[p]][q] deg[p] exp(-2 sigma2 q^2)
-// (the fused sum's adjoint).  Interpolation transposed with the column ranges tspan of S.
+// (the fused sum's adjoint).  Interpolation transposed with the column ranges tspan of S.  A block per path, as k_chi_fine
+// (396 paths x 60 energies x 401 points: 24 us with a warp per path, 13 now).
 template <typename R>
-__global__ void __launch_bounds__(256) k_fine_adjoint(int64_t B, int E, int NK, int mode,
+__global__ void __launch_bounds__(128) k_fine_adjoint(int64_t B, int E, int NK, int mode,
                                                        const C2<R> *__restrict__ cchi, const R *__restrict__ reff_r,
                                                        const double *__restrict__ reff_d, const R *__restrict__ q_r,
                                                        const double *__restrict__ q_d, const R *__restrict__ S_r,
@@ -1134,84 +1135,79 @@ __global__ void __launch_bounds__(256) k_fine_adjoint(int64_t B, int E, int NK, 
                                                        const double *__restrict__ deg,
                                                        const double *__restrict__ sigma2, C2<R> *__restrict__ gbar,
                                                        R *__restrict__ greff_r, double *__restrict__ greff_d,
-                                                       double *__restrict__ gsig, int *status, size_t wbytes)
+                                                       double *__restrict__ gsig, int *status)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     if (status && (*(volatile const int *)status & kBadLayout)) return;   // a batch that k_validate refused
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    unsigned char *base = smem + (size_t)w * wbytes;
-    double *amp = reinterpret_cast<double *>(base);        // FP64, as the forward forms it
-    double *pha = reinterpret_cast<double *>(base + align_up((size_t)E * 8, 16));
-    double *dA = reinterpret_cast<double *>(base + 2 * align_up((size_t)E * 8, 16));
-    double *dP = dA + NK;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double *amp = reinterpret_cast<double *>(smem), *pha = amp + E, *dA = amp + max(2 * E, 8), *dP = dA + NK;
+    double *red = amp;                                     // the four warps' sums, once amp and pha have been used
     auto Sv = [&](int k, int j) { return S_d ? S_d[(size_t)k * E + j] : (double)S_r[(size_t)k * E + j]; };
-    for (int64_t p = (int64_t)blockIdx.x * nw + w; p < B; p += (int64_t)gridDim.x * nw) {
+    for (int64_t p = blockIdx.x; p < B; p += gridDim.x) {
         const C2<R> *c = cchi + p * E;
-        amp_phase<R>(E, lane, [&](int e) { return c[e]; }, amp, pha);
-        __syncwarp();
+        amp_phase_block<R>(E, [&](int e) { return c[e]; }, amp, pha);     // FP64, as the forward forms them
         const double rf = reff_d ? reff_d[p] : (double)reff_r[p];
         const double s2 = (mode == 1 && sigma2) ? sigma2[p] : 0.0;
         const double wd = mode == 1 ? deg[p] : 1.0;
         const double *gr = mode == 1 ? grows + (int64_t)row[p] * NK : nullptr;
         double g_reff = 0.0, g_s2 = 0.0;
-        for (int k0 = 0; k0 < NK; k0 += 32) {
-            const int k = k0 + lane;
-            double da = 0.0, dp = 0.0;
-            if (k < NK) {
-                const int lo = span[2 * k], hi = span[2 * k + 1];
-                double a = 0.0, ph = 0.0;
-                for (int j = lo; j < hi; ++j) {
-                    const double sv = Sv(k, j);
-                    a += sv * (double)amp[j];
-                    ph += sv * pha[j];
-                }
-                const double qk = q_d ? q_d[k] : (double)q_r[k];
-                const double damp = s2 != 0.0 ? exp(-2.0 * s2 * qk * qk) : 1.0;
-                const double G = (mode == 1 ? gr[k] * wd : (double)gchi[p * NK + k]) * damp;
-                const double arg = ph + 2.0 * qk * rf;
-                const double sn = sin_arg<R>(arg), cs = sin_arg<R>(arg + 1.5707963267948966);
-                da = G * sn;
-                dp = G * a * cs;
-                g_reff += dp * 2.0 * qk;
-                g_s2 += G * a * sn * (-2.0 * qk * qk);
-                dA[k] = da;
-                dP[k] = dp;
+        for (int k = threadIdx.x; k < NK; k += blockDim.x) {
+            const int lo = span[2 * k], hi = span[2 * k + 1];
+            double a = 0.0, ph = 0.0;
+            for (int j = lo; j < hi; ++j) {
+                const double sv = Sv(k, j);
+                a += sv * amp[j];
+                ph += sv * pha[j];
             }
+            const double qk = q_d ? q_d[k] : (double)q_r[k];
+            const double damp = s2 != 0.0 ? exp(-2.0 * s2 * qk * qk) : 1.0;
+            const double G = (mode == 1 ? gr[k] * wd : (double)gchi[p * NK + k]) * damp;
+            const double arg = ph + 2.0 * qk * rf;
+            const double sn = sin_arg<R>(arg), cs = sin_arg<R>(arg + 1.5707963267948966);
+            const double dp = G * a * cs;
+            g_reff += dp * 2.0 * qk;
+            g_s2 += G * a * sn * (-2.0 * qk * qk);
+            dA[k] = G * sn;
+            dP[k] = dp;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             g_reff += __shfl_xor_sync(0xffffffffu, g_reff, o);
             g_s2 += __shfl_xor_sync(0xffffffffu, g_s2, o);
         }
-        __syncwarp();
-        for (int e0 = 0; e0 < E; e0 += 32) {
-            const int e = e0 + lane;
-            if (e < E) {
-                const int lo = tspan[2 * e], hi = tspan[2 * e + 1];
-                double ga = 0.0, gp = 0.0;
-                for (int k = lo; k < hi; ++k) {
-                    const double sv = Sv(k, e);
-                    ga += sv * dA[k];
-                    gp += sv * dP[k];
-                }
-                const C2<R> cv = c[e];
-                const double x = (double)cv.x, y = (double)cv.y;
-                const double a = sqrt(x * x + y * y + 1e-30);
-                double gx = ga * x / a, gy = ga * y / a;
-                if (a >= 1e-16) {
-                    const double r2 = x * x + y * y;
-                    gx += gp * (-y) / r2;
-                    gy += gp * x / r2;
-                }
-                gbar[p * E + e] = C2<R>{(R)gx, (R)gy};
-            }
-        }
+        __syncthreads();
         if (lane == 0) {
+            red[2 * w] = g_reff;
+            red[2 * w + 1] = g_s2;
+        }
+        for (int e = threadIdx.x; e < E; e += blockDim.x) {
+            const int lo = tspan[2 * e], hi = tspan[2 * e + 1];
+            double ga = 0.0, gp = 0.0;
+            for (int k = lo; k < hi; ++k) {
+                const double sv = Sv(k, e);
+                ga += sv * dA[k];
+                gp += sv * dP[k];
+            }
+            const C2<R> cv = c[e];
+            const double x = (double)cv.x, y = (double)cv.y;
+            const double a = sqrt(x * x + y * y + 1e-30);
+            double gx = ga * x / a, gy = ga * y / a;
+            if (a >= 1e-16) {
+                const double r2 = x * x + y * y;
+                gx += gp * (-y) / r2;
+                gy += gp * x / r2;
+            }
+            gbar[p * E + e] = C2<R>{(R)gx, (R)gy};
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            g_reff = (red[0] + red[2]) + (red[4] + red[6]);
+            g_s2 = (red[1] + red[3]) + (red[5] + red[7]);
             if (greff_d) greff_d[p] = g_reff;
             if (greff_r) greff_r[p] = (R)g_reff;
             if (gsig) gsig[p] = g_s2;
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -1253,14 +1249,12 @@ fg_status launch_fine_adjoint(const StageView &sv, int64_t B, int NK, int mode, 
                               const double *deg, const double *sigma2, C2<R> *gbar, R *greff_r,
                               double *greff_d, double *gsig, int *status, cudaStream_t st)
 {
-    const size_t wb = 2 * align_up((size_t)sv.E * 8, 16) + align_up((size_t)NK * 16, 16);
-    const int warps = fit_warps(4, wb, sv.max_smem), threads = warps * 32;
+    const size_t smem = (size_t)std::max(2 * sv.E, 8) * 8 + (size_t)NK * 16;
     auto kern = k_fine_adjoint<R>;
     int blocks = 0;
-    if (fg_status rc = grid_for(kern, threads, wb * warps, sv.num_sms, B, blocks)) return rc;
-    kern<<<blocks, threads, wb * warps, st>>>(B, sv.E, NK, mode, static_cast<const C2<R> *>(cchi), reff_r, reff_d, q_r,
-                                              q_d, S_r, S_d, span, tspan, gchi, grows, row, deg, sigma2, gbar,
-                                              greff_r, greff_d, gsig, status, wb);
+    if (fg_status rc = grid_for(kern, 128, smem, sv.num_sms, B * 4, blocks)) return rc;
+    kern<<<blocks, 128, smem, st>>>(B, sv.E, NK, mode, static_cast<const C2<R> *>(cchi), reff_r, reff_d, q_r, q_d, S_r, S_d,
+                                    span, tspan, gchi, grows, row, deg, sigma2, gbar, greff_r, greff_d, gsig, status);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }

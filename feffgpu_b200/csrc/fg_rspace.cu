@@ -101,7 +101,7 @@ extern "C" fg_status fg_rspace_misfit(int64_t B, int32_t NK, int32_t NR, const d
     if (B > 0x7fffffffLL / kBlocks) return fail(FG_ERR_VALUE, "too many rows for one call");
     const size_t smem = (size_t)((NK + 1) & ~1) * sizeof(double) + (size_t)NR * sizeof(double2);
     if (smem > 200 * 1024) return fail(FG_ERR_VALUE, "NK and NR too large for one block's shared memory");
-    if (smem > 48 * 1024) FG_CUDA(cudaFuncSetAttribute(k_rspace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 40 * 1024) FG_CUDA(cudaFuncSetAttribute(k_rspace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_rspace<<<(unsigned)(B * kBlocks), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
         NK, NR, rows, reinterpret_cast<const double2 *>(F), reinterpret_cast<const double2 *>(target), inv_norm, R,
         grad);

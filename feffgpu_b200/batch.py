@@ -77,7 +77,6 @@ class PathBatch:
         self.row = row.to(d)
         self.order = torch.as_tensor(order).to(d)
         self.counts = {int(k): int(v) for k, v in zip(*np.unique(nl_np, return_counts=True))}
-        self._ws = {}
         self._tuned = {}             # launch shapes chosen for this batch, per (stage, precision, k points)
 
     def sample(self, max_paths: int) -> "PathBatch":
@@ -94,15 +93,6 @@ class PathBatch:
             groups.append((self.coords[sel, :n].cpu(), self.ipots[sel, :n].cpu(), self.deg[sel].cpu(),
                            self.row[sel].cpu()))
         return PathBatch(groups, nrows=self.nrows, device=self.device)
-
-    def workspace(self, nbytes: int, backward: bool = False) -> torch.Tensor:
-        """A cached device scratch buffer of at least nbytes (one per direction)."""
-        key = "bwd" if backward else "fwd"
-        ws = self._ws.get(key)
-        if ws is None or ws.numel() < max(nbytes, 1):
-            ws = torch.empty(max(nbytes, 1), device=self.device, dtype=torch.uint8)
-            self._ws[key] = ws
-        return ws
 
     def __len__(self) -> int:
         return self.n

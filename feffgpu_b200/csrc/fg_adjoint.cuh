@@ -1291,6 +1291,7 @@ fg_status cchi_bwd_call(const StageView &sv, const Tables<R> &T, int64_t B, int 
                                                                    st, nullptr, &head->general))
                         return rc;
                 }
+                timer_end(st);               // begun in adjoint
             }
             return FG_OK;
         }
@@ -1363,6 +1364,7 @@ fg_status Launch<R, EDGE>::fused_bwd(const StageView &sv, const Tables<R> &T, co
                     return rc;
                 if (!pl.force)
                     if (fg_status rc = general(t0, s.n, &head->general)) return rc;
+                timer_end(st);                   // begun in adjoint
             }
             return FG_OK;
         }

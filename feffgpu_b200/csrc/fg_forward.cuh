@@ -334,6 +334,158 @@ __device__ __forceinline__ C2<R> cfac(const WarpPath<R> &g, const Tables<R> &T, 
     return cmul(ex, cinv(prho));
 }
 
+// ------------------------------------------------------------------------------------------------ flip basis
+// F~ commutes with the signed flip (S v)_m = (-1)^m v_(-m), so in the basis u_m = v_m + (-1)^m v_(-m) (and v_0 of each
+// n), w_m = v_m - (-1)^m v_(-m) it is two blocks: 4 x 4 over u = (0,0), (0,1), 1, 2 and 2 x 2 over w = 1, 2.  A chain step
+// costs 80 complex multiply-adds instead of 144, and the Euler phase e^{-i eta m} mixes u_m and w_m by cos and -i sin.
+// Every form of the forward (k_fused, k_cchi, the staged and the shared kernels) takes its chain product through these
+// functions, so that a path's signal is the same bits whichever form a call takes.
+template <int KIND> struct Flip {
+    static constexpr LamTab L = lamtab(KIND);
+    static_assert(L.N == 6 && L.MM == 2, "the six-entry sets of orders 0-2");
+    static constexpr int NE0 = L.N0 == 4 ? 3 : 4, NO0 = L.N0 == 4 ? 1 : 2;   // u and w entries within the final state
+    // (m, n) of u entry i; w entry i: m = i + 1
+    static __host__ __device__ constexpr int em(int i) { return i < 2 ? 0 : i - 1; }
+    static __host__ __device__ constexpr int en(int i) { return i == 1; }
+    // position of (m, n) in the lambda set
+    static __host__ __device__ constexpr int at(int m, int n)
+    {
+        const LamTab t = lamtab(KIND);
+        for (int i = 0; i < 6; ++i)
+            if (t.m[i] == m && t.n[i] == n) return i;
+        return 0;
+    }
+};
+
+// The block entries (u block row-major, then w block) from the canonical entries of a matrix formed for the rows lam1 < NR
+// and columns lam2 < NC (all, or those within the final state; entries beyond them are zero)
+template <typename R, int KIND, int NR, int NC>
+__device__ __forceinline__ void to_blocks(const C2<R> (&acc)[RepTab<KIND, NR, NC>().n], C2<R> (&f)[20])
+{
+    constexpr LamTab L = lamtab(KIND);
+    constexpr RepTab<KIND, NR, NC> RT{};
+    using B = Flip<KIND>;
+    constexpr int ru = NR == L.N ? 4 : B::NE0, rw = NR == L.N ? 2 : B::NO0, cu = NC == L.N ? 4 : B::NE0,
+                  cw = NC == L.N ? 2 : B::NO0;
+    auto F = [&](int a, int b) { return RT.sg[a][b] > 0 ? acc[RT.rep[a][b]] : cscl(acc[RT.rep[a][b]], R(-1)); };
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            f[4 * i + j] = cz<R>();
+            if (i >= ru || j >= cu) continue;
+            const int a = B::at(B::em(i), B::en(i)), b = B::at(B::em(j), B::en(j));
+            C2<R> v = F(a, b);
+            if (B::em(j)) {
+                if (B::em(i)) {
+                    const C2<R> x = F(a, B::at(-B::em(j), 0));
+                    v = (B::em(j) & 1) ? csub(v, x) : cadd(v, x);
+                }
+            } else if (B::em(i)) {
+                v = cscl(v, R(2));
+            }
+            f[4 * i + j] = v;
+        }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            f[16 + 2 * i + j] = cz<R>();
+            if (i >= rw || j >= cw) continue;
+            const int a = B::at(i + 1, 0);
+            const C2<R> v = F(a, B::at(j + 1, 0)), x = F(a, B::at(-j - 1, 0));
+            f[16 + 2 * i + j] = j == 0 ? cadd(v, x) : csub(v, x);
+        }
+}
+
+// (u, w) turned by the Euler phase e^{-i eta m}, given as ph = e^{-i eta m}: (c u - i s w, c w - i s u)
+template <typename R> __device__ __forceinline__ void turn(C2<R> ph, C2<R> &u, C2<R> &w)
+{
+    const R c = ph.x, s = -ph.y;
+    const C2<R> a = u, b = w;
+    u = C2<R>{fma(c, a.x, s * b.y), fma(c, a.y, -s * b.x)};
+    w = C2<R>{fma(c, b.x, s * a.y), fma(c, b.y, -s * a.x)};
+}
+
+// One column (u entries x[0..3], w entries x[4..5]) times the blocks, then the phase; rows: only the first NE0 u and NO0
+// w entries are formed (what the termination reads)
+template <typename R, int KIND>
+__device__ __forceinline__ void block_step(const C2<R> (&f)[20], C2<R> e1, C2<R> e2, bool all, C2<R> (&x)[6])
+{
+    using B = Flip<KIND>;
+    C2<R> y[6];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        y[i] = cz<R>();
+        if (all || i < B::NE0)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[i] = cfma(f[4 * i + j], x[j], y[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        y[4 + i] = cz<R>();
+        if (all || i < B::NO0)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) y[4 + i] = cfma(f[16 + 2 * i + j], x[4 + j], y[4 + i]);
+    }
+    turn(e1, y[2], y[4]);
+    turn(e2, y[3], y[5]);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) x[i] = y[i];
+}
+
+// The first matrix's column c of the N0 (u columns, then w columns): a block column, then the phase
+template <typename R, int KIND>
+__device__ __forceinline__ void block_first(const C2<R> (&f)[20], C2<R> e1, C2<R> e2, int c, C2<R> (&x)[6])
+{
+    using B = Flip<KIND>;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) x[i] = cz<R>();
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (j < B::NE0 && c == j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = f[4 * i + j];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+        if (j < B::NO0 && c == B::NE0 + j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) x[4 + i] = f[16 + 2 * i + j];
+    turn(e1, x[2], x[4]);
+    turn(e2, x[3], x[5]);
+}
+
+// The chain product back in the lambda set's entries, Q[b][a] for a, b < N0, from its columns P(c)[i]
+template <typename R, int KIND, class PF>
+__device__ __forceinline__ void from_blocks(const PF &P, C2<R> (&Q)[lamtab(KIND).N0][lamtab(KIND).N0])
+{
+    constexpr LamTab L = lamtab(KIND);
+    using B = Flip<KIND>;
+#pragma unroll
+    for (int a = 0; a < L.N0; ++a) {
+        const int am = L.m[a] < 0 ? -L.m[a] : L.m[a];
+        // the column of entry a: u_am (+-) w_am
+        C2<R> x[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            if (am == 0) {
+                x[i] = P(L.n[a], i);
+            } else {
+                const C2<R> u = P(am + 1, i), w = P(B::NE0 + am - 1, i);
+                if (L.m[a] > 0) x[i] = cadd(u, w);
+                else x[i] = (am & 1) ? csub(w, u) : csub(u, w);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < L.N0; ++b) {
+            const int bm = L.m[b] < 0 ? -L.m[b] : L.m[b];
+            if (bm == 0) Q[b][a] = x[L.n[b]];
+            else if (L.m[b] > 0) Q[b][a] = cscl(cadd(x[bm + 1], x[3 + bm]), R(0.5));
+            else Q[b][a] = cscl((bm & 1) ? csub(x[3 + bm], x[bm + 1]) : csub(x[bm + 1], x[3 + bm]), R(0.5));
+        }
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ one energy
 // Paths with two or more scatterers (nleg >= 3).  Every scattering matrix is accumulated as a full lamx x lamx
 // matrix -- the first matrix's columns beyond laml0x and the last one's rows beyond laml0x are computed and not
@@ -367,7 +519,8 @@ __device__ C2<R> energy_ms(const WarpPath<R> &g, const R *dh, const Tables<R> &T
     const size_t dleg = (size_t)(T.L1 + 1) * DS, tlip = (size_t)(T.L1 + 1) * E;
     const C2<R> ck = T.ck[e];
     if (fabs((double)ck.x) + fabs((double)ck.y) <= 1e-16) return cz<R>();
-    C2<R> P[N][N0];
+    constexpr bool FLIP = N == 6;                   // the sets of orders 0-2; order 3 multiplies the matrices as they are
+    C2<R> P[N][N0], X[N0][6];
     for (int k = 1; k <= nsc; ++k) {
         C2<R> acc[RT.n];
         const int ip = g.ip[k];
@@ -383,6 +536,19 @@ __device__ C2<R> energy_ms(const WarpPath<R> &g, const R *dh, const Tables<R> &T
         accumulate_f<R, KIND, N, N, sizeof(R) == 4 ? 2 : 1>(acc, dh + (k - 1) * dleg, tk, tstride, ilx,
                                                            zfac(cscl(ck, (R)g.ri[k + 1])), zfac(cscl(ck, (R)g.ri[k])));
         mask_lambda<R, KIND, N, N>(acc, T.nlam);
+        if constexpr (FLIP) {
+            C2<R> f[20];
+            to_blocks<R, KIND, N, N>(acc, f);
+            const C2<R> e1 = g.phs[k + 1], e2 = cmul(e1, e1);
+            if (k == 1) {
+#pragma unroll
+                for (int c = 0; c < N0; ++c) block_first<R, KIND>(f, e1, e2, c, X[c]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < N0; ++c) block_step<R, KIND>(f, e1, e2, k < nsc, X[c]);
+            }
+            continue;
+        }
         C2<R> ph[2 * MM + 1];
         phase_powers<R, MM>(g.phs[k + 1], ph);
         C2<R> Pn[N][N0];
@@ -409,8 +575,15 @@ __device__ C2<R> energy_ms(const WarpPath<R> &g, const R *dh, const Tables<R> &T
 #pragma unroll
             for (int b = 0; b < N0; ++b) P[a][b] = Pn[a][b];
     }
-    const C2<R> ptrac = termination<R, KIND>(g, T, e, nleg, ck, [&](int b, int a) { return P[b][a]; });
-    return cmul(ptrac, cfac(g, T, e, nleg, ck));
+    if constexpr (FLIP) {
+        C2<R> Q[N0][N0];
+        from_blocks<R, KIND>([&](int c, int i) { return X[c][i]; }, Q);
+        const C2<R> ptrac = termination<R, KIND>(g, T, e, nleg, ck, [&](int b, int a) { return Q[b][a]; });
+        return cmul(ptrac, cfac(g, T, e, nleg, ck));
+    } else {
+        const C2<R> ptrac = termination<R, KIND>(g, T, e, nleg, ck, [&](int b, int a) { return P[b][a]; });
+        return cmul(ptrac, cfac(g, T, e, nleg, ck));
+    }
 }
 // Three legs alone (k_stage_energies): with only a first and a last matrix in the kernel, each is accumulated as far as
 // it is read, the first one's columns and the last one's rows within the final state (14 of 20 canonical entries each at
@@ -419,51 +592,37 @@ template <typename R, int KIND>
 __device__ C2<R> energy_ms3(const WarpPath<R> &g, const R *dh, const Tables<R> &T, int e)
 {
     constexpr LamTab L = lamtab(KIND);
-    constexpr int N = L.N, N0 = L.N0, MM = L.MM, DS = dstride(MM), UNR = sizeof(R) == 4 ? 2 : 1;
+    constexpr int N = L.N, N0 = L.N0, DS = dstride(L.MM), UNR = sizeof(R) == 4 ? 2 : 1;
     const int E = T.E;
     const size_t tlip = (size_t)(T.L1 + 1) * E;
     const C2<R> ck = T.ck[e];
     if (fabs((double)ck.x) + fabs((double)ck.y) <= 1e-16) return cz<R>();
     const C2<R> z2 = zfac(cscl(ck, (R)g.ri[2]));
-    C2<R> P[N][N0];
+    C2<R> X[N0][6], f[20];
     {
-        constexpr RepTab<KIND, N, N0> RT{};
-        C2<R> acc[RT.n];
+        C2<R> acc[RepTab<KIND, N, N0>().n];
         const int ip = g.ip[1];
         accumulate_f<R, KIND, N, N0, UNR>(acc, dh, T.tl + ip * tlip + e, E, T.lmax[ip * E + e] + 1, z2,
                                           zfac(cscl(ck, (R)g.ri[1])));
         mask_lambda<R, KIND, N, N0>(acc, T.nlam);
-        C2<R> ph[2 * MM + 1];
-        phase_powers<R, MM>(g.phs[2], ph);
+        to_blocks<R, KIND, N, N0>(acc, f);
+        const C2<R> e1 = g.phs[2], e2 = cmul(e1, e1);
 #pragma unroll
-        for (int a = 0; a < N; ++a)
-#pragma unroll
-            for (int b = 0; b < N0; ++b) {
-                const C2<R> v = acc[RT.rep[a][b]];
-                P[a][b] = cmul(ph[L.m[a] + MM], RT.sg[a][b] > 0 ? v : cscl(v, R(-1)));
-            }
+        for (int c = 0; c < N0; ++c) block_first<R, KIND>(f, e1, e2, c, X[c]);
     }
-    constexpr RepTab<KIND, N0, N> RT{};
-    C2<R> acc[RT.n];
-    const int ip = g.ip[2];
-    accumulate_f<R, KIND, N0, N, UNR>(acc, dh + (size_t)(T.L1 + 1) * DS, T.tl + ip * tlip + e, E, T.lmax[ip * E + e] + 1,
-                                      zfac(cscl(ck, (R)g.ri[3])), z2);
-    mask_lambda<R, KIND, N0, N>(acc, T.nlam);
-    C2<R> ph[2 * MM + 1];
-    phase_powers<R, MM>(g.phs[3], ph);
+    {
+        C2<R> acc[RepTab<KIND, N0, N>().n];
+        const int ip = g.ip[2];
+        accumulate_f<R, KIND, N0, N, UNR>(acc, dh + (size_t)(T.L1 + 1) * DS, T.tl + ip * tlip + e, E,
+                                          T.lmax[ip * E + e] + 1, zfac(cscl(ck, (R)g.ri[3])), z2);
+        mask_lambda<R, KIND, N0, N>(acc, T.nlam);
+        to_blocks<R, KIND, N0, N>(acc, f);
+        const C2<R> e1 = g.phs[3], e2 = cmul(e1, e1);
+#pragma unroll
+        for (int c = 0; c < N0; ++c) block_step<R, KIND>(f, e1, e2, false, X[c]);
+    }
     C2<R> Q[N0][N0];
-#pragma unroll
-    for (int a = 0; a < N0; ++a)
-#pragma unroll
-        for (int b = 0; b < N0; ++b) {
-            C2<R> s = cz<R>();
-#pragma unroll
-            for (int c = 0; c < N; ++c) {
-                const C2<R> f = acc[RT.rep[a][c]];
-                s = RT.sg[a][c] > 0 ? cfma(f, P[c][b], s) : cfms(f, P[c][b], s);
-            }
-            Q[a][b] = cmul(ph[L.m[a] + MM], s);
-        }
+    from_blocks<R, KIND>([&](int c, int i) { return X[c][i]; }, Q);
     const C2<R> ptrac = termination<R, KIND>(g, T, e, 3, ck, [&](int b, int a) { return Q[b][a]; });
     return cmul(ptrac, cfac(g, T, e, 3, ck));
 }

@@ -95,6 +95,7 @@ fg_status cchi_call(const StageView &sv, const Tables<R> &T, int64_t B, int nleg
                     if (fg_status rc = launch_cchi<R, EDGE, CT>(sv, T, s.n, nleg, c, ip, out, reff + t0, bad, warps,
                                                                 &head->general, st))
                         return rc;
+                timer_end(st);               // begun in signals: whichever form evaluated the paths
             }
             return FG_OK;
         }
@@ -157,6 +158,7 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
                                                              status, shape, &head->general, st))
                         return rc;
                 }
+                timer_end(st);                   // begun in signals: whichever form evaluated the paths, and the fine grid
             }
         }
     } else if (P->n > 0) {

@@ -17,9 +17,11 @@
 // that of the one-kernel form (k_fused, k_cchi): the results are the same bits.
 //
 // Measured on B200 (fused forward, 401 energies and k points): 128,844 paths of two to eight legs, 530,707 scatterers
-// in 49,006 classes, mixed form 29.1 -> 12.3 ms (k_share_chain 8.2, k_share_f 2.1, k_share_fine 1.9 ms); 31,142 paths
-// of up to seven legs, FP64 form 14.3 -> 5.65 ms.  What bounds it: the chain product's 144 complex multiply-adds per
-// scatterer and energy and the 160 bytes (FP32) of matrix it reads for them, 4.3 TB/s from L2 and HBM.
+// in 49,006 classes, mixed form 29.1 -> 9.4 ms (k_share_chain 5.2, k_share_f 2.5, k_share_fine 1.3 ms); 31,142 paths of up
+// to seven legs, FP64 form 14.3 -> 4.5 ms.  What bounds the chain: issue (57 % of cycles) of its 80 complex multiply-adds
+// a step and the latency of the 160 bytes (FP32) of matrix from L1 (13 % hits) and L2 (49 %); fetching the next matrix
+// into shared memory while one is multiplied measured the same (5.3 ms), pair instructions 2 % slower, 128 MB passes
+// instead of 1 GB 10 % slower.
 #pragma once
 #include "fg_adjoint.cuh"
 
@@ -69,150 +71,6 @@ template <typename R, int NE> __device__ __forceinline__ void load_f(const unsig
         for (int i = 0; i < NE; ++i) {
             const double2 v = reinterpret_cast<const double2 *>(at)[i * 32 + lane];
             f[i] = C2<R>{v.x, v.y};
-        }
-    }
-}
-
-// ------------------------------------------------------------------------------------------------ flip basis
-// F~ commutes with the signed flip (S v)_m = (-1)^m v_(-m), so in the basis u_m = v_m + (-1)^m v_(-m) (and v_0 of each
-// n), w_m = v_m - (-1)^m v_(-m) it is two blocks: 4 x 4 over u = (0,0), (0,1), 1, 2 and 2 x 2 over w = 1, 2.  The classes
-// keep the 20 block entries, formed once per class, and a chain step costs 80 complex multiply-adds instead of 144; the
-// Euler phase e^{-i eta m} mixes u_m and w_m by cos and -i sin.  (In k_fused, which forms every matrix in the registers
-// of its chain, the same basis cost more registers than it saved work.)
-template <int KIND> struct Flip {
-    static constexpr LamTab L = lamtab(KIND);
-    static_assert(L.N == 6 && L.MM == 2, "the six-entry sets of orders 0-2");
-    static constexpr int NE0 = L.N0 == 4 ? 3 : 4, NO0 = L.N0 == 4 ? 1 : 2;   // u and w entries within the final state
-    // (m, n) of u entry i; w entry i: m = i + 1
-    static __host__ __device__ constexpr int em(int i) { return i < 2 ? 0 : i - 1; }
-    static __host__ __device__ constexpr int en(int i) { return i == 1; }
-    // position of (m, n) in the lambda set
-    static __host__ __device__ constexpr int at(int m, int n)
-    {
-        const LamTab t = lamtab(KIND);
-        for (int i = 0; i < 6; ++i)
-            if (t.m[i] == m && t.n[i] == n) return i;
-        return 0;
-    }
-};
-
-// The block entries (u block row-major, then w block) from the canonical entries
-template <typename R, int KIND> __device__ __forceinline__ void to_blocks(const C2<R> (&acc)[20], C2<R> (&f)[20])
-{
-    constexpr LamTab L = lamtab(KIND);
-    constexpr RepTab<KIND, L.N, L.N> RT{};
-    using B = Flip<KIND>;
-    auto F = [&](int a, int b) { return RT.sg[a][b] > 0 ? acc[RT.rep[a][b]] : cscl(acc[RT.rep[a][b]], R(-1)); };
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int a = B::at(B::em(i), B::en(i)), b = B::at(B::em(j), B::en(j));
-            C2<R> v = F(a, b);
-            if (B::em(j)) {
-                if (B::em(i)) {
-                    const C2<R> x = F(a, B::at(-B::em(j), 0));
-                    v = (B::em(j) & 1) ? csub(v, x) : cadd(v, x);
-                }
-            } else if (B::em(i)) {
-                v = cscl(v, R(2));
-            }
-            f[4 * i + j] = v;
-        }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int a = B::at(i + 1, 0);
-            const C2<R> v = F(a, B::at(j + 1, 0)), x = F(a, B::at(-j - 1, 0));
-            f[16 + 2 * i + j] = j == 0 ? cadd(v, x) : csub(v, x);
-        }
-}
-
-// (u, w) turned by the Euler phase e^{-i eta m}, given as ph = e^{-i eta m}: (c u - i s w, c w - i s u)
-template <typename R> __device__ __forceinline__ void turn(C2<R> ph, C2<R> &u, C2<R> &w)
-{
-    const R c = ph.x, s = -ph.y;
-    const C2<R> a = u, b = w;
-    u = C2<R>{fma(c, a.x, s * b.y), fma(c, a.y, -s * b.x)};
-    w = C2<R>{fma(c, b.x, s * a.y), fma(c, b.y, -s * a.x)};
-}
-
-// One column (u entries x[0..3], w entries x[4..5]) times the blocks, then the phase; rows: only the first NE0 u and NO0
-// w entries are formed (what the termination reads)
-template <typename R, int KIND>
-__device__ __forceinline__ void block_step(const C2<R> (&f)[20], C2<R> e1, C2<R> e2, bool all, C2<R> (&x)[6])
-{
-    using B = Flip<KIND>;
-    C2<R> y[6];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        y[i] = cz<R>();
-        if (all || i < B::NE0)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) y[i] = cfma(f[4 * i + j], x[j], y[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        y[4 + i] = cz<R>();
-        if (all || i < B::NO0)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) y[4 + i] = cfma(f[16 + 2 * i + j], x[4 + j], y[4 + i]);
-    }
-    turn(e1, y[2], y[4]);
-    turn(e2, y[3], y[5]);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) x[i] = y[i];
-}
-
-// The first matrix's column c of the N0 (u columns, then w columns): a block column, then the phase
-template <typename R, int KIND>
-__device__ __forceinline__ void block_first(const C2<R> (&f)[20], C2<R> e1, C2<R> e2, int c, C2<R> (&x)[6])
-{
-    using B = Flip<KIND>;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) x[i] = cz<R>();
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (j < B::NE0 && c == j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = f[4 * i + j];
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-        if (j < B::NO0 && c == B::NE0 + j)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) x[4 + i] = f[16 + 2 * i + j];
-    turn(e1, x[2], x[4]);
-    turn(e2, x[3], x[5]);
-}
-
-// The chain product back in the lambda set's entries, Q[b][a] for a, b < N0, from its columns P(c)[i]
-template <typename R, int KIND, class PF>
-__device__ __forceinline__ void from_blocks(const PF &P, C2<R> (&Q)[lamtab(KIND).N0][lamtab(KIND).N0])
-{
-    constexpr LamTab L = lamtab(KIND);
-    using B = Flip<KIND>;
-#pragma unroll
-    for (int a = 0; a < L.N0; ++a) {
-        const int am = L.m[a] < 0 ? -L.m[a] : L.m[a];
-        // the column of entry a: u_am (+-) w_am
-        C2<R> x[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            if (am == 0) {
-                x[i] = P(L.n[a], i);
-            } else {
-                const C2<R> u = P(am + 1, i), w = P(B::NE0 + am - 1, i);
-                if (L.m[a] > 0) x[i] = cadd(u, w);
-                else x[i] = (am & 1) ? csub(w, u) : csub(u, w);
-            }
-        }
-#pragma unroll
-        for (int b = 0; b < L.N0; ++b) {
-            const int bm = L.m[b] < 0 ? -L.m[b] : L.m[b];
-            if (bm == 0) Q[b][a] = x[L.n[b]];
-            else if (L.m[b] > 0) Q[b][a] = cscl(cadd(x[bm + 1], x[3 + bm]), R(0.5));
-            else Q[b][a] = cscl((bm & 1) ? csub(x[3 + bm], x[bm + 1]) : csub(x[bm + 1], x[3 + bm]), R(0.5));
         }
     }
 }
@@ -385,7 +243,7 @@ __global__ void __launch_bounds__(128) k_share_f(Tables<R> T, Share<R> s, int pa
                         zfac(cscl(ck, (R)__longlong_as_double((long long)key.x))));
                     mask_lambda<R, KIND, L.N, L.N>(acc, T.nlam);
                     C2<R> f[20];
-                    to_blocks<R, KIND>(acc, f);
+                    to_blocks<R, KIND, L.N, L.N>(acc, f);
                     store_f<R, 20>(s.F + (c * G + (it - n_two) % ng) * f_chunk_bytes<R, KIND>(), lane, f);
                 }
             }
@@ -675,7 +533,6 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
         if (fg_status rc = grid_for(ke, 32 * ew, wb * ew, sv.num_sms, s.n * pl.split, eb)) return rc;
         timer_begin(st);
         ke<<<eb, 32 * ew, wb * ew, st>>>(T, s, pl.split, out, wb);
-        timer_end(st);
         FG_CUDA(cudaGetLastError());
         return FG_OK;
     }
@@ -698,7 +555,6 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
         kf<<<fb, 32 * fw, wb * fw, st>>>(T, s, pass, out, wb);
         kc<<<cb, 128, wc, st>>>(T, s, pass, split, out);
     }
-    timer_end(st);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
@@ -931,9 +787,9 @@ __global__ void __launch_bounds__(128) k_share_f_adj(Tables<R> T, Share<R> s, in
                 mask_lambda<R, KIND, L.N, L.N>(b, T.nlam);
                 unsigned char *at = s.F + ((c * G + gc) * 4 + 2 * half) * f_chunk_bytes<R, KIND>();
                 C2<R> f[20];
-                to_blocks<R, KIND>(a, f);
+                to_blocks<R, KIND, L.N, L.N>(a, f);
                 store_f<R, 20>(at, lane, f);
-                to_blocks<R, KIND>(b, f);
+                to_blocks<R, KIND, L.N, L.N>(b, f);
                 store_f<R, 20>(at + f_chunk_bytes<R, KIND>(), lane, f);
             }
         }
@@ -1270,7 +1126,6 @@ fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T,
         }
         kc<<<bc, 128, wc, st>>>(T, s, pass, split, gbar, gpar);
     }
-    timer_end(st);
     k_share_coord_grad<R, KIND><<<pb, 128, 0, st>>>(s, split, gpar, greff_d, greff_r, gout_d, gout_r);
     FG_CUDA(cudaGetLastError());
     return FG_OK;

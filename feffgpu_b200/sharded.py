@@ -93,7 +93,9 @@ class _ChiReduceAllRanks(torch.autograd.Function):
         # every rank holds the same loss of the summed rows: its paths receive the upstream gradient
         coords, sigma2, q, S, cchi, reff = ctx.saved_tensors
         want_s2 = sigma2 is not None and ctx.needs_input_grad[1]
-        gc, gs = ctx.stage._chi_reduce_backward(ctx.batch, coords, sigma2, q, S, ctx.prec, g, cchi, reff, want_s2)
+        # the one-kernel adjoint: a path's gradient is then the same bits whichever rank evaluates it
+        gc, gs = ctx.stage._chi_reduce_backward(ctx.batch, coords, sigma2, q, S, ctx.prec, g, cchi, reff, want_s2,
+                                                one_kernel=True)
         return (gc if ctx.needs_input_grad[0] else None), (gs if want_s2 else None), None, None, None, None, None, None
 
 

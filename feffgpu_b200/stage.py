@@ -34,6 +34,10 @@ def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+def _up256(n: int) -> int:
+    return (n + 255) // 256 * 256
+
+
 def _stream(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
@@ -112,6 +116,16 @@ class GPUPathStage:
                 pass
             self._h = None
 
+    def _scratch(self, full: int, least: int) -> torch.Tensor:
+        """Device scratch of a call, from torch's stream-ordered pool for its length: what lets equal scatterers be
+        evaluated once, or, on a device too full for that, what the one-kernel forms need."""
+        try:
+            return torch.empty(max(full, least), device=self.device, dtype=torch.uint8)
+        except torch.cuda.OutOfMemoryError:
+            if full <= least:
+                raise
+            return torch.empty(least, device=self.device, dtype=torch.uint8)
+
     # -- per-path signal ------------------------------------------------------------------------------------
     def _check_ipots(self, ipots: torch.Tensor) -> None:
         if ipots.numel():
@@ -134,16 +148,15 @@ class GPUPathStage:
             raise ValueError("paths have 2 to 9 legs")
         if ipots.shape != (B, nleg):
             raise ValueError("ipots must be (B, nleg)")
+        coords, ipots = coords.contiguous(), ipots.contiguous()
         self._check_ipots(ipots)
-        coords = coords.contiguous()
-        ipots = ipots.contiguous()
         out = torch.empty(B, self.E, device=self.device, dtype=self.cdtype)
         reff = torch.empty(B, device=self.device, dtype=self.rdtype)
-        ws_n = int(self._lib.fg_cchi_workspace(self._h, B, nleg))
-        ws = torch.empty(ws_n, device=self.device, dtype=torch.uint8) if ws_n else None
+        ws = self._scratch(int(self._lib.fg_cchi_workspace(self._h, B, nleg)), 0)
         _lib.check(self._lib.fg_cchi_ws(self._h, self.prec, B, nleg, coords.data_ptr(),
                                         int(coords.dtype == torch.float64), ipots.data_ptr(), out.data_ptr(),
-                                        reff.data_ptr(), None, _ptr(ws), ws_n, _stream(self.device)))
+                                        reff.data_ptr(), None, ws.data_ptr() or None, ws.numel(),
+                                        _stream(self.device)))
         return out, reff
 
     def _cchi_backward(self, coords, ipots, g_cchi, g_reff):
@@ -153,11 +166,10 @@ class GPUPathStage:
         g_cchi = g_cchi.to(self.cdtype).contiguous()
         g_reff = None if g_reff is None else g_reff.to(self.rdtype).contiguous()
         grad = torch.empty(B, nleg, 3, device=self.device, dtype=self.rdtype)
-        ws_n = int(self._lib.fg_cchi_backward_workspace(self._h, B, nleg))
-        ws = torch.empty(max(ws_n, 1), device=self.device, dtype=torch.uint8)
+        ws = self._scratch(int(self._lib.fg_cchi_backward_workspace(self._h, B, nleg)), 256)
         _lib.check(self._lib.fg_cchi_backward(self._h, self.prec, B, nleg, coords.data_ptr(),
                                               int(coords.dtype == torch.float64), ipots.contiguous().data_ptr(),
-                                              g_cchi.data_ptr(), _ptr(g_reff), grad.data_ptr(), ws.data_ptr(), ws_n,
+                                              g_cchi.data_ptr(), _ptr(g_reff), grad.data_ptr(), ws.data_ptr(), ws.numel(),
                                               _stream(self.device)))
         return grad
 
@@ -390,8 +402,7 @@ class GPUPathStage:
         NK = q.shape[0]
         ps = self._paths_struct(batch, coords, sigma2)
         words = torch.empty(2, batch.nrows, NK, device=self.device, dtype=torch.int64)
-        ws_n = int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK))
-        ws = torch.empty(max(ws_n, 256), device=self.device, dtype=torch.uint8)
+        ws = self._scratch(int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK)), 256)
         cchi = reff = None
         if save:
             cchi = torch.empty(batch.n, self.E, device=self.device,
@@ -407,8 +418,8 @@ class GPUPathStage:
         NK = q.shape[0]
         ps = self._paths_struct(batch, coords, sigma2)
         rows = torch.empty(batch.nrows, NK, device=self.device, dtype=torch.float64)
-        ws_n = int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK))
-        ws = torch.empty(max(ws_n, 1), device=self.device, dtype=torch.uint8)
+        ws = self._scratch(int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK)),
+                           256 + _up256(16 * batch.nrows * NK))
         cchi = reff = None
         if save:
             cchi = torch.empty(batch.n, self.E, device=self.device,
@@ -416,10 +427,13 @@ class GPUPathStage:
             reff = torch.empty(batch.n, device=self.device, dtype=torch.float64)
         _lib.check(self._lib.fg_chi_reduce(self._h, prec, C.byref(ps), NK, q.data_ptr(), S.data_ptr(),
                                            self._span(S).data_ptr(), rows.data_ptr(), _ptr(cchi), _ptr(reff),
-                                           ws.data_ptr(), ws_n, _stream(self.device)))
+                                           ws.data_ptr(), ws.numel(), _stream(self.device)))
         return rows, cchi, reff
 
-    def _chi_reduce_backward(self, batch, coords, sigma2, q, S, prec, g_rows, cchi, reff, want_s2: bool):
+    def _chi_reduce_backward(self, batch, coords, sigma2, q, S, prec, g_rows, cchi, reff, want_s2: bool,
+                             one_kernel: bool = False):
+        """one_kernel: the adjoint's one-kernel form whatever the batch, whose per-path gradients do not depend on which
+        other paths are in the call (the shared form sums in another order)."""
         choice = batch._tuned.get((id(self), prec, int(q.shape[0]))) if self.autotune else None
         if choice is not None:
             self.set_launch(*choice)
@@ -428,13 +442,14 @@ class GPUPathStage:
         ps = self._paths_struct(batch, coords, sigma2)
         gc = torch.empty_like(coords)
         gs = torch.empty(batch.n, device=self.device, dtype=torch.float64) if want_s2 else None
-        ws_n = int(self._lib.fg_chi_reduce_backward_workspace(self._h, C.byref(ps), NK))
-        ws = batch.workspace(ws_n, backward=True)
+        least = 256 + _up256(batch.n * self.E * 16) + _up256(batch.n * 8) + _up256(batch.n * 256)
+        full = least if one_kernel else int(self._lib.fg_chi_reduce_backward_workspace(self._h, C.byref(ps), NK))
+        ws = self._scratch(full, least)
         _lib.check(self._lib.fg_chi_reduce_backward(self._h, prec, C.byref(ps), NK, q.data_ptr(), S.data_ptr(),
                                                     self._span(S).data_ptr(), self._span(S, True).data_ptr(),
                                                     g_rows.contiguous().data_ptr(),
                                                     cchi.data_ptr(), reff.data_ptr(), gc.data_ptr(), _ptr(gs),
-                                                    ws.data_ptr(), ws_n, _stream(self.device)))
+                                                    ws.data_ptr(), ws.numel(), _stream(self.device)))
         return gc, gs
 
 

@@ -143,7 +143,7 @@ typedef struct fg_paths {
 
 /* Workspace of the fused calls: a work-queue counter and status word, the rows' exact sums (2 x nrows x NK 64-bit
  * words) and, for batches with paths of four and more legs and for small ones, the arrays with which equal scatterers
- * of the paths are evaluated once (up to about 3 GB, whatever the number of paths).  A call given only the first two
+ * of the paths are evaluated once (up to about 4 GB, whatever the number of paths).  A call given only the first two
  * (256 + 16 nrows NK bytes, rounded up to 256) evaluates every scatterer on its own; the rows are the same. */
 FG_API size_t fg_chi_reduce_workspace(const fg_stage *stage, const fg_paths *paths, int32_t NK);
 
@@ -196,6 +196,9 @@ FG_API fg_status fg_chi_reduce_noalloc(const fg_stage *stage, fg_precision prec,
  * grad_rows (nrows, NK), using the saved cchi and reff; tspan as in fg_chi_fine_backward.  No reference
  * counterpart for sigma^2 (a new input).  The batch is checked as in fg_chi_reduce (outside stream capture the call
  * waits for its stream and returns FG_ERR_VALUE on a bad index). */
+/* Given only 256 + 16 n E + 8 n + 256 n bytes (each term rounded up to 256) instead of fg_chi_reduce_backward_workspace's,
+ * every scatterer is differentiated on its own: a path's gradient is then the same bits whatever other paths are in the
+ * call (with the full workspace, equal scatterers share their derivatives and sums are taken in another order). */
 FG_API size_t fg_chi_reduce_backward_workspace(const fg_stage *stage, const fg_paths *paths, int32_t NK);
 FG_API fg_status fg_chi_reduce_backward(const fg_stage *stage, fg_precision prec, const fg_paths *paths, int32_t NK,
                                  const double *q, const double *S, const int32_t *span, const int32_t *tspan,

@@ -29,7 +29,7 @@ EXPORTS = ("fg_stage_create", "fg_stage_destroy", "fg_stage_get_info", "fg_stage
            "fg_stage_set_launch", "fg_stage_set_fused_variant", "fg_pf_candidates", "fg_pf_extend", "fg_pf_terminal", "fg_pf_describe",
            "fg_pf_windows", "fg_pair_histogram", "fg_pair_ss_grad", "fg_rspace_misfit",
            "fg_path_columns", "fg_chi_reduce_words", "fg_rows_from_words", "fg_path_geometry", "fg_path_geometry_backward", "fg_shard_lpt", "fg_pf_enumerate_one", "fg_pf_result_gather", "fg_pf_result_destroy",
-           "fg_path_gather", "fg_path_scatter")
+           "fg_path_gather", "fg_path_scatter", "fg_stage_check_range")
 
 
 class PhaseDesc(C.Structure):
@@ -107,6 +107,7 @@ _SIGS = {
                                       C.POINTER(C.c_float), _P]),
     "fg_pf_result_gather": (C.c_int, [_P, C.c_int32, _P, _P, _P, _P, _P, _P]),
     "fg_pf_result_destroy": (None, [_P]),
+    "fg_stage_check_range": (C.c_int, [_P, C.c_int64, C.c_int64, _P, C.POINTER(C.c_int32), _P]),
     "fg_path_gather": (C.c_int, [C.c_int64, C.c_int32, _P, _P, _P, C.c_double, _P, _P, _P]),
     "fg_path_scatter": (C.c_int, [C.c_int64, C.c_int32, _P, _P, _P, _P, _P, _P]),
 }

@@ -45,6 +45,10 @@ struct fg_stage {
     Tables<float> tf{};
     Tables<double> td{};
     std::vector<void *> bufs;
+    // pinned, mapped words for the small answers that calls wait for, one borrowed per call (word_borrow)
+    int *words = nullptr;
+    std::vector<int *> free_words;
+    std::mutex words_mu;
 };
 
 namespace {
@@ -346,6 +350,14 @@ extern "C" fg_status fg_stage_create(const fg_phase_desc *d, int device, fg_stag
     fg_status st = build_tables<float>(s, s->tf, tl, ck, dk, wt, xfac, xn, rc, lmax_t);
     if (!st) st = build_tables<double>(s, s->td, tl, ck, dk, wt, xfac, xn, rc, lmax_t);
     if (st) { fg_stage_destroy(s); return st; }
+    constexpr int kWords = 32;
+    void *pw = nullptr;
+    if (cudaHostAlloc(&pw, kWords * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
+        s->words = static_cast<int *>(pw);
+        for (int i = 0; i < kWords; ++i) s->free_words.push_back(s->words + i);
+    } else {
+        cudaGetLastError();
+    }
     *out = s;
     return FG_OK;
 }
@@ -357,6 +369,7 @@ extern "C" void fg_stage_destroy(fg_stage *s)
     cudaGetDevice(&prev);
     cudaSetDevice(s->device);
     for (void *p : s->bufs) cudaFree(p);
+    if (s->words) cudaFreeHost(s->words);
     cudaSetDevice(prev);
     delete s;
 }
@@ -388,6 +401,32 @@ extern "C" fg_status fg_stage_xk(const fg_stage *s, double *out)
 
 // ================================================================================================ dispatch
 namespace {
+
+// A pinned word of the stage for the length of a call; null (the call then does without) when more calls are under way at
+// once than it has words, or none could be allocated.
+class word_borrow {
+public:
+    explicit word_borrow(const fg_stage *s) : s_(const_cast<fg_stage *>(s))
+    {
+        std::lock_guard<std::mutex> lock(s_->words_mu);
+        if (!s_->free_words.empty()) {
+            w_ = s_->free_words.back();
+            s_->free_words.pop_back();
+        }
+    }
+    ~word_borrow()
+    {
+        if (!w_) return;
+        std::lock_guard<std::mutex> lock(s_->words_mu);
+        s_->free_words.push_back(w_);
+    }
+    word_borrow(const word_borrow &) = delete;
+    int *get() const { return w_; }
+
+private:
+    fg_stage *s_;
+    int *w_ = nullptr;
+};
 
 fg_status set_device(const fg_stage *s)
 {
@@ -456,6 +495,29 @@ fg_status check_paths(const fg_paths *P)
 }
 
 }  // namespace
+
+extern "C" fg_status fg_stage_check_range(const fg_stage *s, int64_t n, int64_t hi, const int64_t *values, int32_t *inside,
+                                          void *stream)
+{
+    g_err.clear();
+    if (!s || n < 0 || !inside || (n > 0 && !values)) return fail(FG_ERR_VALUE, "bad argument");
+    *inside = 1;
+    if (n == 0) return FG_OK;
+    if (fg_status rc = set_device(s)) return rc;
+    word_borrow word(s);
+    int *w = word.get(), *d = nullptr;
+    if (!w || cudaHostGetDevicePointer(reinterpret_cast<void **>(&d), w, 0) != cudaSuccess) {
+        cudaGetLastError();
+        *inside = -1;
+        return FG_OK;
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    *w = 0;
+    if (fg_status rc = launch_range(n, hi, values, d, st)) return rc;
+    FG_CUDA(cudaStreamSynchronize(st));
+    *inside = *(volatile int *)w == 0;
+    return FG_OK;
+}
 
 extern "C" size_t fg_cchi_workspace(const fg_stage *s, int64_t B, int32_t nleg)
 {
@@ -584,7 +646,8 @@ extern "C" fg_status fg_chi_reduce(const fg_stage *s, fg_precision prec, const f
                                       static_cast<unsigned char *>(workspace) + need, workspace_bytes - need);
         }))
         return rc;
-    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st);
+    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st,
+                       word_borrow(s).get());
 }
 
 extern "C" fg_status fg_chi_reduce_words(const fg_stage *s, fg_precision prec, const fg_paths *P, int32_t NK,
@@ -611,7 +674,8 @@ extern "C" fg_status fg_chi_reduce_words(const fg_stage *s, fg_precision prec, c
                                       workspace_bytes - kCounterBytes);
         }))
         return rc;
-    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st);
+    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st,
+                       word_borrow(s).get());
 }
 
 extern "C" fg_status fg_rows_from_words(int64_t nrows, int32_t NK, const uint64_t *words, double *rows, void *stream)
@@ -654,7 +718,8 @@ extern "C" fg_status fg_chi_reduce_backward(const fg_stage *s, fg_precision prec
                                           workspace_bytes, bwd_warps(s), st);
         }))
         return rc;
-    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st);
+    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(workspace) + kStatusOffset), st,
+                       word_borrow(s).get());
 }
 
 // ------------------------------------------------------------------------------------------------ no-allocation variant
@@ -706,5 +771,6 @@ extern "C" fg_status fg_chi_reduce_noalloc(const fg_stage *s, fg_precision prec,
                                       static_cast<unsigned char *>(ws), fused_shape(s), st);
         }))
         return rc;
-    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(ws) + kStatusOffset), st);
+    return read_status(reinterpret_cast<const int *>(static_cast<unsigned char *>(ws) + kStatusOffset), st,
+                       word_borrow(s).get());
 }

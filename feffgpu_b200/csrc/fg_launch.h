@@ -88,7 +88,12 @@ fg_status launch_row_finish(int64_t nrows, int NK, const unsigned long long *rac
 // The status word of a call's kernels (device int) turned into a return code: outside stream capture the call waits
 // for its stream and reads the word (FG_ERR_VALUE with a message if a bit is set); under capture it returns FG_OK
 // without waiting (the rows of a replay that meets a bad input are NaN).
-fg_status read_status(const int *status, cudaStream_t st);
+// word: pinned host memory for the copy (a copy into pageable memory goes through the driver's staging buffer and costs
+// several microseconds more), or null.
+fg_status read_status(const int *status, cudaStream_t st, int *word = nullptr);
+
+// *out = 1 where one of n integers lies outside 0..hi (out: mapped host memory; left alone otherwise)
+fg_status launch_range(int64_t n, int64_t hi, const int64_t *values, int *out, cudaStream_t st);
 
 // The one-absorber path finder's device steps (fg_paths.cu).  candidates_one: the candidates of one absorber in atom
 // order (cand_atom, cand_rel; n entries at most), their number in *nc and off = {0, nc}, the single-scattering partial

@@ -2,6 +2,8 @@
 // a fixed-point number of resolution 2^-64 (fixed_add, two 64-bit integer words per row entry), and the rows are read
 // out once all paths are done.  Integer addition is associative, so the rows are exact sums of the rounded terms,
 // bit for bit the same whatever the order in which paths finish, the launch shape or the GPU.
+#include <algorithm>
+
 #include "fg_launch.h"
 
 namespace fg {
@@ -65,14 +67,32 @@ fg_status launch_row_finish(int64_t nrows, int NK, const unsigned long long *rac
     return FG_OK;
 }
 
-fg_status read_status(const int *status, cudaStream_t st)
+namespace {
+__global__ void __launch_bounds__(256) k_range(int64_t n, int64_t hi, const int64_t *__restrict__ v, int *out)
+{
+    bool bad = false;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        bad |= v[i] < 0 || v[i] > hi;
+    if (__syncthreads_or(bad) && threadIdx.x == 0) *(volatile int *)out = 1;
+}
+}  // namespace
+
+fg_status launch_range(int64_t n, int64_t hi, const int64_t *values, int *out, cudaStream_t st)
+{
+    k_range<<<(unsigned)std::min<int64_t>((n + 255) / 256, 592), 256, 0, st>>>(n, hi, values, out);
+    FG_CUDA(cudaGetLastError());
+    return FG_OK;
+}
+
+fg_status read_status(const int *status, cudaStream_t st, int *word)
 {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     FG_CUDA(cudaStreamIsCapturing(st, &cs));
     if (cs != cudaStreamCaptureStatusNone) return FG_OK;
     int v = 0;
-    FG_CUDA(cudaMemcpyAsync(&v, status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    FG_CUDA(cudaMemcpyAsync(word ? word : &v, status, sizeof(int), cudaMemcpyDeviceToHost, st));
     FG_CUDA(cudaStreamSynchronize(st));
+    if (word) v = *word;
     if (v & kBadIpot) return fail(FG_ERR_VALUE, "potential index outside 0..nph (the rows are NaN)");
     if (v & kBadRange)
         return fail(FG_ERR_VALUE, "a weighted path term is not finite or its magnitude is 2^31 or more (the rows are "

@@ -129,8 +129,14 @@ class GPUPathStage:
     # -- per-path signal ------------------------------------------------------------------------------------
     def _check_ipots(self, ipots: torch.Tensor) -> None:
         if ipots.numel():
-            lo, hi = (int(v) for v in torch.stack(torch.aminmax(ipots)).cpu())    # one synchronisation
-            if lo < 0 or hi > self.P.nph:
+            inside = C.c_int32()
+            v = ipots.contiguous()
+            _lib.check(self._lib.fg_stage_check_range(self._h, v.numel(), int(self.P.nph), v.data_ptr(),
+                                                      C.byref(inside), _stream(self.device)))
+            if inside.value < 0:                     # no pinned word free: the same by torch, one synchronisation
+                lo, hi = (int(x) for x in torch.stack(torch.aminmax(v)).cpu())
+                inside.value = int(lo >= 0 and hi <= self.P.nph)
+            if not inside.value:
                 raise IndexError(f"potential index out of range 0..{self.P.nph}")
 
     def cchi(self, coords, ipots):

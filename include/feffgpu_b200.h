@@ -92,6 +92,10 @@ FG_API const char *fg_last_error(void);
  * (a device int32, left untouched when every index is valid). */
 FG_API fg_status fg_cchi(const fg_stage *stage, fg_precision prec, int64_t B, int32_t nleg, const void *coords,
                   int32_t coords_f64, const int64_t *ipots, void *cchi, void *reff, int32_t *bad_ipot, void *stream);
+/* Whether every one of n device integers lies in 0..hi: *inside = 1 or 0, -1 where the answer could not be had (more calls
+ * of the stage under way than it keeps words for).  Waits for `stream`. */
+FG_API fg_status fg_stage_check_range(const fg_stage *stage, int64_t n, int64_t hi, const int64_t *values,
+                                      int32_t *inside, void *stream);
 /* The same call with device scratch: with workspace_bytes >= fg_cchi_workspace(...) (0: it would not be used) equal
  * scatterers of the paths are evaluated once and small calls spread their energies over the GPU; with less, as fg_cchi.
  * The workspace is free again when the call's work on `stream` is done. */

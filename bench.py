@@ -145,6 +145,16 @@ def finder_leg(args, dev, world, rank):
     return out
 
 
+def own_launches(step) -> int:
+    """This package's kernels in one step, counted by the profiler outside the timed region."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with torch.no_grad(), profile(activities=[ProfilerActivity.CUDA]) as p:
+        step()
+        torch.cuda.synchronize()
+    return sum(e.count for e in p.key_averages() if "fg::" in e.key)
+
+
 # ------------------------------------------------------------------------------------------------ clocks
 class Clocks:
     """nvidia-smi samples of the GPU's clocks and throttle reasons during the timed region."""
@@ -863,6 +873,7 @@ def main():
     with torch.no_grad():
         with Clocks(uuid) as clk:
             ms, kern = timed(lambda: step_rows(), args.steps, args.warmup, kernel_time=True)
+    launches = own_launches(step_rows)
     value = n_total * NK / (ms * 1e-3)
 
     e2e = fwd_bwd = plain = md = rmc = pf = pairs = ref_gpu = saved = None
@@ -877,37 +888,22 @@ def main():
             md = md_extra(args, dev, timed, world, rank)
         if args.rmc_steps > 0:
             rmc = rmc_extra(args, dev, world, rank)
-    # roofline of the dominant kernel (the fused per-path kernel): algorithmic FLOPs of the reference's loops
+    # roofline of the dominant kernels (the scattering matrices and the chain products of the batch): the operations of
+    # the form that ran, which forms a matrix once per different scatterer, beside those of the reference's loops
     import ctypes
+    from feffgpu_b200.roofline import shared_flops
     peak = ctypes.c_double()
     _lib.check(lib.fg_fp32_fma_peak(ctypes.byref(peak), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
-    flops = batch_flops(batch.nleg.cpu().numpy(), batch.ipots.cpu().numpy(), stage.lmax.cpu().numpy())
+    ref_flops = batch_flops(batch.nleg.cpu().numpy(), batch.ipots.cpu().numpy(), stage.lmax.cpu().numpy())
+    flops, classes = shared_flops(batch.coords, batch.nleg, batch.ipots, batch.row, stage.lmax.cpu().numpy())
     kern_ms = float(np.mean(kern)) if kern else None
     achieved = flops / (kern_ms * 1e-3) / 1e12 if kern_ms else None
-    traffic, traffic_src = None, None
-    tf = ROOT / "profiles" / "k_fused_feopt_traffic.txt"
-    if tf.exists():
-        for line in tf.read_text().splitlines():
-            if line.startswith("bytes_per_launch"):
-                traffic = float(line.split("=")[1])
-            if line.startswith("captured"):
-                traffic_src = line.split("=", 1)[1].strip()
-    pipe, pipe_src = None, None
-    pf_ = ROOT / "profiles" / "k_fused_fma_pipe_full_size.md"
-    if pf_.exists():
-        for line in pf_.read_text().splitlines():
-            if line.startswith("captured=") and "fma_pipe_pct=" in line:
-                kv = dict(x.split("=", 1) for x in line.split())
-                pipe, pipe_src = float(kv["fma_pipe_pct"]), kv["captured"]
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
-            "frac": achieved / peak.value if achieved else None, "traffic": traffic,
-            "traffic_source": f"not measured in this run: ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
-                              f"full-size launch, profiles/k_fused_feopt_traffic.txt ({traffic_src})",
-            "fma_pipe_active_pct": pipe,
-            "fma_pipe_source": f"not measured in this run: ncu sm__pipe_fma_cycles_active of one full-size launch, "
-                               f"profiles/k_fused_fma_pipe_full_size.md ({pipe_src})",
-            "kernel": "k_fused (per-path signal, all leg counts, one persistent launch)",
-            "kernel_ms": kern_ms, "flops_per_launch": flops,
+            "frac": achieved / peak.value if achieved else None,
+            "kernel": "k_share_f + k_share_chain + k_share_fine, all passes of a step (scattering matrices of the different "
+                      "scatterers, then every path's chain product, termination, cfac and fine grid)",
+            "kernel_ms": kern_ms, "flops_per_step": flops, "different_scatterers": classes,
+            "reference_loop_flops": ref_flops,
             "peak_source": "measured on this GPU by fg_fp32_fma_peak (FFMA chains on every SM); "
                            "MEASURED_PEAKS.json holds no FP32 figure"}
 
@@ -955,7 +951,7 @@ def main():
         "reference_cpu": ref_cpu, "pair_tables": pairs, "path_finder": pf, "md_batch": md, "rmc_refinement": rmc,
         "reference_gpu": ref_gpu, "plain_fp64": plain, "fwd_bwd": fwd_bwd,
         "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "parity": parity,
-        "gpu_launches": 3 * args.steps, "clocks": clk.summary(), "summary": summary,
+        "gpu_launches": launches * args.steps, "clocks": clk.summary(), "summary": summary,
     }
     if rank == 0:
         print(json.dumps(out))

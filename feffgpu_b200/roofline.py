@@ -67,3 +67,42 @@ def batch_flops(nleg, ipots, lmax_e_ip) -> float:
         mean_L = counts @ L.T / (n - 1)                         # (paths, E)
         total += float(np.sum(OFFSET[int(n)] + SLOPE[int(n)] * mean_L))
     return total
+
+
+# Operations of the form with shared scattering matrices (csrc/fg_shared.cuh), which forms a matrix once per different
+# scatterer and energy.  Per partial wave: 20 canonical entries complex x real + add (4), 6 spherical-wave products and 2
+# with the t-matrix (6 each), and 5 columns of the recursion (an add and a complex multiply-subtract: 10).  Per scatterer
+# and energy of a path: 80 complex multiply-adds (8) and 8 phase turns (12).  Per path and energy: the termination and
+# cfac, about 700.
+_SHARED_WAVE = 20 * 4 + 8 * 6 + 5 * 10
+_SHARED_STEP = 80 * 8 + 8 * 12
+_SHARED_END = 700
+
+
+def shared_flops(coords, nleg, ipots, row, lmax_e_ip) -> tuple[float, int]:
+    """(operations, different scatterers) of a batch whose equal scatterers are formed once: coords (n, nleg_max, 3) on
+    any device, rows telling one absorber's coordinates from another's."""
+    import torch
+    c = torch.as_tensor(coords)
+    nl = torch.as_tensor(nleg, device=c.device).long()
+    ip = torch.as_tensor(ipots, device=c.device).double()
+    rw = torch.as_tensor(row, device=c.device).double()
+    keys = []
+    for n in sorted(set(nl.tolist())):
+        if n == 2:
+            continue
+        sel = nl == n
+        x = torch.cat([c[sel, :n], c[sel, :1]], 1)
+        for k in range(1, n):
+            keys.append(torch.cat([x[:, k - 1], x[:, k], x[:, k + 1], ip[sel, k:k + 1], rw[sel, None]], 1))
+    L = torch.as_tensor(np.asarray(lmax_e_ip, float) + 1.0).sum(0)              # (nph + 1) partial waves over all energies
+    E = len(lmax_e_ip)
+    steps = float((nl[nl > 2] - 1).sum())
+    total = len(nl) * E * _SHARED_END + steps * E * _SHARED_STEP
+    classes = 0
+    if keys:
+        u = torch.unique(torch.cat(keys), dim=0)
+        classes = int(u.shape[0])
+        total += float(L[u[:, 9].long().cpu()].sum()) * _SHARED_WAVE
+    two = ip[nl == 2][:, 1].long().cpu()
+    return total + float(L[two].sum()) * _SHARED_WAVE, classes

@@ -31,3 +31,18 @@ def test_mean_over_scatterers_per_energy():
     ipots = np.array([[0, 1, 2, 0]])                          # a three-leg path through potentials 1 and 2
     want = flops_per_energy(3, (10 + 20) / 2) + flops_per_energy(3, (5 + 25) / 2)
     assert abs(path_flops([3], ipots, lmax)[0] - want) < 1e-6
+
+
+def test_shared_operations_count_each_different_scatterer_once():
+    from feffgpu_b200.roofline import _SHARED_END, _SHARED_STEP, _SHARED_WAVE, shared_flops
+    lmax = np.array([[0, 9, 19], [0, 4, 24]])
+    c = np.zeros((3, 4, 3))
+    c[0, 1:4] = c[1, 1:4] = [[2, 0, 0], [2, 2, 0], [0, 2, 0]]
+    c[1, 3] = [0, 0, 2]                                        # shares (0, a, b) with the first path
+    c[2, 1] = [0, 0, 2]                                        # two legs
+    ip = np.array([[0, 1, 2, 1], [0, 1, 2, 1], [0, 2, 0, 0]])
+    got, classes = shared_flops(c, [4, 4, 2], ip, [0, 0, 0], lmax)
+    waves = {1: 15, 2: 45}
+    assert classes == 5
+    want = _SHARED_WAVE * (waves[1] + 2 * (waves[2] + waves[1]) + waves[2]) + 6 * 2 * _SHARED_STEP + 3 * 2 * _SHARED_END
+    assert abs(got - want) < 1e-6

@@ -81,7 +81,8 @@ class _ChiReduceAllRanks(torch.autograd.Function):
     def forward(ctx, coords, sigma2, q, S, stage, batch, prec, group):
         need = ctx.needs_input_grad[0] or (sigma2 is not None and ctx.needs_input_grad[1])
         words, cchi, reff = stage._chi_reduce_words(batch, coords, sigma2, q, S, prec, save=need)
-        if dist.is_available() and dist.is_initialized() and dist.get_world_size(group) > 1:
+        ctx.split = dist.is_available() and dist.is_initialized() and dist.get_world_size(group) > 1
+        if ctx.split:
             dist.all_reduce(words, op=dist.ReduceOp.SUM, group=group)     # 64-bit integers: exact, any order
         if need:
             ctx.save_for_backward(coords, sigma2, q, S, cchi, reff)
@@ -93,9 +94,9 @@ class _ChiReduceAllRanks(torch.autograd.Function):
         # every rank holds the same loss of the summed rows: its paths receive the upstream gradient
         coords, sigma2, q, S, cchi, reff = ctx.saved_tensors
         want_s2 = sigma2 is not None and ctx.needs_input_grad[1]
-        # the one-kernel adjoint: a path's gradient is then the same bits whichever rank evaluates it
+        # over several ranks the one-kernel adjoint: a path's gradient is then the same bits whichever rank evaluates it
         gc, gs = ctx.stage._chi_reduce_backward(ctx.batch, coords, sigma2, q, S, ctx.prec, g, cchi, reff, want_s2,
-                                                one_kernel=True)
+                                                one_kernel=ctx.split)
         return (gc if ctx.needs_input_grad[0] else None), (gs if want_s2 else None), None, None, None, None, None, None
 
 

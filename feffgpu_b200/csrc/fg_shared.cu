@@ -21,13 +21,12 @@ __global__ void __launch_bounds__(256) k_share_insert(ShareIdx s)
 {
     if (s.refused()) return;
     const int64_t total = s.n * s.nsc_max;
+    unsigned mine = 0;                                   // scatterers of this thread, at most 2^21 in all
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = t / s.nsc_max;
         const int nleg = s.legs(s.order ? s.order[i] : i);
-        const bool live = nleg > 2 && (int)(t % s.nsc_max) < nleg - 1;
-        const unsigned votes = __ballot_sync(__activemask(), live);
-        if (!live) continue;
-        if ((threadIdx.x & 31) == __ffs(votes) - 1) atomicAdd((unsigned long long *)&s.head->scatterers, (unsigned long long)__popc(votes));
+        if (nleg <= 2 || (int)(t % s.nsc_max) >= nleg - 1) continue;
+        ++mine;
         const ShareKey k = s.key[t];
         unsigned h = key_hash(k) & s.hmask;
         for (unsigned probe = 0; probe <= s.hmask; ++probe, h = (h + 1) & s.hmask) {
@@ -43,6 +42,8 @@ __global__ void __launch_bounds__(256) k_share_insert(ShareIdx s)
         }
         s.slot_of[t] = (int)h;
     }
+    mine = __reduce_add_sync(0xffffffffu, mine);         // after the loop, where the whole warp is together again
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd((unsigned long long *)&s.head->scatterers, (unsigned long long)mine);
 }
 }  // namespace
 

@@ -125,3 +125,9 @@ def test_potential_index_errors_raise_index_error():
             L.check(L.FG_ERR_VALUE)
     finally:
         L._lib.fg_last_error = orig
+
+
+def test_no_warp_vote_over_the_lanes_that_happen_to_run():
+    """Which lanes __activemask() names where a loop's lanes diverge is not defined, so nothing is counted with it."""
+    csrc = HEADER.parents[1] / "feffgpu_b200" / "csrc"
+    assert [p.name for p in sorted(csrc.iterdir()) if "__activemask" in p.read_text()] == []

@@ -99,9 +99,11 @@ class _Gather(torch.autograd.Function):
         x = pos.detach().contiguous()
         out = torch.empty(b.n, b.nleg_max, 3, device=x.device, dtype=torch.float64)
         box = float(mi.cell) if mi.cell is not None and mi.cell18 is None else -1.0
-        _lib.check(_lib.load().fg_path_gather(b.n, b.nleg_max, x.data_ptr(), model.atoms.data_ptr(), b.nleg.data_ptr(),
-                                              box, None if mi.cell18 is None else mi.cell18.data_ptr(),
-                                              out.data_ptr(), torch.cuda.current_stream(x.device).cuda_stream))
+        with torch.cuda.device(x.device):        # the entry point takes no stage: it launches on the current device
+            _lib.check(_lib.load().fg_path_gather(b.n, b.nleg_max, x.data_ptr(), model.atoms.data_ptr(),
+                                                  b.nleg.data_ptr(), box,
+                                                  None if mi.cell18 is None else mi.cell18.data_ptr(),
+                                                  out.data_ptr(), torch.cuda.current_stream(x.device).cuda_stream))
         ctx.model = model
         return out
 
@@ -110,9 +112,10 @@ class _Gather(torch.autograd.Function):
         m = ctx.model
         g = g.contiguous()
         out = torch.empty(m.natoms, 3, device=g.device, dtype=torch.float64)
-        _lib.check(_lib.load().fg_path_scatter(m.natoms, m.batch.nleg_max, m.entry_off.data_ptr(), m.entry.data_ptr(),
-                                               m.batch.nleg.data_ptr(), g.data_ptr(), out.data_ptr(),
-                                               torch.cuda.current_stream(g.device).cuda_stream))
+        with torch.cuda.device(g.device):
+            _lib.check(_lib.load().fg_path_scatter(m.natoms, m.batch.nleg_max, m.entry_off.data_ptr(),
+                                                   m.entry.data_ptr(), m.batch.nleg.data_ptr(), g.data_ptr(),
+                                                   out.data_ptr(), torch.cuda.current_stream(g.device).cuda_stream))
         return out, None
 
 

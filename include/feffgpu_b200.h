@@ -351,7 +351,8 @@ FG_API fg_status fg_path_geometry_backward(int64_t B, int32_t nleg, const double
 /* Coordinates (n, nleg_max, 3) FP64 of paths held as atom indices atoms (n, nleg_max), absorber first, at positions pos
  * (N, 3) FP64: relative to the absorber under the minimum image (box: a cubic length, not positive for none; cell: the
  * cell's rows and its inverse, 18 doubles, or NULL), zero at slots past nleg[p] (exafs/forward.py:664-725).  The indices
- * are the caller's to keep within the positions. */
+ * are the caller's to keep within the positions.  Takes no stage: the arrays and `stream` belong to the current device, as
+ * in fg_path_scatter. */
 FG_API fg_status fg_path_gather(int64_t n, int32_t nleg_max, const double *pos, const int64_t *atoms,
                                 const int32_t *nleg, double box, const double *cell, double *coords, void *stream);
 /* Its adjoint: grad_pos (natoms, 3) from grad_coords (n, nleg_max, 3).  off (natoms + 1) and entry: for every atom the

@@ -110,6 +110,8 @@ class _Gather(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         m = ctx.model
+        if m.batch.n == 0:                       # no slot holds an atom, and the empty arrays have no address
+            return torch.zeros(m.natoms, 3, device=g.device, dtype=torch.float64), None
         g = g.contiguous()
         out = torch.empty(m.natoms, 3, device=g.device, dtype=torch.float64)
         with torch.cuda.device(g.device):

@@ -45,6 +45,19 @@ def test_gather_and_scatter(box, counts):
     assert torch.all(g0[16:] == 0)
 
 
+def test_a_model_without_paths_has_zero_rows_and_gradient():
+    from feffgpu_b200 import GPUPathStage
+    from feffgpu_b200.model import PathModel
+    st = GPUPathStage(phase("cfg4_fe_phase"), device="cuda")
+    m = PathModel(st, [(np.zeros((0, 3), int), np.zeros((0, 3), int))], np.eye(4, 3), nrows=2)
+    x = torch.tensor(np.eye(4, 3), device="cuda", requires_grad=True)
+    q = torch.arange(1, 12, dtype=torch.float64, device="cuda")
+    rows = m.rows(x, q, st.linear_matrix(q.cpu().numpy()).double())
+    assert rows.shape == (2, 11) and torch.all(rows == 0)
+    g, = torch.autograd.grad(rows.sum(), x)
+    assert g.shape == (4, 3) and torch.all(g == 0)
+
+
 def test_out_of_range_atoms_are_refused():
     from feffgpu_b200 import GPUPathStage
     from feffgpu_b200.model import PathModel

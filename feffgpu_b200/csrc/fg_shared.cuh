@@ -104,7 +104,7 @@ template <typename R, typename CT>
 __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, const CT *__restrict__ coords,
                                                     const int64_t *__restrict__ ipots, int *status, int PB)
 {
-    if (status && (*(volatile const int *)status & kBadLayout)) return;
+    if (s.refused()) return;            // not by status: the drop-in call's is the caller's word, whatever it holds
     extern __shared__ __align__(16) unsigned char smem[];
     double *half = reinterpret_cast<double *>(smem + (size_t)PB * s.rec_bytes);      // cos, sin of beta_nleg / 2
     const int tid = threadIdx.x, nl = s.nsc_max + 1;

@@ -256,3 +256,25 @@ def test_forms_replay_in_a_graph(counts):
         r0, g0 = rows.clone(), gx.clone()
         r1, g1 = step()
         assert torch.equal(r0, r1) and torch.equal(g0, g1)
+
+
+def test_drop_in_signal_leaves_the_callers_word_alone():
+    """bad_ipot is the caller's, whatever it holds: it does not steer the call, and only a bad index is added to it."""
+    from feffgpu_b200 import GPUPathStage, _lib
+    P = phase("case_A014")
+    st = GPUPathStage(P, device="cuda")
+    nleg, B = 4, 700
+    c, ip, _, _ = _list(P.nph, {nleg: B}, 6, seed=3)[0]
+    c, ip = torch.tensor(c, device="cuda", dtype=st.rdtype), torch.tensor(ip, device="cuda")
+    ref, rr = st.cchi(c, ip)
+    bytes_ = int(st._lib.fg_cchi_workspace(st._h, B, nleg))
+    assert bytes_ > 0
+    for before in (0, 2, -1):
+        word = torch.tensor([before], device="cuda", dtype=torch.int32)
+        ws = torch.zeros(bytes_, dtype=torch.uint8, device="cuda")
+        got, rf = torch.empty_like(ref), torch.empty_like(rr)
+        _lib.check(st._lib.fg_cchi_ws(st._h, st.prec, B, nleg, c.data_ptr(), 0, ip.data_ptr(), got.data_ptr(),
+                                      rf.data_ptr(), word.data_ptr(), ws.data_ptr(), bytes_,
+                                      torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(got, ref) and torch.equal(rf, rr)
+        assert int(word) == before

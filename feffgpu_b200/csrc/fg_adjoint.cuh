@@ -1269,7 +1269,7 @@ fg_status cchi_bwd_call(const StageView &sv, const Tables<R> &T, int64_t B, int 
     FG_CUDA(cudaMemsetAsync(ws, 0, kCounterBytes, st));
     if constexpr (EDGE <= 3) {
         const SharePlan pl = share_plan(B, nleg, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit, true);
-        if (pl.sub && ws_bytes >= kCounterBytes + pl.total) {
+        if (pl.sub && ws_bytes >= kCounterBytes + pl.total && share_aligned(ws)) {
             unsigned char *sw = ws + kCounterBytes;
             ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
             Share<R> s = share_view<R, EDGE>(pl, sw, head, status, sv.L1);
@@ -1351,7 +1351,7 @@ fg_status Launch<R, EDGE>::fused_bwd(const StageView &sv, const Tables<R> &T, co
     const size_t used = fused_bwd_workspace(P, NK, sv.E);
     const SharePlan pl = share_plan(P->n, P->nleg_max, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit, true);
     if constexpr (EDGE <= 3)
-        if (pl.sub && ws_bytes >= used + pl.total) {
+        if (pl.sub && ws_bytes >= used + pl.total && share_aligned(ws)) {
             ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
             Share<R> s = share_view<R, EDGE>(pl, ws + used, head, status, sv.L1);
             s.stride = P->nleg_max;

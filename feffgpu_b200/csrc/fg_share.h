@@ -5,6 +5,10 @@
 
 namespace fg {
 
+// The workspace of the shared and staged forms holds 16-byte words (records, keys, matrices); the one-kernel forms need no
+// more than 8-byte alignment, so a call whose workspace does not start on a 16-byte boundary takes those.
+inline bool share_aligned(const void *ws) { return (reinterpret_cast<uintptr_t>(ws) & 15) == 0; }
+
 // The workspace as the kernels of one sub-batch see it.
 template <typename R> struct Share : ShareIdx {
     unsigned char *rec;          // n records of rec_bytes (WarpPath<R>)
@@ -80,7 +84,7 @@ fg_status cchi_call(const StageView &sv, const Tables<R> &T, int64_t B, int nleg
 {
     const SharePlan pl = ws ? share_plan(B, nleg, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit) : SharePlan{};
     if constexpr (EDGE <= 3)
-        if (pl.sub && ws_bytes >= kCounterBytes + pl.total) {
+        if (pl.sub && ws_bytes >= kCounterBytes + pl.total && share_aligned(ws)) {
             ShareHead *head = reinterpret_cast<ShareHead *>(ws);
             Share<R> s = share_view<R, EDGE>(pl, ws + kCounterBytes, head, nullptr, sv.L1);
             s.stride = s.nleg_uniform = nleg;
@@ -134,7 +138,7 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
     }
     if (fg_status rc = launch_validate(P, sv.nph1, status, st)) return rc;
     const SharePlan pl = P->n > 0 ? share_plan(P->n, P->nleg_max, sv.E, sv.L1, sizeof(R) == 8, sv.iorder, sv.ilinit, false, NK) : SharePlan{};
-    if (pl.sub && share_ws && share_bytes >= pl.total) {
+    if (pl.sub && share_ws && share_bytes >= pl.total && share_aligned(share_ws)) {
         if constexpr (EDGE <= 3) {
             ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
             Share<R> s = share_view<R, EDGE>(pl, share_ws, head, status, sv.L1);

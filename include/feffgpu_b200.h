@@ -97,7 +97,8 @@ FG_API fg_status fg_cchi(const fg_stage *stage, fg_precision prec, int64_t B, in
 FG_API fg_status fg_stage_check_range(const fg_stage *stage, int64_t n, int64_t hi, const int64_t *values,
                                       int32_t *inside, void *stream);
 /* The same call with device scratch: with workspace_bytes >= fg_cchi_workspace(...) (0: it would not be used) equal
- * scatterers of the paths are evaluated once and small calls spread their energies over the GPU; with less, as fg_cchi.
+ * scatterers of the paths are evaluated once and small calls spread their energies over the GPU; with less, or with a
+ * workspace that does not start on a 16-byte boundary, as fg_cchi (so too in the calls below).
  * The workspace is free again when the call's work on `stream` is done. */
 FG_API size_t fg_cchi_workspace(const fg_stage *stage, int64_t B, int32_t nleg);
 FG_API fg_status fg_cchi_ws(const fg_stage *stage, fg_precision prec, int64_t B, int32_t nleg, const void *coords,

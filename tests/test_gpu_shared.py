@@ -278,3 +278,48 @@ def test_drop_in_signal_leaves_the_callers_word_alone():
                                       torch.cuda.current_stream().cuda_stream))
         assert torch.equal(got, ref) and torch.equal(rf, rr)
         assert int(word) == before
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_workspace_on_an_8_byte_boundary(dtype):
+    """Every call with a workspace of full size that starts 8 bytes past a 16-byte boundary: the one-kernel form's bits."""
+    from feffgpu_b200 import GPUPathStage, PathBatch, _lib
+    from feffgpu_b200.pad import resample_phase
+    P = resample_phase(phase("cfg2_phase"), np.linspace(0.0, 20.0, 131))
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    b = PathBatch(_list(P.nph, {2: 7, 4: 500}, 7, seed=4), nrows=3, device="cuda")
+    q = torch.arange(1, 202, dtype=torch.float64, device="cuda") * 0.1
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    g = torch.randn(3, 201, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    ref, cc, rf, offered = _rows(st, b, q, S, False)
+    gref, _, _ = _grads(st, b, q, S, False, g, None)
+    span, tspan, ps = st._span(S), st._span(S, True), st._paths_struct(b, b.coords, None)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def odd(n):
+        return torch.empty(n + 8, dtype=torch.uint8, device="cuda")[8:]
+
+    assert offered
+    ws = odd(int(st._lib.fg_chi_reduce_workspace(st._h, C.byref(ps), 201)))
+    rows = torch.empty_like(ref)
+    _lib.check(st._lib.fg_chi_reduce(st._h, st.prec, C.byref(ps), 201, q.data_ptr(), S.data_ptr(), span.data_ptr(),
+                                     rows.data_ptr(), None, None, ws.data_ptr(), ws.numel(), stream))
+    ws = odd(int(st._lib.fg_chi_reduce_backward_workspace(st._h, C.byref(ps), 201)))
+    gc = torch.empty_like(gref)
+    _lib.check(st._lib.fg_chi_reduce_backward(st._h, st.prec, C.byref(ps), 201, q.data_ptr(), S.data_ptr(),
+                                              span.data_ptr(), tspan.data_ptr(), g.data_ptr(), cc.data_ptr(),
+                                              rf.data_ptr(), gc.data_ptr(), None, ws.data_ptr(), ws.numel(), stream))
+    assert ws.data_ptr() % 16 == 8 and torch.equal(rows, ref) and torch.equal(gc, gref)
+    sel = (b.nleg == 4).nonzero().squeeze(1)
+    c, ip = b.coords[sel, :4].to(st.rdtype).contiguous(), b.ipots[sel, :4].contiguous()
+    n = len(sel)
+    ws, sig, reff = odd(int(st._lib.fg_cchi_workspace(st._h, n, 4))), *map(torch.empty_like, st.cchi(c, ip))
+    _lib.check(st._lib.fg_cchi_ws(st._h, st.prec, n, 4, c.data_ptr(), int(dtype == torch.complex128), ip.data_ptr(),
+                                  sig.data_ptr(), reff.data_ptr(), None, ws.data_ptr(), ws.numel(), stream))
+    assert torch.equal(sig, st.cchi(c, ip)[0])
+    gs = torch.randn(n, st.E, 2, dtype=st.rdtype, device="cuda", generator=torch.Generator("cuda").manual_seed(6))
+    ws, x, y = odd(int(st._lib.fg_cchi_backward_workspace(st._h, n, 4))), torch.empty_like(c), torch.empty_like(c)
+    for out, w, size in ((x, ws, ws.numel()), (y, torch.empty(256, dtype=torch.uint8, device="cuda"), 256)):
+        _lib.check(st._lib.fg_cchi_backward(st._h, st.prec, n, 4, c.data_ptr(), int(dtype == torch.complex128),
+                                            ip.data_ptr(), gs.data_ptr(), None, out.data_ptr(), w.data_ptr(), size, stream))
+    assert torch.equal(x, y)

@@ -1274,6 +1274,7 @@ fg_status cchi_bwd_call(const StageView &sv, const Tables<R> &T, int64_t B, int 
             ShareHead *head = reinterpret_cast<ShareHead *>(ws + kShareHeadOffset);
             Share<R> s = share_view<R, EDGE>(pl, sw, head, status, sv.L1);
             s.stride = s.nleg_uniform = nleg;
+            timer_begin(st);
             for (int64_t t0 = 0; t0 < B; t0 += pl.sub) {
                 s.n = std::min<int64_t>(pl.sub, B - t0);
                 const CT *c = coords + t0 * nleg * 3;
@@ -1291,8 +1292,8 @@ fg_status cchi_bwd_call(const StageView &sv, const Tables<R> &T, int64_t B, int 
                                                                    st, nullptr, &head->general))
                         return rc;
                 }
-                timer_end(st);               // begun in adjoint
             }
+            timer_end(st);
             return FG_OK;
         }
     }
@@ -1356,6 +1357,7 @@ fg_status Launch<R, EDGE>::fused_bwd(const StageView &sv, const Tables<R> &T, co
             Share<R> s = share_view<R, EDGE>(pl, ws + used, head, status, sv.L1);
             s.stride = P->nleg_max;
             s.nlegs = P->nleg;
+            timer_begin(st);
             for (int64_t t0 = 0; t0 < P->n; t0 += pl.sub) {
                 s.n = std::min<int64_t>(pl.sub, P->n - t0);
                 s.order = P->order + t0;
@@ -1364,8 +1366,8 @@ fg_status Launch<R, EDGE>::fused_bwd(const StageView &sv, const Tables<R> &T, co
                     return rc;
                 if (!pl.force)
                     if (fg_status rc = general(t0, s.n, &head->general)) return rc;
-                timer_end(st);                   // begun in adjoint
             }
+            timer_end(st);
             return FG_OK;
         }
     return general(0, P->n, nullptr);

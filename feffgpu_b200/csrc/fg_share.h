@@ -88,6 +88,7 @@ fg_status cchi_call(const StageView &sv, const Tables<R> &T, int64_t B, int nleg
             ShareHead *head = reinterpret_cast<ShareHead *>(ws);
             Share<R> s = share_view<R, EDGE>(pl, ws + kCounterBytes, head, nullptr, sv.L1);
             s.stride = s.nleg_uniform = nleg;
+            timer_begin(st);
             for (int64_t t0 = 0; t0 < B; t0 += pl.sub) {
                 s.n = std::min<int64_t>(pl.sub, B - t0);
                 const CT *c = coords + t0 * nleg * 3;
@@ -99,8 +100,8 @@ fg_status cchi_call(const StageView &sv, const Tables<R> &T, int64_t B, int nleg
                     if (fg_status rc = launch_cchi<R, EDGE, CT>(sv, T, s.n, nleg, c, ip, out, reff + t0, bad, warps,
                                                                 &head->general, st))
                         return rc;
-                timer_end(st);               // begun in signals: whichever form evaluated the paths
             }
+            timer_end(st);
             return FG_OK;
         }
     timer_begin(st);
@@ -146,6 +147,7 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
             s.nlegs = P->nleg;
             s.by_path = cchi_save != nullptr;
             C2<R> *sig = cchi_save ? static_cast<C2<R> *>(cchi_save) : reinterpret_cast<C2<R> *>(share_ws + pl.sig);
+            timer_begin(st);
             for (int64_t t0 = 0; t0 < P->n; t0 += pl.sub) {
                 s.n = std::min<int64_t>(pl.sub, P->n - t0);
                 s.order = P->order + t0;
@@ -162,8 +164,8 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
                                                              status, shape, &head->general, st))
                         return rc;
                 }
-                timer_end(st);                   // begun in signals: whichever form evaluated the paths, and the fine grid
             }
+            timer_end(st);
         }
     } else if (P->n > 0) {
         const PathsDev pd{P->n, P->nleg_max, P->nrows, P->coords, P->ipots, P->nleg, P->deg, P->sigma2, P->order, P->row};

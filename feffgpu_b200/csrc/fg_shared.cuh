@@ -531,7 +531,6 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
         const int ew = fit_warps(4, wb, sv.max_smem);
         int eb = 0;
         if (fg_status rc = grid_for(ke, 32 * ew, wb * ew, sv.num_sms, s.n * pl.split, eb)) return rc;
-        timer_begin(st);
         ke<<<eb, 32 * ew, wb * ew, st>>>(T, s, pl.split, out, wb);
         FG_CUDA(cudaGetLastError());
         return FG_OK;
@@ -550,7 +549,6 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
     const int split = pl.split;
     const size_t wc = 4 * s.rec_bytes;
     if (fg_status rc = grid_for(kc, 128, wc, sv.num_sms, s.n * split, cb)) return rc;
-    timer_begin(st);
     for (int pass = 0; pass < pl.passes; ++pass) {
         kf<<<fb, 32 * fw, wb * fw, st>>>(T, s, pass, out, wb);
         kc<<<cb, 128, wc, st>>>(T, s, pass, split, out);
@@ -1110,7 +1108,6 @@ fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T,
     const size_t wc = 4 * s.rec_bytes;
     if (fg_status rc = grid_for(kc, 128, wc, sv.num_sms, s.n * split, bc)) return rc;
     if (fg_status rc = grid_for(k2, 32 * n2, w2 * n2, sv.num_sms, s.n * split, b2)) return rc;
-    timer_begin(st);
     k2<<<b2, 32 * n2, w2 * n2, st>>>(T, s, split, gbar, gpar, w2);
     for (int pass = 0; pass < pl.passes; ++pass) {
         if (pass == 0) {                                     // beside the two-leg paths' kernel, not after it

@@ -211,9 +211,10 @@ FG_API fg_status fg_chi_reduce_backward(const fg_stage *stage, fg_precision prec
                                  const void *cchi_saved, const double *reff_saved, double *grad_coords,
                                  double *grad_sigma2, void *workspace, size_t workspace_bytes, void *stream);
 
-/* Device timing of the library's main kernel (the per-path kernel of each call), for profiling and autotuning:
- * while enabled, every call records CUDA events around its main kernel on the call's stream; fg_kernel_time_ms
- * waits for the last recorded end event and returns the elapsed milliseconds. */
+/* Device timing of the kernels that evaluate a call's paths, for profiling and autotuning: while enabled, every call
+ * records CUDA events on its stream before the first and after the last of them (one kernel, or, where equal scatterers
+ * are evaluated once or short paths in stages, everything from the first path's geometry to the last path's fine grid or
+ * gradient); fg_kernel_time_ms waits for the last recorded end event and returns the elapsed milliseconds. */
 FG_API fg_status fg_set_kernel_timing(int32_t enable);
 FG_API fg_status fg_kernel_time_ms(float *ms);
 

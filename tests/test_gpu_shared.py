@@ -323,3 +323,39 @@ def test_workspace_on_an_8_byte_boundary(dtype):
         _lib.check(st._lib.fg_cchi_backward(st._h, st.prec, n, 4, c.data_ptr(), int(dtype == torch.complex128),
                                             ip.data_ptr(), gs.data_ptr(), None, out.data_ptr(), w.data_ptr(), size, stream))
     assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("backward", [False, True])
+@pytest.mark.parametrize("case,counts", [("cfg4_fe_phase", {3: 33000}), ("case_A014", {4: (1 << 18) + 5})],
+                         ids=["staged", "shared"])
+def test_kernel_timing_spans_every_sub_batch(case, counts, backward):
+    """A list one sub-batch and a little more: the time is of all of it, most of what the call takes on the device (the
+    rest are the check, the sums' clearing and reading out, and in the backward the fine grid's adjoint)."""
+    from feffgpu_b200 import GPUPathStage, PathBatch, _lib
+    if backward and 3 in counts:
+        pytest.skip("the staged form has no backward")
+    st = GPUPathStage(phase(case), device="cuda")
+    b = PathBatch(_list(st.P.nph, counts, 7, seed=9), nrows=3, device="cuda")
+    q = torch.arange(1, 21, dtype=torch.float64, device="cuda")
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    g = torch.ones(3, 20, dtype=torch.float64, device="cuda")
+    _, cc, rf = st._chi_reduce_forward(b, b.coords, None, q, S, st.prec, True)
+
+    def call():
+        if backward:
+            st._chi_reduce_backward(b, b.coords, None, q, S, st.prec, g, cc, rf, False)
+        else:
+            st._chi_reduce_forward(b, b.coords, None, q, S, st.prec, False)
+
+    call()
+    e0, e1, ms = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True), C.c_float()
+    st._lib.fg_set_kernel_timing(1)
+    try:
+        e0.record()
+        call()
+        e1.record()
+        e1.synchronize()
+        _lib.check(st._lib.fg_kernel_time_ms(C.byref(ms)))
+    finally:
+        st._lib.fg_set_kernel_timing(0)
+    assert 0.5 * e0.elapsed_time(e1) <= ms.value <= e0.elapsed_time(e1)

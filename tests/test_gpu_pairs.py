@@ -109,3 +109,25 @@ def test_pair_tables_equal_the_two_leg_paths_of_the_path_stage():
     xg = x.clone().requires_grad_(True)
     (pt.single_scattering(xg) ** 2).sum().backward()
     assert torch.isfinite(xg.grad).all() and float(xg.grad.abs().max()) > 0
+
+
+@pytest.mark.parametrize("boxes", [1.0, 1e5, 1e6, 1e8, 1e10])
+def test_image_of_pairs_many_boxes_apart(boxes):
+    """Pairs half a box from a tie between two images, up to 1e10 boxes apart as an unwrapped trajectory leaves them: the
+    image is the one that the quotient r / b rounds to, seen in the direction of the gradient (no tolerance)."""
+    from feffgpu_b200 import _lib
+    rng = np.random.default_rng(7)
+    n, b = 20000, 8.3
+    x = b * (np.floor(rng.uniform(0.1, 1.0, n) * boxes) + 0.5)
+    x += rng.integers(-3, 4, n) * np.spacing(x)
+    pos = np.zeros((n, 2, 3))
+    pos[:, 1, 0] = x
+    want = np.sign(x - b * np.rint(x / b))
+    t = torch.tensor(pos, device="cuda")
+    D = torch.arange(40, dtype=torch.float64, device="cuda")
+    ip = torch.ones(2, dtype=torch.int32, device="cuda")
+    g = torch.zeros_like(t)
+    _lib.check(_lib.load().fg_pair_ss_grad(t.data_ptr(), n, 2, b, None, ip.data_ptr(), 1, D.data_ptr(), 1.0, 0.25, 40,
+                                           0.9 * b, 1.0, g.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    got = g.cpu().numpy()
+    assert np.array_equal(np.sign(got[:, 0, 0]), -want) and np.array_equal(np.sign(got[:, 1, 0]), want)

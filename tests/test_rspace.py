@@ -100,3 +100,40 @@ def test_misfit_kernel_pinned_to_the_reference_losses():
             ref_v, ref_g = z[f"R{key}_{i}"], z[f"grad{key}_{i}"]
             np.testing.assert_allclose(v.detach().cpu().numpy(), ref_v, rtol=tol, atol=0)
             assert np.abs(x.grad.cpu().numpy() - ref_g).max() <= tol * np.abs(ref_g).max()
+
+
+def _raw(rows, F, t, grad=True):
+    from feffgpu_b200 import _lib
+    B, NK = rows.shape
+    R = torch.empty(B, device="cuda", dtype=torch.float64)
+    g = torch.empty_like(rows) if grad else None
+    _lib.check(_lib.load().fg_rspace_misfit(B, NK, F.shape[0], rows.data_ptr(), F.data_ptr(), t.data_ptr(), 1.0,
+                                            R.data_ptr(), g.data_ptr() if grad else None,
+                                            torch.cuda.current_stream().cuda_stream))
+    return R, g
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("NK,NR", [(401, 163), (1, 1), (65, 7), (130, 66), (513, 8)])
+def test_a_row_has_the_same_bits_whatever_the_number_of_rows(NK, NR):
+    """Up to 148 rows go to a cluster of blocks each, more to a block each: the same sums in the same order."""
+    gen = torch.Generator("cuda").manual_seed(NK)
+    rows = torch.randn(149, NK, device="cuda", dtype=torch.float64, generator=gen)
+    F = torch.randn(NR, NK, 2, device="cuda", dtype=torch.float64, generator=gen)
+    t = torch.randn(NR, 2, device="cuda", dtype=torch.float64, generator=gen)
+    R, g = _raw(rows, F, t)
+    parts = [_raw(r.contiguous(), F, t) for r in (rows[:148], rows[148:])]
+    assert torch.equal(R, torch.cat([p[0] for p in parts])) and torch.equal(g, torch.cat([p[1] for p in parts]))
+    d = torch.einsum("mkc,bk->bmc", F, rows) - t
+    ref = (d ** 2).sum((1, 2))
+    gref = 2 * torch.einsum("bmc,mkc->bk", d, F)
+    assert (R - ref).abs().max() <= 1e-12 * ref.max() and (g - gref).abs().max() <= 1e-11 * gref.abs().max()
+
+
+@pytest.mark.gpu
+def test_more_rows_than_clusters_of_eight_fit_a_grid():
+    B = 1 << 28
+    rows = torch.arange(B, device="cuda", dtype=torch.float64)[:, None] % 1021
+    one = torch.tensor([[[1.0, 0.0]]], device="cuda", dtype=torch.float64)
+    R, _ = _raw(rows, one, torch.zeros(1, 2, device="cuda", dtype=torch.float64), grad=False)
+    assert torch.equal(R, rows[:, 0] ** 2)

@@ -167,23 +167,36 @@ __device__ __forceinline__ void amp_phase_block(int E, const Load &load, A *amp,
     __syncthreads();
 }
 
-// A block per path: the front ends call it on chunks of tens to thousands of paths, and a warp per path spent most of a
-// call in thirteen rounds of arc tangents and sines one after the other (59 paths x 60 energies x 401 points: 18 us; 3,152
-// x 401 x 401 in FP64: 59 us); now 8 and 36 us.
-template <typename R>
-__global__ void __launch_bounds__(128) k_chi_fine(int64_t B, int E, const C2<R> *__restrict__ cchi,
-                                                   const R *__restrict__ reff, int NK, const R *__restrict__ q,
-                                                   const R *__restrict__ S, const int *__restrict__ span,
-                                                   R *__restrict__ chi)
+// A block or, WARP, a warp per path, the same operations in the same order.  The front ends call it on chunks of tens to
+// thousands of paths, where a warp per path spends most of a call in thirteen rounds of arc tangents and sines one after
+// the other (B200, 60 energies x 401 points, 600 paths: 18.7 us, 7.8 with a block; 401 energies, 2,400 paths: 27.7 and
+// 23.1); with paths enough for every warp slot the block's three warps that wait for the first one's unwrapping are what
+// costs (60 energies, 65,536 paths: 218 us with a warp, 252 with a block; 401 energies: 488 and 549).  The two meet at
+// 10,000 to 15,000 paths.
+constexpr int kFineWarp = 96;              // paths per SM from which a warp takes a path
+template <typename R, bool WARP>
+__global__ void __launch_bounds__(WARP ? 256 : 128) k_chi_fine(int64_t B, int E, const C2<R> *__restrict__ cchi,
+                                                               const R *__restrict__ reff, int NK,
+                                                               const R *__restrict__ q, const R *__restrict__ S,
+                                                               const int *__restrict__ span, R *__restrict__ chi,
+                                                               size_t bytes)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    double *pha = reinterpret_cast<double *>(smem);
+    const int w = WARP ? threadIdx.x >> 5 : 0, nw = WARP ? blockDim.x >> 5 : 1;
+    const int tid = WARP ? threadIdx.x & 31 : threadIdx.x, threads = WARP ? 32 : blockDim.x;
+    double *pha = reinterpret_cast<double *>(smem + (size_t)w * bytes);
     R *amp = reinterpret_cast<R *>(pha + E);
-    for (int64_t p = blockIdx.x; p < B; p += gridDim.x) {
+    for (int64_t p = (int64_t)blockIdx.x * nw + w; p < B; p += (int64_t)gridDim.x * nw) {
         const C2<R> *c = cchi + p * E;
-        amp_phase_block<R>(E, [&](int e) { return c[e]; }, amp, pha);
+        auto load = [&](int e) { return c[e]; };
+        if constexpr (WARP) {
+            amp_phase<R>(E, tid, load, amp, pha);
+            __syncwarp();
+        } else {
+            amp_phase_block<R>(E, load, amp, pha);
+        }
         const double rf = (double)reff[p];
-        for (int k = threadIdx.x; k < NK; k += blockDim.x) {
+        for (int k = tid; k < NK; k += threads) {
             const int lo = span[2 * k], hi = span[2 * k + 1];
             double a = 0.0, ph = 0.0;
             for (int j = lo; j < hi; ++j) {
@@ -193,7 +206,8 @@ __global__ void __launch_bounds__(128) k_chi_fine(int64_t B, int E, const C2<R> 
             }
             chi[p * NK + k] = (R)(a * sin_arg<R>(ph + 2.0 * (double)q[k] * rf));
         }
-        __syncthreads();
+        if constexpr (WARP) __syncwarp();
+        else __syncthreads();
     }
 }
 
@@ -337,12 +351,16 @@ template <typename R>
 fg_status LaunchCommon<R>::chi_fine(const StageView &sv, int64_t B, const void *cchi, const void *reff, int NK,
                                     const void *q, const void *S, const int *span, void *chi, cudaStream_t st)
 {
-    const size_t smem = (size_t)sv.E * (sizeof(R) + sizeof(double));
-    auto kern = k_chi_fine<R>;
+    const size_t bytes = align_up((size_t)sv.E * (sizeof(R) + sizeof(double)), 16);
+    const bool warp = B >= (int64_t)kFineWarp * sv.num_sms;
+    const int warps = warp ? fit_warps(8, bytes, sv.max_smem) : 4;
+    const size_t smem = bytes * (warp ? warps : 1);
+    auto kern = warp ? k_chi_fine<R, true> : k_chi_fine<R, false>;
     int blocks = 0;
-    if (fg_status rc = grid_for(kern, 128, smem, sv.num_sms, B * 4, blocks)) return rc;
-    kern<<<blocks, 128, smem, st>>>(B, sv.E, static_cast<const C2<R> *>(cchi), static_cast<const R *>(reff), NK,
-                                    static_cast<const R *>(q), static_cast<const R *>(S), span, static_cast<R *>(chi));
+    if (fg_status rc = grid_for(kern, 32 * warps, smem, sv.num_sms, warp ? B : B * 4, blocks)) return rc;
+    kern<<<blocks, 32 * warps, smem, st>>>(B, sv.E, static_cast<const C2<R> *>(cchi), static_cast<const R *>(reff), NK,
+                                           static_cast<const R *>(q), static_cast<const R *>(S), span,
+                                           static_cast<R *>(chi), bytes);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }

@@ -47,3 +47,20 @@ def test_chi_fine_and_its_gradient(dtype, NK):
     tol = 1e-10 if dtype == torch.complex128 else 1e-5
     for a, b in zip(got, ref):
         assert torch.allclose(a, b, rtol=0, atol=tol * float(b.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("NK", [1, 33, 401])
+def test_a_path_has_the_same_bits_whatever_the_number_of_paths(dtype, NK):
+    """Calls of 96 paths per SM and more take a warp per path instead of a block: the same operations in the same order."""
+    from feffgpu_b200 import GPUPathStage
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    B = 96 * torch.cuda.get_device_properties(0).multi_processor_count + 3
+    gen = torch.Generator("cuda").manual_seed(NK)
+    c = torch.view_as_complex(torch.randn(B, E, 2, device="cuda", dtype=st.rdtype, generator=gen))
+    rf = 2.0 + 3.0 * torch.rand(B, device="cuda", dtype=st.rdtype, generator=gen)
+    q = torch.linspace(0.5, 15.0, NK, dtype=torch.float64)
+    S = st.linear_matrix(q.numpy())
+    got = st.chi_fine(c, rf, q, S)
+    parts = [st.chi_fine(c[i:i + 5000], rf[i:i + 5000], q, S) for i in range(0, B, 5000)]
+    assert torch.isfinite(got).all() and torch.equal(got, torch.cat(parts))

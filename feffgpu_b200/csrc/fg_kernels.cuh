@@ -60,10 +60,8 @@ __device__ __forceinline__ C2<R> path_energy(const WarpPath<R> &g, const R *dh, 
 template <typename R, int EDGE, typename CT>
 __global__ void __launch_bounds__(256) k_cchi(Tables<R> T, const CT *__restrict__ coords,
                                                const int64_t *__restrict__ ipots, int64_t B, int nleg,
-                                               C2<R> *__restrict__ out, R *__restrict__ reff, int *bad, size_t wbytes,
-                                               const int *gate)
+                                               C2<R> *__restrict__ out, R *__restrict__ reff, int *bad, size_t wbytes)
 {
-    if (gate && !*(volatile const int *)gate) return;       // the shared-matrix form took the call
     using K = Kinds<EDGE>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -271,12 +269,11 @@ __global__ void __launch_bounds__(128, MINB)
     k_fused(Tables<R> T, PathsDev P, int NK, const double *__restrict__ q, const double *__restrict__ S,
             const int *__restrict__ span, unsigned long long *__restrict__ racc, C2<R> *__restrict__ cchi_save,
             double *__restrict__ reff_save, unsigned long long *counter, int *status, int nsc_max, size_t wbytes,
-            int stage_t, const int *gate)
+            int stage_t)
 {
     using K = Kinds<EDGE>;
     extern __shared__ __align__(16) unsigned char smem[];
     if (*(volatile const int *)status & kBadLayout) return;
-    if (gate && !*(volatile const int *)gate) return;       // the shared-matrix form took the call
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int E = T.E, L1 = T.L1;
     unsigned char *base = smem + (size_t)w * wbytes;
@@ -326,12 +323,11 @@ inline fg_status grid_for(KernelT kern, int threads, size_t smem, int num_sms, i
     return FG_OK;
 }
 
-// The one-kernel form over pd's paths; gate: it returns at once unless *gate is set (null: always runs).
+// The one-kernel form over pd's paths.
 template <typename R, int EDGE>
 fg_status launch_fused(const StageView &sv, const Tables<R> &T, const PathsDev &pd, int NK, const double *q,
                        const double *S, const int *span, unsigned long long *racc, void *cchi_save, double *reff_save,
-                       unsigned long long *counter, int *status, const FusedShape &shape, const int *gate,
-                       cudaStream_t st)
+                       unsigned long long *counter, int *status, const FusedShape &shape, cudaStream_t st)
 {
     using K = Kinds<EDGE>;
     const int nsc_max = pd.nleg_max - 1;
@@ -342,7 +338,7 @@ fg_status launch_fused(const StageView &sv, const Tables<R> &T, const PathsDev &
     int blocks = 0;
     if (fg_status rc = grid_for(kern, threads, wb * warps, sv.num_sms, pd.n, blocks)) return rc;
     kern<<<blocks, threads, wb * warps, st>>>(T, pd, NK, q, S, span, racc, static_cast<C2<R> *>(cchi_save), reff_save,
-                                              counter, status, nsc_max, wb, shape.stage_t ? 1 : 0, gate);
+                                              counter, status, nsc_max, wb, shape.stage_t ? 1 : 0);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }

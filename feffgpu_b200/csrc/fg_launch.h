@@ -131,7 +131,7 @@ constexpr int64_t kStageSub = 1 << 15;                     // paths per sub-batc
 constexpr int64_t kShareSmall = 8192;                      // (path, 32 energies) items of a small call
 constexpr size_t kShareMatrixBytes = (size_t)1 << 30;      // the classes' matrices: 2e5 classes, 32 energies, FP32
 struct ShareHead {                      // counters of one sub-batch, in the workspace head
-    int classes, two, general, pad;     // classes, two-leg paths, 1: the one-kernel form evaluates this sub-batch
+    int classes, two, general, pad;     // classes, two-leg paths, 1: the shared form is not taken for this sub-batch
     long long scatterers;               // scatterers of paths of three and more legs
 };
 constexpr size_t kShareHeadOffset = 128;
@@ -159,7 +159,8 @@ fg_status launch_share_insert(const ShareIdx &s, cudaStream_t st);
 // Sizes and offsets of the shared form's workspace for calls of n paths of up to nleg_max legs; sub: paths per
 // sub-batch (0: the form does not apply).
 struct SharePlan {
-    int64_t sub = 0, cls_cap = 0;
+    int64_t sub = 0, cls_cap = 0, part = 0;      // part, part_split: paths at a time, and parts of a path's energies, of
+    int part_split = 1;                          // the staged kernels where classes were looked for and not found
     int nsc_max = 0, chunks = 0, passes = 0, split = 1, force = 0, mats = 1, staged = 0;
     unsigned hcap = 0;
     size_t rec = 0, key = 0, slot = 0, hash = 0, cls = 0, owner = 0, two = 0, tab = 0, F = 0, f_bytes = 0, sig = 0,

@@ -44,8 +44,9 @@ Share<R> share_view(const SharePlan &pl, unsigned char *ws, ShareHead *head, con
     return s;
 }
 
-// One sub-batch.  Where the form is not taken, signals and adjoint set head->general and write nothing else; coords,
-// ipots and the gradients are whole arrays indexed by path (order picks the sub-batch) or the sub-batch's own.
+// One sub-batch.  Where the shared form is not taken, signals goes on in the staged form, and adjoint sets head->general and
+// writes nothing else; coords, ipots and the gradients are whole arrays indexed by path (order picks the sub-batch) or the
+// sub-batch's own.
 template <typename R, int EDGE> struct ShareLaunch {
     template <typename CT>
     static fg_status signals(const StageView &sv, const Tables<R> &T, const SharePlan &pl, Share<R> &s, const CT *coords,
@@ -61,10 +62,10 @@ template <typename R, int EDGE> struct ShareLaunch {
 };
 
 // ------------------------------------------------------------------------------------------------ forward calls
-// The one-kernel form of the drop-in call; gate as in launch_fused.
+// The one-kernel form of the drop-in call.
 template <typename R, int EDGE, typename CT>
 fg_status launch_cchi(const StageView &sv, const Tables<R> &T, int64_t B, int nleg, const CT *coords,
-                      const int64_t *ipots, C2<R> *cchi, R *reff, int *bad, int warps, const int *gate, cudaStream_t st)
+                      const int64_t *ipots, C2<R> *cchi, R *reff, int *bad, int warps, cudaStream_t st)
 {
     using K = Kinds<EDGE>;
     const size_t wb = warp_bytes<R>(sv.L1, nleg - 1, nleg == 2 ? K::MMSS : K::MMMS, sv.E, false);
@@ -72,7 +73,7 @@ fg_status launch_cchi(const StageView &sv, const Tables<R> &T, int64_t B, int nl
     int blocks = 0;
     auto kern = k_cchi<R, EDGE, CT>;
     if (fg_status rc = grid_for(kern, warps * 32, wb * warps, sv.num_sms, B, blocks)) return rc;
-    kern<<<blocks, warps * 32, wb * warps, st>>>(T, coords, ipots, B, nleg, cchi, reff, bad, wb, gate);
+    kern<<<blocks, warps * 32, wb * warps, st>>>(T, coords, ipots, B, nleg, cchi, reff, bad, wb);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
@@ -96,16 +97,12 @@ fg_status cchi_call(const StageView &sv, const Tables<R> &T, int64_t B, int nleg
                 C2<R> *out = cchi + t0 * sv.E;
                 if (fg_status rc = ShareLaunch<R, EDGE>::template signals<CT>(sv, T, pl, s, c, ip, bad, out, st)) return rc;
                 if (fg_status rc = ShareLaunch<R, EDGE>::reff(s, reff + t0, st)) return rc;
-                if (!pl.force)
-                    if (fg_status rc = launch_cchi<R, EDGE, CT>(sv, T, s.n, nleg, c, ip, out, reff + t0, bad, warps,
-                                                                &head->general, st))
-                        return rc;
             }
             timer_end(st);
             return FG_OK;
         }
     timer_begin(st);
-    if (fg_status rc = launch_cchi<R, EDGE, CT>(sv, T, B, nleg, coords, ipots, cchi, reff, bad, warps, nullptr, st)) return rc;
+    if (fg_status rc = launch_cchi<R, EDGE, CT>(sv, T, B, nleg, coords, ipots, cchi, reff, bad, warps, st)) return rc;
     timer_end(st);
     return FG_OK;
 }
@@ -158,12 +155,6 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
                 if (fg_status rc = ShareLaunch<R, EDGE>::fine(sv, s, pd, NK, q, S, span, share_ws + pl.pts, t0 == 0, sig, racc,
                                                               reff_save, status, st))
                     return rc;
-                if (!pl.force) {
-                    if (t0) FG_CUDA(cudaMemsetAsync(counter, 0, sizeof(*counter), st));
-                    if (fg_status rc = launch_fused<R, EDGE>(sv, T, pd, NK, q, S, span, racc, cchi_save, reff_save, counter,
-                                                             status, shape, &head->general, st))
-                        return rc;
-                }
             }
             timer_end(st);
         }
@@ -171,7 +162,7 @@ fg_status Launch<R, EDGE>::fused(const StageView &sv, const Tables<R> &T, const 
         const PathsDev pd{P->n, P->nleg_max, P->nrows, P->coords, P->ipots, P->nleg, P->deg, P->sigma2, P->order, P->row};
         timer_begin(st);
         if (fg_status rc = launch_fused<R, EDGE>(sv, T, pd, NK, q, S, span, racc, cchi_save, reff_save, counter, status,
-                                                 shape, nullptr, st))
+                                                 shape, st))
             return rc;
         timer_end(st);
     }

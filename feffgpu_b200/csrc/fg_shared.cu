@@ -96,6 +96,13 @@ SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iord
     const size_t per = p.mats * 20 * 2 * real * 32;          // one class, one chunk: 20 canonical entries (orders 0-2)
     const size_t all = (size_t)scat * p.chunks * per;
     p.f_bytes = std::min(all, adjoint ? 2 * kShareMatrixBytes : kShareMatrixBytes);
+    if (!adjoint) {
+        // one path's tables in the staged form (as few parts as can be: where the form is taken, each is two idle launches)
+        const size_t tables = (size_t)p.nsc_max * (L1 + 1) * dstride(ilinit == 1 ? 2 : 3) * real;
+        p.f_bytes = std::max(p.f_bytes, tables);
+        p.part = std::min<int64_t>(p.sub, (int64_t)(p.f_bytes / tables));
+        p.part_split = (int)std::min<int64_t>(chunks, (kShareItems / 4 + p.part - 1) / p.part);
+    }
     p.cls_cap = std::min<int64_t>(scat, (int64_t)(p.f_bytes / per));
     const int fit = (int)std::min<size_t>(p.chunks, p.f_bytes / ((size_t)scat * per));   // chunks per pass at worst
     p.passes = fit ? (p.chunks + fit - 1) / fit : p.chunks;

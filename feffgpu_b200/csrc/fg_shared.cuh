@@ -100,7 +100,8 @@ __device__ __forceinline__ void share_keys(const Share<R> &s, const WarpPath<R> 
 // Records, keys and the list of two-leg paths (a batch that k_validate refused is left alone).  A block takes PB paths
 // at a time, a thread per (path, leg) where path_setup has a warp per path with a lane per leg: same operations, most of
 // the lanes busy (128,844 paths of up to eight legs: 134 us, 292 us with a warp per path).
-template <typename R, typename CT>
+// KEYS: the keys and the list of two-leg paths alone (the adjoint, whose records are made once the form is taken).
+template <typename R, typename CT, bool KEYS>
 __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, const CT *__restrict__ coords,
                                                     const int64_t *__restrict__ ipots, int *status, int PB)
 {
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, con
             };
             const LegGeom lg = leg_geometry<double>(rat, j, nleg);
             g.ri[j] = lg.ri; g.beta[j] = lg.beta; g.alpha[j] = lg.alpha; g.gamma[j] = lg.gamma;
-            if (j == nleg) {
+            if (!KEYS && j == nleg) {
                 half[2 * l] = cos(0.5 * lg.beta);
                 half[2 * l + 1] = sin(0.5 * lg.beta);
             }
@@ -149,14 +150,16 @@ __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, con
             const int l = t / nl, j = t % nl + 1, nleg = s.legs(s.path(i0 + l));
             if (j > nleg) continue;
             WarpPath<R> &g = rec(l);
-            const double eta = g.alpha[j == 1 ? nleg : j - 1] + g.gamma[j];
-            double sn, cs;
-            sincos(eta, &sn, &cs);
-            g.phs[j] = C2<R>{(R)cs, (R)(-sn)};
-            if (j == 1) {
-                double r = 0.0;
-                for (int q = 1; q <= nleg; ++q) r += g.ri[q];
-                g.reff = 0.5 * r;
+            if constexpr (!KEYS) {
+                const double eta = g.alpha[j == 1 ? nleg : j - 1] + g.gamma[j];
+                double sn, cs;
+                sincos(eta, &sn, &cs);
+                g.phs[j] = C2<R>{(R)cs, (R)(-sn)};
+                if (j == 1) {
+                    double r = 0.0;
+                    for (int q = 1; q <= nleg; ++q) r += g.ri[q];
+                    g.reff = 0.5 * r;
+                }
             }
             if (s.key) {
                 if (nleg == 2) {
@@ -166,14 +169,16 @@ __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, con
                 }
             }
         }
-        for (int t = tid; t < cnt * T.nterm * 49; t += 128) {
-            const int l = t / (T.nterm * 49), q = t % (T.nterm * 49), e = q % 49;
-            rec(l).dterm[q / 49][e] = (R)wigner_small(T.term_l[q / 49], e / 7 - 3, e % 7 - 3, half[2 * l], half[2 * l + 1],
-                                                      seed_table(T));
+        if constexpr (!KEYS) {
+            for (int t = tid; t < cnt * T.nterm * 49; t += 128) {
+                const int l = t / (T.nterm * 49), q = t % (T.nterm * 49), e = q % 49;
+                rec(l).dterm[q / 49][e] = (R)wigner_small(T.term_l[q / 49], e / 7 - 3, e % 7 - 3, half[2 * l],
+                                                          half[2 * l + 1], seed_table(T));
+            }
+            __syncthreads();
+            for (size_t t = tid; t < cnt * s.rec_bytes / 16; t += 128)
+                reinterpret_cast<uint4 *>(s.rec + i0 * s.rec_bytes)[t] = reinterpret_cast<const uint4 *>(smem)[t];
         }
-        __syncthreads();
-        for (size_t t = tid; t < cnt * s.rec_bytes / 16; t += 128)
-            reinterpret_cast<uint4 *>(s.rec + i0 * s.rec_bytes)[t] = reinterpret_cast<const uint4 *>(smem)[t];
         __syncthreads();
     }
 }
@@ -184,7 +189,7 @@ template <typename R, int KIND> __global__ void __launch_bounds__(128) k_share_t
     constexpr int MM = lamtab(KIND).MM, NC = ncanon(MM), DS = dstride(MM);
     if (s.refused()) return;
     if (!share_chunks<R, KIND>(s)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) s.head->general = 1;       // the one-kernel form that follows runs
+        if (blockIdx.x == 0 && threadIdx.x == 0) s.head->general = 1;       // the staged kernels that follow run
         return;
     }
     const int64_t tasks = (int64_t)s.head->classes * NC;
@@ -316,44 +321,61 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 2)
 // of 2,048 absorbers, 60 energies, 401 points, mixed: 15.0 -> 9.5 ms (energies 5.5, fine grid 1.9, tables 1.1, geometry
 // 0.7 ms); 4,438 paths of up to four legs: 178 -> 140 us.  What bounds it: the energies' FP32 multiply-adds and their
 // fixed latencies at 12 (three legs) and 8 warps per SM.
-template <typename R, int EDGE> __global__ void __launch_bounds__(128) k_stage_tables(Tables<R> T, Share<R> s)
+//
+// The kernels take the positions i0 .. i0 + n of the sub-batch, whose tables (tab_len entries a scatterer) are at tab; gate:
+// they return at once unless *gate is set (the shared form's kernels, which ran before them, found too little to share).
+template <typename R> struct StagePart {
+    R *tab;
+    int tab_len;
+    int64_t i0, n;
+    const int *gate;
+    __device__ __forceinline__ bool off(const Share<R> &s) const
+    {
+        return s.refused() || (gate && !*(volatile const int *)gate);
+    }
+};
+
+template <typename R, int EDGE>
+__global__ void __launch_bounds__(128) k_stage_tables(Tables<R> T, Share<R> s, StagePart<R> part)
 {
     using K = Kinds<EDGE>;
     constexpr int NC = ncanon(K::MM);
-    if (s.refused()) return;
-    const int64_t tasks = s.n * s.nsc_max * NC;
+    if (part.off(s)) return;
+    const int64_t tasks = part.n * s.nsc_max * NC;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tasks; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = t / NC, i = c / s.nsc_max;
+        const int64_t c = t / NC, i = part.i0 + c / s.nsc_max;
         const int r = (int)(t % NC), k = (int)(c % s.nsc_max) + 1, nleg = s.legs(s.path(i));
         const int MM = nleg == 2 ? K::MMSS : K::MMMS;
         if (k >= nleg || r >= ncanon(MM)) continue;
         const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(s.rec + i * s.rec_bytes);
-        rotation_column<R>(s.tab + c * s.tab_len, T, g.beta[k], MM, dstride(MM), r);
+        rotation_column<R>(part.tab + c * part.tab_len, T, g.beta[k], MM, dstride(MM), r);
     }
 }
 
 // SHORT: no path has more than three legs
 template <typename R, int EDGE, bool SHORT>
-__global__ void __launch_bounds__(128, FusedMinBlocks<R>::def) k_stage_energies(Tables<R> T, Share<R> s, int split,
-                                                                                C2<R> *__restrict__ out, size_t wbytes)
+__global__ void __launch_bounds__(128, FusedMinBlocks<R>::def) k_stage_energies(Tables<R> T, Share<R> s, StagePart<R> part,
+                                                                                int split, C2<R> *__restrict__ out,
+                                                                                size_t wbytes)
 {
     using K = Kinds<EDGE>;
-    if (s.refused()) return;
+    if (part.off(s)) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, E = T.E;
     unsigned char *base = smem + (size_t)w * wbytes;
     const WarpPath<R> &g = *reinterpret_cast<const WarpPath<R> *>(base);
     R *dh = reinterpret_cast<R *>(base + s.rec_bytes);
-    for (int64_t it = (int64_t)blockIdx.x * nw + w; it < s.n * split; it += (int64_t)gridDim.x * nw) {
-        const int64_t i = it / split, o = s.row(i) * E;
+    // all paths' first part of the energies, then the next part: parts differ by a chunk, and every warp gets of each
+    for (int64_t it = (int64_t)blockIdx.x * nw + w; it < part.n * split; it += (int64_t)gridDim.x * nw) {
+        const int64_t j = it % part.n, i = part.i0 + j, o = s.row(i) * E;
         const int nleg = s.legs(s.path(i)), MM = nleg == 2 ? K::MMSS : K::MMMS;
         copy16(base, s.rec + i * s.rec_bytes, s.rec_bytes, lane);
         // the tables of a path's scatterers, one after the other as the energies read them
         const int len = (T.L1 + 1) * dstride(MM);
         for (int k = 0; k < nleg - 1; ++k)
-            copy16(dh + k * len, s.tab + (i * s.nsc_max + k) * s.tab_len, (size_t)len * sizeof(R), lane);
+            copy16(dh + k * len, part.tab + (j * s.nsc_max + k) * part.tab_len, (size_t)len * sizeof(R), lane);
         __syncwarp();
-        for (int gc = (int)(it % split); gc < s.chunks; gc += split) {
+        for (int gc = (int)(it / part.n); gc < s.chunks; gc += split) {
             const int e = first_chunk(E) + 32 * gc + lane;
             if (e < 0 || e >= E) continue;
             if (nleg > 2) {
@@ -394,14 +416,13 @@ static __global__ void k_fine_points(int NK, int E, const double *__restrict__ q
 // together -- a row's 401 points take one addition each per block and not per path, which is what a small batch on one row
 // waits for: 4,438 paths on 60 energies 84 -> 25 us; 537,000 paths on 64 rows 2.29 -> 1.94 ms (4.3 ms a warp per path with
 // S read in place).  On 401 energies (128,844 paths, 1.29 ms) the FP64 arc tangents and square roots of the phases bound it.
-template <typename R, int KIND, int PG, bool ACC>
-__global__ void __launch_bounds__(256) k_share_fine(Share<R> s, PathsDev P, int E, int NK, const double *__restrict__ S,
-                                                    const FinePoint *__restrict__ pts, const C2<R> *__restrict__ cchi,
-                                                    unsigned long long *__restrict__ racc,
-                                                    double *__restrict__ reff_save, int *status, int64_t range,
-                                                    size_t wbytes)
+template <typename R, int PG, bool ACC>
+__global__ void __launch_bounds__(256, PG == 1 ? 4 : 2)          // the blocks that the records and sums leave room for
+    k_share_fine(Share<R> s, PathsDev P, int E, int NK, const double *__restrict__ S, const FinePoint *__restrict__ pts,
+                 const C2<R> *__restrict__ cchi, unsigned long long *__restrict__ racc, double *__restrict__ reff_save,
+                 int *status, int64_t range, size_t wbytes)
 {
-    if (s.refused() || (s.key && !share_chunks<R, KIND>(s))) return;
+    if (s.refused()) return;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int last_row[8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, E2 = (E + 1) & ~1;
@@ -495,14 +516,51 @@ __global__ void __launch_bounds__(256) k_share_fine(Share<R> s, PathsDev P, int 
 }
 
 // reff of the drop-in call from the records
-template <typename R, int KIND> __global__ void k_share_reff(Share<R> s, R *__restrict__ reff)
+template <typename R> __global__ void k_share_reff(Share<R> s, R *__restrict__ reff)
 {
-    if (s.key && !share_chunks<R, KIND>(s)) return;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < s.n; p += (int64_t)gridDim.x * blockDim.x)
         reff[p] = (R)(reinterpret_cast<const WarpPath<R> *>(s.rec + p * s.rec_bytes)->reff * kBohr);
 }
 
 // ------------------------------------------------------------------------------------------------ launches
+// Records, keys and two-leg list (or the keys alone): paths per block such that a thread has a leg, fewer where the paths
+// do not fill the chip that way.
+template <bool KEYS, typename R, typename CT>
+fg_status launch_geom(const StageView &sv, const Tables<R> &T, const Share<R> &s, const CT *coords, const int64_t *ipots,
+                      int *status, cudaStream_t st)
+{
+    const int PB = (int)std::max<int64_t>(1, std::min<int64_t>(128 / (s.nsc_max + 1), s.n / (sv.num_sms * 4)));
+    const size_t gb = PB * (s.rec_bytes + 16);
+    int blocks = 0;
+    auto kg = k_share_geom<R, CT, KEYS>;
+    if (fg_status rc = grid_for(kg, 128, gb, sv.num_sms, (s.n + PB - 1) / PB * 4, blocks)) return rc;
+    kg<<<blocks, 128, gb, st>>>(T, s, coords, ipots, status, PB);
+    FG_CUDA(cudaGetLastError());
+    return FG_OK;
+}
+
+// The staged form's tables and energies of a part of the sub-batch
+template <typename R, int EDGE>
+fg_status launch_stage(const StageView &sv, const Tables<R> &T, const Share<R> &s, const StagePart<R> &part, int split,
+                       C2<R> *out, cudaStream_t st)
+{
+    using K = Kinds<EDGE>;
+    const int64_t tasks = part.n * s.nsc_max * ncanon(K::MM);
+    auto kt = k_stage_tables<R, EDGE>;
+    int tb = 0;
+    if (fg_status rc = grid_for(kt, 128, 0, sv.num_sms, (tasks + 31) / 32, tb)) return rc;
+    kt<<<tb, 128, 0, st>>>(T, s, part);
+    FG_CUDA(cudaGetLastError());
+    auto ke = s.nsc_max <= 2 ? k_stage_energies<R, EDGE, true> : k_stage_energies<R, EDGE, false>;
+    const size_t wb = s.rec_bytes + align_up((size_t)s.nsc_max * part.tab_len * sizeof(R), 16);
+    const int ew = fit_warps(4, wb, sv.max_smem);
+    int eb = 0;
+    if (fg_status rc = grid_for(ke, 32 * ew, wb * ew, sv.num_sms, part.n * split, eb)) return rc;
+    ke<<<eb, 32 * ew, wb * ew, st>>>(T, s, part, split, out, wb);
+    FG_CUDA(cudaGetLastError());
+    return FG_OK;
+}
+
 template <typename R, int EDGE>
 template <typename CT>
 fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T, const SharePlan &pl, Share<R> &s, const CT *coords,
@@ -514,27 +572,9 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
         FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
         FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
     }
-    // paths per block of the geometry: a thread per leg, fewer where the paths do not fill the chip that way
-    const int PB = (int)std::max<int64_t>(1, std::min<int64_t>(128 / (s.nsc_max + 1), s.n / (sv.num_sms * 4)));
-    const size_t gb = PB * (s.rec_bytes + 16);
-    int blocks = 0;
-    auto kg = k_share_geom<R, CT>;
-    if (fg_status rc = grid_for(kg, 128, gb, sv.num_sms, (s.n + PB - 1) / PB * 4, blocks)) return rc;
-    kg<<<blocks, 128, gb, st>>>(T, s, coords, ipots, status, PB);
-    FG_CUDA(cudaGetLastError());
-    if (pl.staged) {
-        const int64_t tasks = s.n * s.nsc_max * ncanon(K::MM);
-        k_stage_tables<R, EDGE><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
-        FG_CUDA(cudaGetLastError());
-        auto ke = s.nsc_max <= 2 ? k_stage_energies<R, EDGE, true> : k_stage_energies<R, EDGE, false>;
-        const size_t wb = s.rec_bytes + align_up((size_t)s.nsc_max * s.tab_len * sizeof(R), 16);
-        const int ew = fit_warps(4, wb, sv.max_smem);
-        int eb = 0;
-        if (fg_status rc = grid_for(ke, 32 * ew, wb * ew, sv.num_sms, s.n * pl.split, eb)) return rc;
-        ke<<<eb, 32 * ew, wb * ew, st>>>(T, s, pl.split, out, wb);
-        FG_CUDA(cudaGetLastError());
-        return FG_OK;
-    }
+    if (fg_status rc = launch_geom<false>(sv, T, s, coords, ipots, status, st)) return rc;
+    if (pl.staged)
+        return launch_stage<R, EDGE>(sv, T, s, StagePart<R>{s.tab, s.tab_len, 0, s.n, nullptr}, pl.split, out, st);
     if (fg_status rc = launch_share_insert(s, st)) return rc;
     const int64_t tasks = std::min<int64_t>(s.n * s.nsc_max, s.cls_cap) * ncanon(K::MMMS);
     k_share_tables<R, KIND><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
@@ -554,6 +594,17 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
         kc<<<cb, 128, wc, st>>>(T, s, pass, split, out);
     }
     FG_CUDA(cudaGetLastError());
+    if (pl.force) return FG_OK;
+    // Nothing of this happens where the form was taken; where it was not, the records are there already, and the matrices'
+    // memory holds the tables.  (Handing such a list to k_fused instead, which does its own geometry, cost what the search
+    // had taken: 1,500 paths of 3-4 legs, 401 energies: 496 us without the search, 551 with it, 428 now; 5,000 paths 1,020,
+    // 1,083 and 983; 20,000 paths on 60 energies 859, 1,005 and 778.)
+    const int len = (sv.L1 + 1) * dstride(K::MM);
+    static_assert(K::MM <= (EDGE == 1 ? 2 : 3), "the tables that share_plan makes room for");
+    for (int64_t i0 = 0; i0 < s.n; i0 += pl.part) {
+        const StagePart<R> part{reinterpret_cast<R *>(s.F), len, i0, std::min<int64_t>(pl.part, s.n - i0), &s.head->general};
+        if (fg_status rc = launch_stage<R, EDGE>(sv, T, s, part, pl.part_split, out, st)) return rc;
+    }
     return FG_OK;
 }
 
@@ -567,9 +618,8 @@ fg_status ShareLaunch<R, EDGE>::fine(const StageView &sv, const Share<R> &s, con
     // Four paths at a time where their amplitudes and phases are small (537,000 paths, 60 energies: 2.3 ms, two at a time
     // 2.6) and there are paths enough; the rows' sums in shared memory up to 1,024 points.
     const bool four = sv.E <= 128 && s.n >= (int64_t)sv.num_sms * 64, acc = NK <= 1024;
-    using K = Kinds<EDGE>;
-    auto kern = four ? (acc ? k_share_fine<R, K::MS, 4, true> : k_share_fine<R, K::MS, 4, false>)
-                     : (acc ? k_share_fine<R, K::MS, 1, true> : k_share_fine<R, K::MS, 1, false>);
+    auto kern = four ? (acc ? k_share_fine<R, 4, true> : k_share_fine<R, 4, false>)
+                     : (acc ? k_share_fine<R, 1, true> : k_share_fine<R, 1, false>);
     const size_t wb = (size_t)2 * (four ? 4 : 1) * ((sv.E + 1) & ~1) * sizeof(double) + (acc ? (size_t)NK * 16 : 0);
     const int warps = fit_warps(8, wb, sv.max_smem / 2);
     int blocks = 0;
@@ -582,7 +632,7 @@ fg_status ShareLaunch<R, EDGE>::fine(const StageView &sv, const Share<R> &s, con
 
 template <typename R, int EDGE> fg_status ShareLaunch<R, EDGE>::reff(const Share<R> &s, R *out, cudaStream_t st)
 {
-    k_share_reff<R, Kinds<EDGE>::MS><<<(int)std::min<int64_t>((s.n + 255) / 256, 148 * 4), 256, 0, st>>>(s, out);
+    k_share_reff<R><<<(int)std::min<int64_t>((s.n + 255) / 256, 148 * 4), 256, 0, st>>>(s, out);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
@@ -593,7 +643,8 @@ template <typename R, int EDGE> fg_status ShareLaunch<R, EDGE>::reff(const Share
 // running the partial waves again: 60 complex multiply-adds and 480 bytes per scatterer and energy (FP32) against
 // about 25 x 60 multiply-adds.
 //
-//   k_share_geom_adj    a warp per path: the record with the frame and d/dbeta of the termination, the keys
+//   k_share_geom        the keys (k_share_insert then finds the classes)
+//   k_share_geom_adj    a warp per path, once the form is taken: the record with the frame and d/dbeta of the termination
 //   k_share_tables_adj  a thread per (class, entry): D and D'
 //   k_share_f_adj       two warps per (class, 32 energies): (F~, dF~/dbeta) and (dF~/drho_in, dF~/drho_out)
 //   k_share_chain_adj   a warp per (path, energies): energy_ms_adj's sweeps with the matrices read
@@ -604,12 +655,14 @@ template <typename R> __device__ __forceinline__ AdjExtra<R> &adj_extra(unsigned
     return *reinterpret_cast<AdjExtra<R> *>(rec + geo_bytes<R>());
 }
 
-template <typename R, typename CT>
+// taken: the form is taken whatever the keys show, so this kernel writes them (a launch less); otherwise they are there and
+// decide whether the records are needed
+template <typename R, int KIND, typename CT>
 __global__ void __launch_bounds__(128) k_share_geom_adj(Tables<R> T, Share<R> s, const CT *__restrict__ coords,
                                                         const int64_t *__restrict__ ipots, int *status, int MM_ss,
-                                                        int MM_ms)
+                                                        int MM_ms, int taken)
 {
-    if (*(volatile const int *)status & kBadLayout) return;
+    if (s.refused() || (!taken && !share_chunks<R, KIND>(s))) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned char *base = smem + (size_t)w * s.rec_bytes;
@@ -625,7 +678,7 @@ __global__ void __launch_bounds__(128) k_share_geom_adj(Tables<R> T, Share<R> s,
         if (lane == 0) adj_extra<R>(base).frame = frame;
         __syncwarp();
         copy16(s.rec + i * s.rec_bytes, base, s.rec_bytes, lane);
-        share_keys(s, g, i, nleg, lane);
+        if (taken) share_keys(s, g, i, nleg, lane);
         __syncwarp();
     }
 }
@@ -1091,9 +1144,15 @@ fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T,
     FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
     FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
     const int pb = (int)std::min<int64_t>((s.n + 3) / 4, (int64_t)sv.num_sms * 16);
-    k_share_geom_adj<R, CT><<<pb, 128, 4 * s.rec_bytes, st>>>(T, s, coords, ipots, status, K::MMSS, K::MMMS);
-    FG_CUDA(cudaGetLastError());
+    auto records = [&]() -> fg_status {
+        k_share_geom_adj<R, KIND, CT><<<pb, 128, 4 * s.rec_bytes, st>>>(T, s, coords, ipots, status, K::MMSS, K::MMMS, pl.force);
+        FG_CUDA(cudaGetLastError());
+        return FG_OK;
+    };
+    if (fg_status rc = pl.force ? records() : launch_geom<true>(sv, T, s, coords, ipots, status, st)) return rc;
     if (fg_status rc = launch_share_insert(s, st)) return rc;
+    if (!pl.force)
+        if (fg_status rc = records()) return rc;
     const int64_t tasks = std::min<int64_t>(s.n * s.nsc_max, s.cls_cap) * ncanon(K::MMMS);
     k_share_tables_adj<R, KIND><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
     FG_CUDA(cudaGetLastError());

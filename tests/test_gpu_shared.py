@@ -110,8 +110,8 @@ def test_staged_form_equals_one_kernel_form(dtype, case, counts):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_shared_form_over_two_sub_batches_and_without_sharing(dtype):
-    """More paths than one sub-batch holds (2^18); and as many paths with no two scatterers alike, which the call leaves
-    to the one-kernel form after it has counted them."""
+    """More paths than one sub-batch holds (2^18); and paths with no two scatterers alike, with which the call goes on in
+    the staged form after it has counted them."""
     from feffgpu_b200 import GPUPathStage, PathBatch
     P = phase("case_A014")
     st = GPUPathStage(P, device="cuda", dtype=dtype)
@@ -359,3 +359,44 @@ def test_kernel_timing_spans_every_sub_batch(case, counts, backward):
     finally:
         st._lib.fg_set_kernel_timing(0)
     assert 0.5 * e0.elapsed_time(e1) <= ms.value <= e0.elapsed_time(e1)
+
+
+def _own(nph, counts, seed):
+    """Lists of paths with no two scatterers alike (every path has its own 0.05 A displacements)."""
+    rng = np.random.default_rng(seed)
+    return [(c + np.where(np.arange(c.shape[1])[None, :, None] > 0, rng.normal(0, 0.05, c.shape), 0.0), i, d, r)
+            for c, i, d, r in _list(nph, counts, 6, seed=seed)]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case,nk", [("cfg2_phase", 131), ("case_A014", 0)])
+@pytest.mark.parametrize("rest", [3, 1700], ids=["one part", "two parts"])
+def test_list_without_sharing_in_every_call(dtype, case, nk, rest):
+    """Two scatterers a class or more are not there: the forward goes on in the staged form, in as many parts as its tables
+    fit the matrices' memory; the backward in the one-kernel form.  The bits of a call without workspace either way."""
+    from feffgpu_b200 import GPUPathStage, PathBatch, _lib
+    from feffgpu_b200.pad import resample_phase
+    P = resample_phase(phase(case), np.linspace(0.0, 20.0, nk)) if nk else phase(case)
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    real = 4 if dtype == torch.complex64 else 8
+    entries = 16 if st.ilinit == 1 else 28                       # of a table's row, K edge and others
+    cap = (1 << 30) // (8 * (st.L1 + 1) * entries * real)        # nine-leg paths whose tables fit 1 GiB
+    counts = {4: 17000, 2: rest} if rest == 3 else {9: cap + rest}
+    b = PathBatch(_own(P.nph, counts, 11), nrows=3, device="cuda")
+    q = torch.arange(1, 31, dtype=torch.float64, device="cuda") * 0.5
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    got, cc, rf, offered = _rows(st, b, q, S, True)
+    ref, cr, rr, _ = _rows(st, b, q, S, False)
+    assert offered and torch.isfinite(torch.view_as_real(cr)).all()
+    assert torch.equal(cc, cr) and torch.equal(got, ref) and torch.equal(rf, rr)
+    if rest == 3:
+        g = torch.randn(3, 30, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+        a, _, full = _grads(st, b, q, S, True, g, None)
+        assert full and torch.equal(a, _grads(st, b, q, S, False, g, None)[0])
+        sel = (b.nleg == 4).nonzero().squeeze(1)
+        c, ip = b.coords[sel, :4].to(st.rdtype).contiguous(), b.ipots[sel, :4].contiguous()
+        sig, reff = st.cchi(c, ip)
+        x, y = torch.empty_like(sig), torch.empty_like(reff)
+        _lib.check(st._lib.fg_cchi(st._h, st.prec, len(sel), 4, c.data_ptr(), int(real == 8), ip.data_ptr(), x.data_ptr(),
+                                   y.data_ptr(), None, torch.cuda.current_stream().cuda_stream))
+        assert int(st._lib.fg_cchi_workspace(st._h, len(sel), 4)) > 0 and torch.equal(sig, x) and torch.equal(reff, y)

@@ -10,7 +10,9 @@ The adjoint's shape is its warps per CTA, i.e. paths in flight per CTA.  The for
 * the t-matrix source: read through L1, or each scatterer's column copied into a shared-memory tile per warp first
   (asynchronous copies), which takes shared memory from L1.
 
-Which shape is fastest depends on the precision, the leg mix and the energy count.  The autotuner times every
+Only the one-kernel form takes these shapes (small calls, calls without the workspace of the other forms, lambda order 3,
+and the adjoint where it finds too little to share), so that form is what the candidates are timed in.  Which shape is
+fastest depends on the precision, the leg mix and the energy count.  The autotuner times every
 candidate on the device (CUDA events on the current stream, one warm-up and three timed launches each, on a
 stratified sample of the batch), keeps the fastest per workload signature, and persists the choice per GPU model in
 a JSON file (``$FEFFGPU_B200_TUNE_CACHE``, default ``~/.cache/feffgpu_b200/autotune.json``), so a workload is tuned
@@ -147,7 +149,7 @@ def _pick(ms: dict, tol: float = 0.01):
 
 def _time_candidate(kind: str, stage, batch, q, S, prec: int, shape, reps: int = 3) -> float:
     """Milliseconds of the forward (kind 'fwd', shape = (warps, register budget, t staging)) or adjoint ('bwd',
-    shape = warps) call on batch."""
+    shape = warps) call on batch, in the one-kernel form: the other forms' kernels do not take these shapes."""
     lib = stage._lib
     coords = batch.coords.contiguous()
     if kind == "fwd":
@@ -160,13 +162,14 @@ def _time_candidate(kind: str, stage, batch, q, S, prec: int, shape, reps: int =
         with torch.no_grad():
             if kind == "fwd":
                 def run():
-                    stage._chi_reduce_forward(batch, coords, None, q, S, prec, save=False)
+                    stage._chi_reduce_forward(batch, coords, None, q, S, prec, save=False, one_kernel=True)
             else:
                 _, cchi, reff = stage._chi_reduce_forward(batch, coords, None, q, S, prec, save=True)
                 g = torch.ones(batch.nrows, int(q.shape[0]), device=stage.device, dtype=torch.float64)
 
                 def run():
-                    stage._chi_reduce_backward(batch, coords, None, q, S, prec, g, cchi, reff, False)
+                    stage._chi_reduce_backward(batch, coords, None, q, S, prec, g, cchi, reff, False,
+                                               one_kernel=True)
             run()
             ms = []
             for _ in range(reps):

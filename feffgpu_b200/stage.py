@@ -419,13 +419,15 @@ class GPUPathStage:
                                                  ws.data_ptr(), ws.numel(), _stream(self.device)))
         return words, cchi, reff
 
-    def _chi_reduce_forward(self, batch, coords, sigma2, q, S, prec, save: bool):
+    def _chi_reduce_forward(self, batch, coords, sigma2, q, S, prec, save: bool, one_kernel: bool = False):
+        """one_kernel: the one-kernel form whatever the batch (the rows are the same bits)."""
         coords = coords.contiguous()
         NK = q.shape[0]
         ps = self._paths_struct(batch, coords, sigma2)
         rows = torch.empty(batch.nrows, NK, device=self.device, dtype=torch.float64)
-        ws = self._scratch(int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK)),
-                           256 + _up256(16 * batch.nrows * NK))
+        least = 256 + _up256(16 * batch.nrows * NK)
+        full = least if one_kernel else int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK))
+        ws = self._scratch(full, least)
         cchi = reff = None
         if save:
             cchi = torch.empty(batch.n, self.E, device=self.device,

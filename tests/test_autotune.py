@@ -88,3 +88,40 @@ def test_sample_is_stratified():
     # the sampled rows are rows of the batch
     full = {tuple(np.round(c.numpy(), 12).ravel()) for c in b.coords}
     assert all(tuple(np.round(c.numpy(), 12).ravel()) in full for c in s.coords)
+
+
+def test_candidates_are_timed_in_the_form_that_takes_their_shape(monkeypatch):
+    """The forward and the adjoint are timed in the one-kernel form, whatever form the batch's own calls take."""
+    from types import SimpleNamespace
+    calls = []
+
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self):
+            pass
+
+        def synchronize(self):
+            pass
+
+        def elapsed_time(self, other):
+            return 1.0
+
+    class Stage(_Stage):
+        _h, _launch = None, (0, 0, 0, 0)
+        _lib = SimpleNamespace(fg_stage_set_launch=lambda *a: 0, fg_stage_set_fused_variant=lambda *a: 0)
+
+        def _chi_reduce_forward(self, batch, coords, sigma2, q, S, prec, save, one_kernel=False):
+            if not save:
+                calls.append(("fwd", one_kernel))
+            return None, None, None
+
+        def _chi_reduce_backward(self, *args, one_kernel=False):
+            calls.append(("bwd", one_kernel))
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    b, q = _batch({4: 20}), torch.arange(5) * 0.5
+    A._time_candidate("fwd", Stage(), b, q, None, 0, (4, 0, 0))
+    A._time_candidate("bwd", Stage(), b, q, None, 0, 4)
+    assert {k for k, _ in calls} == {"fwd", "bwd"} and all(one for _, one in calls)

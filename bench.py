@@ -895,7 +895,8 @@ def main():
     peak = ctypes.c_double()
     _lib.check(lib.fg_fp32_fma_peak(ctypes.byref(peak), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
     ref_flops = batch_flops(batch.nleg.cpu().numpy(), batch.ipots.cpu().numpy(), stage.lmax.cpu().numpy())
-    flops, classes = shared_flops(batch.coords, batch.nleg, batch.ipots, batch.row, stage.lmax.cpu().numpy())
+    flops, classes = shared_flops(batch.coords, batch.nleg, batch.ipots, stage.lmax.cpu().numpy(), stage.geometry,
+                                  k_edge=stage.ilinit == 1)
     kern_ms = float(np.mean(kern)) if kern else None
     achieved = flops / (kern_ms * 1e-3) / 1e12 if kern_ms else None
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",

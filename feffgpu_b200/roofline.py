@@ -71,38 +71,60 @@ def batch_flops(nleg, ipots, lmax_e_ip) -> float:
 
 # Operations of the form with shared scattering matrices (csrc/fg_shared.cuh), which forms a matrix once per different
 # scatterer and energy.  Per partial wave: 20 canonical entries complex x real + add (4), 6 spherical-wave products and 2
-# with the t-matrix (6 each), and 5 columns of the recursion (an add and a complex multiply-subtract: 10).  Per scatterer
-# and energy of a path: 80 complex multiply-adds (8) and 8 phase turns (12).  Per path and energy: the termination and
-# cfac, about 700.
+# with the t-matrix (6 each), and 5 columns of the recursion (an add and a complex multiply-subtract: 10).  A path of three
+# and more legs multiplies its matrices in two blocks, 4 x 4 and 2 x 2, by columns of the final state's entries (four at
+# the K edge, six at L and M edges): the first matrix is copied, every further one costs 20 complex multiply-adds (8) a
+# column, the last one only the rows that the termination reads (14 at the K edge, all at the others); an Euler phase turns
+# two pairs of entries a column (12 each), after the last matrix one at the K edge.  Per path and energy: the termination
+# and cfac, about 700.
 _SHARED_WAVE = 20 * 4 + 8 * 6 + 5 * 10
-_SHARED_STEP = 80 * 8 + 8 * 12
 _SHARED_END = 700
 
 
-def shared_flops(coords, nleg, ipots, row, lmax_e_ip) -> tuple[float, int]:
-    """(operations, different scatterers) of a batch whose equal scatterers are formed once: coords (n, nleg_max, 3) on
-    any device, rows telling one absorber's coordinates from another's."""
+def _chain_ops(nleg: int, k_edge: bool) -> int:
+    """Operations of one path's chain product at one energy."""
+    if nleg == 2:
+        return 0
+    cols, last_rows, last_turns = (4, 14, 1) if k_edge else (6, 20, 2)
+    first, middle = cols * 2 * 12, cols * (20 * 8 + 2 * 12)
+    return first + (nleg - 3) * middle + cols * (last_rows * 8 + last_turns * 12)
+
+
+def _legs(x):
+    """Leg lengths and the cosines at every atom of paths x (B, nleg, 3), legs 1..nleg (the class of a scatterer up to
+    rounding)."""
     import torch
+    v = torch.cat([x[:, 1:], x[:, :1]], 1) - x
+    r = v.norm(dim=2)
+    u = v / r[:, :, None]
+    return r, (u * torch.roll(u, -1, 1)).sum(2)
+
+
+def shared_flops(coords, nleg, ipots, lmax_e_ip, geometry=None, k_edge: bool = True) -> tuple[float, int]:
+    """(operations, different scatterers) of a batch whose equal scatterers are formed once: coords (n, nleg_max, 3) A on
+    any device.  Scatterers are equal where their two legs, the angle between them and the potential are; geometry maps
+    paths (B, nleg, 3) in bohr to (ri, beta, ...) of legs 1..nleg, as GPUPathStage.geometry (the bits that the library
+    compares; default: the same quantities by torch)."""
+    import torch
+    from .pad import BOHR
     c = torch.as_tensor(coords)
     nl = torch.as_tensor(nleg, device=c.device).long()
     ip = torch.as_tensor(ipots, device=c.device).double()
-    rw = torch.as_tensor(row, device=c.device).double()
-    keys = []
-    for n in sorted(set(nl.tolist())):
-        if n == 2:
-            continue
-        sel = nl == n
-        x = torch.cat([c[sel, :n], c[sel, :1]], 1)
-        for k in range(1, n):
-            keys.append(torch.cat([x[:, k - 1], x[:, k], x[:, k + 1], ip[sel, k:k + 1], rw[sel, None]], 1))
     L = torch.as_tensor(np.asarray(lmax_e_ip, float) + 1.0).sum(0)              # (nph + 1) partial waves over all energies
     E = len(lmax_e_ip)
-    steps = float((nl[nl > 2] - 1).sum())
-    total = len(nl) * E * _SHARED_END + steps * E * _SHARED_STEP
+    keys, total = [], 0.0
+    for n in sorted(set(nl.tolist())):
+        sel = nl == n
+        total += int(sel.sum()) * E * (_SHARED_END + _chain_ops(n, k_edge))
+        if n == 2:
+            continue
+        ri, beta = (geometry or _legs)((c[sel, :n].double() / BOHR).contiguous())[:2]
+        for k in range(1, n):                                                   # legs k - 1 -> k and k -> k + 1
+            keys.append(torch.stack([ri[:, k - 1], ri[:, k], beta[:, k - 1], ip[sel, k]], 1))
     classes = 0
     if keys:
         u = torch.unique(torch.cat(keys), dim=0)
         classes = int(u.shape[0])
-        total += float(L[u[:, 9].long().cpu()].sum()) * _SHARED_WAVE
+        total += float(L[u[:, 3].long().cpu()].sum()) * _SHARED_WAVE
     two = ip[nl == 2][:, 1].long().cpu()
     return total + float(L[two].sum()) * _SHARED_WAVE, classes

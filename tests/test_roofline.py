@@ -34,15 +34,27 @@ def test_mean_over_scatterers_per_energy():
 
 
 def test_shared_operations_count_each_different_scatterer_once():
-    from feffgpu_b200.roofline import _SHARED_END, _SHARED_STEP, _SHARED_WAVE, shared_flops
+    from feffgpu_b200.roofline import _SHARED_END, _SHARED_WAVE, shared_flops
     lmax = np.array([[0, 9, 19], [0, 4, 24]])
     c = np.zeros((3, 4, 3))
-    c[0, 1:4] = c[1, 1:4] = [[2, 0, 0], [2, 2, 0], [0, 2, 0]]
-    c[1, 3] = [0, 0, 2]                                        # shares (0, a, b) with the first path
+    c[0, 1:4] = c[1, 1:4] = [[2, 0, 0], [2, 2, 0], [0, 2, 0]]    # a square: two 2 A legs at a right angle at every corner
+    c[1, 3] = [0, 0, 2]                                        # shares the first corner with the first path
     c[2, 1] = [0, 0, 2]                                        # two legs
     ip = np.array([[0, 1, 2, 1], [0, 1, 2, 1], [0, 2, 0, 0]])
-    got, classes = shared_flops(c, [4, 4, 2], ip, [0, 0, 0], lmax)
+    got, classes = shared_flops(c, [4, 4, 2], ip, lmax)
     waves = {1: 15, 2: 45}
-    assert classes == 5
-    want = _SHARED_WAVE * (waves[1] + 2 * (waves[2] + waves[1]) + waves[2]) + 6 * 2 * _SHARED_STEP + 3 * 2 * _SHARED_END
+    assert classes == 4                                        # corners of potential 1 and 2; two of the second path
+    # a four-leg path at the K edge: the first matrix is copied (phases alone), the second 20 multiply-adds a column, the
+    # last the fourteen that the termination reads and one phase
+    chain = 4 * 24 + 4 * (20 * 8 + 24) + 4 * (14 * 8 + 12)
+    want = _SHARED_WAVE * (2 * waves[1] + 2 * waves[2] + waves[2]) + 2 * 2 * chain + 3 * 2 * _SHARED_END
     assert abs(got - want) < 1e-6
+
+
+def test_chain_operations_follow_the_legs():
+    from feffgpu_b200.roofline import _chain_ops
+    assert _chain_ops(2, True) == 0
+    assert _chain_ops(3, True) == 4 * 24 + 4 * (14 * 8 + 12)
+    assert _chain_ops(3, False) == 6 * 24 + 6 * (20 * 8 + 24)
+    for k_edge, step in ((True, 4 * 184), (False, 6 * 184)):
+        assert all(_chain_ops(n + 1, k_edge) - _chain_ops(n, k_edge) == step for n in range(3, 9))

@@ -77,6 +77,7 @@ class PathBatch:
         self.row = row.to(d)
         self.order = torch.as_tensor(order).to(d)
         self.counts = {int(k): int(v) for k, v in zip(*np.unique(nl_np, return_counts=True))}
+        self._ws = {}
         self._tuned = {}             # launch shapes chosen for this batch, per (stage, precision, k points)
 
     def sample(self, max_paths: int) -> "PathBatch":
@@ -93,6 +94,15 @@ class PathBatch:
             groups.append((self.coords[sel, :n].cpu(), self.ipots[sel, :n].cpu(), self.deg[sel].cpu(),
                            self.row[sel].cpu()))
         return PathBatch(groups, nrows=self.nrows, device=self.device)
+
+    def workspace(self, nbytes: int, backward: bool = False) -> torch.Tensor:
+        """A device scratch buffer of at least nbytes that the batch keeps (one per direction), for callers of the library's
+        entry points; GPUPathStage takes its own for the length of a call."""
+        key = "bwd" if backward else "fwd"
+        ws = self._ws.get(key)
+        if ws is None or ws.numel() < max(nbytes, 1):
+            ws = self._ws[key] = torch.empty(max(nbytes, 1), device=self.device, dtype=torch.uint8)
+        return ws
 
     def __len__(self) -> int:
         return self.n

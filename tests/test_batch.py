@@ -40,3 +40,10 @@ def test_errors():
         PathBatch([(c, np.zeros((1, 10), int))], device="cpu")
     with pytest.raises(ValueError):
         PathBatch([(np.zeros((2, 3, 3)), np.zeros((2, 3), int), None, np.array([0, 5]))], nrows=2, device="cpu")
+
+
+def test_workspace_is_kept_per_direction_and_grows():
+    b = PathBatch([(np.zeros((2, 3, 3)), np.zeros((2, 3), int))], device="cpu")
+    w = b.workspace(100)
+    assert w.numel() >= 100 and w.dtype == torch.uint8 and b.workspace(50) is w
+    assert b.workspace(100, backward=True) is not w and b.workspace(200).numel() >= 200 and b.workspace(0).numel() >= 1

@@ -29,7 +29,7 @@ EXPORTS = ("fg_stage_create", "fg_stage_destroy", "fg_stage_get_info", "fg_stage
            "fg_stage_set_launch", "fg_stage_set_fused_variant", "fg_pf_candidates", "fg_pf_extend", "fg_pf_terminal", "fg_pf_describe",
            "fg_pf_windows", "fg_pair_histogram", "fg_pair_ss_grad", "fg_rspace_misfit",
            "fg_path_columns", "fg_chi_reduce_words", "fg_rows_from_words", "fg_path_geometry", "fg_path_geometry_backward", "fg_shard_lpt", "fg_pf_enumerate_one", "fg_pf_result_gather", "fg_pf_result_destroy",
-           "fg_path_gather", "fg_path_scatter", "fg_stage_check_range")
+           "fg_path_gather", "fg_path_scatter", "fg_stage_check_range", "fg_share_workspace")
 
 
 class PhaseDesc(C.Structure):
@@ -64,6 +64,7 @@ _SIGS = {
     "fg_stage_xk": (C.c_int, [_P, _P]),
     "fg_last_error": (C.c_char_p, []),
     "fg_cchi": (C.c_int, [_P, C.c_int, C.c_int64, C.c_int32, _P, C.c_int32, _P, _P, _P, _P, _P]),
+    "fg_share_workspace": (C.c_size_t, [_P, C.c_int, C.c_int64, C.c_int32, C.c_int32, C.c_int32]),
     "fg_cchi_workspace": (C.c_size_t, [_P, C.c_int64, C.c_int32]),
     "fg_cchi_ws": (C.c_int, [_P, C.c_int, C.c_int64, C.c_int32, _P, C.c_int32, _P, _P, _P, _P, _P, C.c_size_t, _P]),
     "fg_cchi_backward_workspace": (C.c_size_t, [_P, C.c_int64, C.c_int32]),

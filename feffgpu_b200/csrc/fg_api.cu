@@ -519,6 +519,13 @@ extern "C" fg_status fg_stage_check_range(const fg_stage *s, int64_t n, int64_t 
     return FG_OK;
 }
 
+extern "C" size_t fg_share_workspace(const fg_stage *s, fg_precision prec, int64_t n, int32_t nleg_max, int32_t NK,
+                                     int32_t backward)
+{
+    if (!s || n < 0 || nleg_max < 2 || nleg_max > kMaxLeg || NK < 0 || (prec != FG_MIXED && prec != FG_FP64)) return 0;
+    return share_plan(n, nleg_max, s->E, s->L1, prec == FG_FP64, s->iorder, s->ilinit, backward != 0, NK).total;
+}
+
 extern "C" size_t fg_cchi_workspace(const fg_stage *s, int64_t B, int32_t nleg)
 {
     if (!s || B < 0 || nleg < 2 || nleg > kMaxLeg) return 0;

@@ -116,13 +116,16 @@ class GPUPathStage:
                 pass
             self._h = None
 
-    def _scratch(self, full: int, least: int) -> torch.Tensor:
-        """Device scratch of a call, from torch's stream-ordered pool for its length: what lets equal scatterers be
-        evaluated once, or, on a device too full for that, what the one-kernel forms need."""
+    def _scratch(self, least: int, prec: int, n: int, nleg_max: int, NK: int = 0, backward: bool = False,
+                 one_kernel: bool = False) -> torch.Tensor:
+        """Device scratch of a call, from torch's stream-ordered pool for its length: the least bytes that the one-kernel
+        forms need and, unless one_kernel or on a device too full for it, what lets equal scatterers of n paths be
+        evaluated once in this precision."""
+        more = 0 if one_kernel else int(self._lib.fg_share_workspace(self._h, prec, n, nleg_max, NK, int(backward)))
         try:
-            return torch.empty(max(full, least), device=self.device, dtype=torch.uint8)
+            return torch.empty(least + more, device=self.device, dtype=torch.uint8)
         except torch.cuda.OutOfMemoryError:
-            if full <= least:
+            if not more:
                 raise
             return torch.empty(least, device=self.device, dtype=torch.uint8)
 
@@ -158,10 +161,10 @@ class GPUPathStage:
         self._check_ipots(ipots)
         out = torch.empty(B, self.E, device=self.device, dtype=self.cdtype)
         reff = torch.empty(B, device=self.device, dtype=self.rdtype)
-        ws = self._scratch(int(self._lib.fg_cchi_workspace(self._h, B, nleg)), 0)
+        ws = self._scratch(256, self.prec, B, nleg)
         _lib.check(self._lib.fg_cchi_ws(self._h, self.prec, B, nleg, coords.data_ptr(),
                                         int(coords.dtype == torch.float64), ipots.data_ptr(), out.data_ptr(),
-                                        reff.data_ptr(), None, ws.data_ptr() or None, ws.numel(),
+                                        reff.data_ptr(), None, ws.data_ptr(), ws.numel(),
                                         _stream(self.device)))
         return out, reff
 
@@ -172,7 +175,7 @@ class GPUPathStage:
         g_cchi = g_cchi.to(self.cdtype).contiguous()
         g_reff = None if g_reff is None else g_reff.to(self.rdtype).contiguous()
         grad = torch.empty(B, nleg, 3, device=self.device, dtype=self.rdtype)
-        ws = self._scratch(int(self._lib.fg_cchi_backward_workspace(self._h, B, nleg)), 256)
+        ws = self._scratch(256, self.prec, B, nleg, backward=True)
         _lib.check(self._lib.fg_cchi_backward(self._h, self.prec, B, nleg, coords.data_ptr(),
                                               int(coords.dtype == torch.float64), ipots.contiguous().data_ptr(),
                                               g_cchi.data_ptr(), _ptr(g_reff), grad.data_ptr(), ws.data_ptr(), ws.numel(),
@@ -408,7 +411,7 @@ class GPUPathStage:
         NK = q.shape[0]
         ps = self._paths_struct(batch, coords, sigma2)
         words = torch.empty(2, batch.nrows, NK, device=self.device, dtype=torch.int64)
-        ws = self._scratch(int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK)), 256)
+        ws = self._scratch(256, prec, batch.n, batch.nleg_max, NK)
         cchi = reff = None
         if save:
             cchi = torch.empty(batch.n, self.E, device=self.device,
@@ -426,8 +429,7 @@ class GPUPathStage:
         ps = self._paths_struct(batch, coords, sigma2)
         rows = torch.empty(batch.nrows, NK, device=self.device, dtype=torch.float64)
         least = 256 + _up256(16 * batch.nrows * NK)
-        full = least if one_kernel else int(self._lib.fg_chi_reduce_workspace(self._h, C.byref(ps), NK))
-        ws = self._scratch(full, least)
+        ws = self._scratch(least, prec, batch.n, batch.nleg_max, NK, one_kernel=one_kernel)
         cchi = reff = None
         if save:
             cchi = torch.empty(batch.n, self.E, device=self.device,
@@ -451,8 +453,7 @@ class GPUPathStage:
         gc = torch.empty_like(coords)
         gs = torch.empty(batch.n, device=self.device, dtype=torch.float64) if want_s2 else None
         least = 256 + _up256(batch.n * self.E * 16) + _up256(batch.n * 8) + _up256(batch.n * 256)
-        full = least if one_kernel else int(self._lib.fg_chi_reduce_backward_workspace(self._h, C.byref(ps), NK))
-        ws = self._scratch(full, least)
+        ws = self._scratch(least, prec, batch.n, batch.nleg_max, backward=True, one_kernel=one_kernel)
         _lib.check(self._lib.fg_chi_reduce_backward(self._h, prec, C.byref(ps), NK, q.data_ptr(), S.data_ptr(),
                                                     self._span(S).data_ptr(), self._span(S, True).data_ptr(),
                                                     g_rows.contiguous().data_ptr(),

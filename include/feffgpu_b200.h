@@ -96,6 +96,13 @@ FG_API fg_status fg_cchi(const fg_stage *stage, fg_precision prec, int64_t B, in
  * of the stage under way than it keeps words for).  Waits for `stream`. */
 FG_API fg_status fg_stage_check_range(const fg_stage *stage, int64_t n, int64_t hi, const int64_t *values,
                                       int32_t *inside, void *stream);
+/* What the scratch of a call in one precision takes beyond its head and sums where equal scatterers are evaluated once or
+ * paths in stages (0: neither applies): n paths of up to nleg_max legs, NK fine-grid points (0 for fg_cchi_ws and the
+ * backward calls).  A call's full workspace is 256 bytes and this for fg_cchi_ws, fg_cchi_backward and
+ * fg_chi_reduce_words, and the least size given at fg_chi_reduce and fg_chi_reduce_backward and this for those two; the
+ * functions named after the calls return it for the larger of the two precisions. */
+FG_API size_t fg_share_workspace(const fg_stage *stage, fg_precision prec, int64_t n, int32_t nleg_max, int32_t NK,
+                                 int32_t backward);
 /* The same call with device scratch: with workspace_bytes >= fg_cchi_workspace(...) (0: it would not be used) equal
  * scatterers of the paths are evaluated once and small calls spread their energies over the GPU; with less, or with a
  * workspace that does not start on a 16-byte boundary, as fg_cchi (so too in the calls below).

@@ -400,3 +400,62 @@ def test_list_without_sharing_in_every_call(dtype, case, nk, rest):
         _lib.check(st._lib.fg_cchi(st._h, st.prec, len(sel), 4, c.data_ptr(), int(real == 8), ip.data_ptr(), x.data_ptr(),
                                    y.data_ptr(), None, torch.cuda.current_stream().cuda_stream))
         assert int(st._lib.fg_cchi_workspace(st._h, len(sel), 4)) > 0 and torch.equal(sig, x) and torch.equal(reff, y)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case,counts", [("cfg2_phase", {6: 900, 4: 300, 2: 9}), ("cfg4_fe_phase", {3: 3000})],
+                         ids=["classes", "staged"])
+def test_scratch_of_one_precision(dtype, case, counts, monkeypatch):
+    """The stage's calls take scratch for their own precision, which is enough for the form; on a device without room for
+    it they run with the least, and give the same rows (and the one-kernel form's gradients)."""
+    from feffgpu_b200 import GPUPathStage, PathBatch, _lib
+    from feffgpu_b200.pad import resample_phase
+    P = phase(case) if 3 in counts else resample_phase(phase(case), np.linspace(0.0, 20.0, 131))
+    st = GPUPathStage(P, device="cuda", dtype=dtype)
+    b = PathBatch(_list(st.P.nph, counts, 7, seed=12), nrows=3, device="cuda")
+    q = torch.arange(1, 102, dtype=torch.float64, device="cuda") * 0.15
+    S = st.linear_matrix(q.cpu().numpy()).double().contiguous()
+    g = torch.randn(3, 101, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    lib, ps = st._lib, st._paths_struct(b, b.coords, None)
+    for back in (0, 1):
+        own, other = (int(lib.fg_share_workspace(st._h, p, b.n, b.nleg_max, 0 if back else 101, back))
+                      for p in (st.prec, _lib.FG_FP64 if st.prec == _lib.FG_MIXED else _lib.FG_MIXED))
+        call = lib.fg_chi_reduce_backward_workspace if back else lib.fg_chi_reduce_workspace
+        least = 256 + (16 * 3 * 101 + 255) // 256 * 256
+        if back:
+            least = 256 + sum((v + 255) // 256 * 256 for v in (b.n * st.E * 16, b.n * 8, b.n * 256))
+        assert int(call(st._h, C.byref(ps), 101)) == least + max(own, other)
+    assert int(lib.fg_share_workspace(st._h, st.prec, b.n, b.nleg_max, 101, 0)) > 0
+    sizes, empty = [], torch.empty
+
+    def recorded(*args, **kw):
+        if kw.get("dtype") == torch.uint8:
+            sizes.append(args[0])
+        return empty(*args, **kw)
+
+    def full(*args, **kw):
+        if kw.get("dtype") == torch.uint8 and args[0] == max(sizes):
+            raise torch.cuda.OutOfMemoryError("full")
+        return recorded(*args, **kw)
+
+    def step():
+        x = b.coords.clone().requires_grad_(True)
+        rows = st.chi_reduce(b, q, S, coords=x)
+        return rows.detach(), torch.autograd.grad(rows, x, g)[0]
+
+    monkeypatch.setattr(torch, "empty", recorded)
+    rows, gx = step()
+    assert len(sizes) == 2
+    one = st._chi_reduce_forward(b, b.coords, None, q, S, st.prec, True, one_kernel=True)
+    gone = st._chi_reduce_backward(b, b.coords, None, q, S, st.prec, g, one[1], one[2], False, one_kernel=True)[0]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        step()
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in p.key_averages())
+    assert ("k_share_chain" if 6 in counts else "k_stage_energies") in names and "k_fused" not in names
+    del sizes[:]
+    sizes.append(256 + (16 * 3 * 101 + 255) // 256 * 256 + int(lib.fg_share_workspace(st._h, st.prec, b.n, b.nleg_max, 101, 0)))
+    monkeypatch.setattr(torch, "empty", full)
+    small, _ = step()
+    assert torch.equal(small, rows) and torch.equal(rows, one[0])
+    _same(gx, gone, {torch.complex64: 1e-5, torch.complex128: 1e-11}[dtype])

@@ -105,7 +105,11 @@ def chi_reduce_all_ranks(stage, batch, q, S=None, coords=None, sigma2=None, dtyp
     split_groups) with the fused stage, the exact row sums are summed over the ranks as 64-bit integers, and the rows
     are formed from the total -- bit for bit the rows one process computes over all the paths, whatever the number of
     ranks or the split.  Same arguments as GPUPathStage.chi_reduce; differentiable in coords and sigma2 (each rank
-    receives the gradient of its own paths).  One all-reduce of 2 x nrows x NK int64 per call."""
+    receives the gradient of its own paths).  One all-reduce of 2 x nrows x NK int64 per call.
+
+    Over several ranks a path's coordinate gradient is the same bits whichever rank evaluates it and whatever else that
+    rank holds (the one-kernel adjoint); one process's chi_reduce over all the paths agrees with it to the rounding of the
+    sums where it shares derivatives between paths, and bit for bit elsewhere."""
     crd, s2, qt, Sd, prec = stage._reduce_args(batch, q, S, coords, sigma2, dtype)
     return _ChiReduceAllRanks.apply(crd, s2, qt, Sd, stage, batch, prec, group)
 

@@ -355,9 +355,13 @@ class GPUPathStage:
     # -- fused stage ----------------------------------------------------------------------------------------
     def chi_reduce(self, batch: "PathBatch", q, S=None, coords=None, sigma2=None, dtype=None):
         """rows (nrows, len(q)) FP64: sum over the batch's paths of deg exp(-2 sigma2 q^2) chi_path(q) into each
-        path's row, exact in the terms (the result does not depend on the evaluation order).  ``coords`` (n, nleg_max, 3) A replaces the batch's coordinates (same
-        paths, new positions); ``sigma2`` (n,) A^2 per path.  Differentiable in coords and sigma2.  ``dtype``
-        complex64 / complex128 overrides the stage's precision for this call."""
+        path's row, exact in the terms (the result does not depend on the evaluation order).  ``coords`` (n, nleg_max, 3)
+        A replaces the batch's coordinates (same paths, new positions); ``sigma2`` (n,) A^2 per path.  Differentiable in
+        coords and sigma2.  ``dtype`` complex64 / complex128 overrides the stage's precision for this call.
+
+        The rows and sigma2's gradient are the same bits whatever other paths are in the batch.  A path's coordinate
+        gradient is that only up to the rounding of its sums: where scatterers are shared, their derivatives are, and how
+        the sums are split depends on the batch (a repeated call gives the same bits)."""
         if S is None:
             S = self.linear_matrix(q)
         Sd = torch.as_tensor(S).to(self.device, torch.float64).contiguous()

@@ -94,7 +94,19 @@ def test_two_ranks_on_the_cuda_stage_equal_one_process():
         np.testing.assert_allclose(out[r][1], full[mine], rtol=0, atol=1e-12 * np.abs(full).max())
 
 
-def _worker_exact(rank, world, port, out, dtype_name):
+def _sharing(name):
+    """(phase, groups) of a list: FEFF's L001 list, on which one process takes the one-kernel adjoint, or paths of up to
+    six legs over seven atoms on 131 energies, on which it takes the shared one."""
+    from tests.fixtures import phase
+    if name == "L001":
+        return phase("case_L001"), _groups()
+    from feffgpu_b200.pad import resample_phase
+    from tests.test_gpu_shared import _list
+    P = resample_phase(phase("cfg2_phase"), np.linspace(0.0, 20.0, 131))
+    return P, [(c, i, d, r % 2) for c, i, d, r in _list(P.nph, {6: 700, 5: 300, 3: 40, 2: 9}, 7, seed=13)]
+
+
+def _worker_exact(rank, world, port, out, dtype_name, name):
     import torch.distributed as dist
     os.environ["MASTER_ADDR"] = "127.0.0.1"
     os.environ["MASTER_PORT"] = str(port)
@@ -102,9 +114,9 @@ def _worker_exact(rank, world, port, out, dtype_name):
     try:
         from feffgpu_b200 import GPUPathStage, PathBatch
         from feffgpu_b200.sharded import chi_reduce_all_ranks, split_groups
-        from tests.fixtures import phase
-        st = GPUPathStage(phase("case_L001"), device="cuda:0", dtype=getattr(torch, dtype_name))
-        mine = split_groups(_groups(), world, rank, lmax=st.lmax.cpu().numpy())
+        P, groups = _sharing(name)
+        st = GPUPathStage(P, device="cuda:0", dtype=getattr(torch, dtype_name))
+        mine = split_groups(groups, world, rank, lmax=st.lmax.cpu().numpy())
         b = PathBatch(mine, nrows=2, device="cuda:0")
         cg = b.coords.clone().requires_grad_(True)
         s2 = torch.full((b.n,), 0.003, dtype=torch.float64, device="cuda:0", requires_grad=True)
@@ -116,37 +128,54 @@ def _worker_exact(rank, world, port, out, dtype_name):
 
 
 @pytest.mark.parametrize("dtype_name", ["complex64", "complex128"])
-def test_two_ranks_exact_rows_equal_one_process_bit_for_bit(dtype_name):
+@pytest.mark.parametrize("name", ["L001", "sharing"])
+def test_two_ranks_exact_rows_equal_one_process_bit_for_bit(dtype_name, name):
     """chi_reduce_all_ranks: the ranks' exact row sums are summed as 64-bit integers before the rows are formed, so
-    the rows of two ranks equal one process's chi_reduce over all the paths bit for bit (mixed and FP64 forms), and
-    every path's coordinate and sigma^2 gradient equals the one-process one."""
+    the rows of two ranks equal one process's chi_reduce over all the paths bit for bit (mixed and FP64 forms), and so does
+    every path's sigma^2 gradient.  The ranks take the one-kernel adjoint, whose coordinate gradients are the same bits
+    whichever rank evaluates a path: one process's too where its list takes that form, and where it takes the shared one
+    within the rounding of its sums (about 100 terms in another order: 1e-5 of the largest mixed, 1e-11 FP64)."""
     from feffgpu_b200 import GPUPathStage, PathBatch
     from feffgpu_b200.roofline import path_flops
     from feffgpu_b200.sharded import shard
-    from tests.fixtures import phase
     world, port = 2, _free_port()
     ctx = mp.get_context("spawn")
     out = ctx.Manager().dict()
-    procs = [ctx.Process(target=_worker_exact, args=(r, world, port, out, dtype_name)) for r in range(world)]
+    procs = [ctx.Process(target=_worker_exact, args=(r, world, port, out, dtype_name, name)) for r in range(world)]
     for p in procs:
         p.start()
     for p in procs:
         p.join(timeout=600)
         assert p.exitcode == 0
-    gs = _groups()
-    st = GPUPathStage(phase("case_L001"), device="cuda:0", dtype=getattr(torch, dtype_name))
+    P, gs = _sharing(name)
+    st = GPUPathStage(P, device="cuda:0", dtype=getattr(torch, dtype_name))
     b = PathBatch(gs, nrows=2, device="cuda:0")
     cg = b.coords.clone().requires_grad_(True)
     s2 = torch.full((b.n,), 0.003, dtype=torch.float64, device="cuda:0", requires_grad=True)
     rows = st.chi_reduce(b, Q, coords=cg, sigma2=s2)
-    (rows * torch.tensor(_weights(), device="cuda:0")).sum().backward()
+    w = torch.tensor(_weights(), device="cuda:0")
+    (rows * w).sum().backward()
     ref = rows.detach().cpu().numpy()
     for r in range(world):
         assert np.array_equal(out[r][0], ref), r          # bit for bit
+    q = torch.as_tensor(Q, device="cuda:0", dtype=torch.float64)
+    S = st.linear_matrix(Q).double().contiguous()
+    x, s = b.coords.contiguous(), s2.detach()
+    _, cc, rf = st._chi_reduce_forward(b, x, s, q, S, st.prec, True)
+    one = st._chi_reduce_backward(b, x, s, q, S, st.prec, w, cc, rf, True, one_kernel=True)
+    shared = st._lib.fg_share_workspace(st._h, st.prec, b.n, b.nleg_max, 0, 1) > 0
+    assert shared == (name == "sharing")
     nl = b.nleg.cpu().numpy()
     owner = shard(nl, world, path_flops(nl, b.ipots.cpu().numpy(), st.lmax.cpu().numpy()))
     full_c, full_s = cg.grad.cpu().numpy(), s2.grad.cpu().numpy()
+    one_c, one_s = (v.cpu().numpy() for v in one)
+    tol = (1e-5 if dtype_name == "complex64" else 1e-11) * np.abs(full_c).max()
     for r in range(world):
         mine = np.nonzero(owner == r)[0]
         assert np.array_equal(out[r][3], nl[mine])
-        assert np.array_equal(out[r][1], full_c[mine]) and np.array_equal(out[r][2], full_s[mine])
+        assert np.array_equal(out[r][1], one_c[mine]) and np.array_equal(out[r][2], one_s[mine])
+        assert np.array_equal(out[r][2], full_s[mine])
+        if shared:
+            np.testing.assert_allclose(out[r][1], full_c[mine], rtol=0, atol=tol)
+        else:
+            assert np.array_equal(out[r][1], full_c[mine])

@@ -1343,7 +1343,7 @@ fg_status Launch<R, EDGE>::fused_bwd(const StageView &sv, const Tables<R> &T, co
                                                            P->nleg_max - 1, n, P->order + t0, gbar, greff, nullptr, nullptr,
                                                            grad_coords, counter, status, warps, st, gpar, gate))
             return rc;
-        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 3) / 4, (int64_t)sv.num_sms * 16));
+        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 3) / 4, (int64_t)sv.num_sms * 5));
         k_coord_grad<double><<<blocks, 128, 0, st>>>(P->coords, P->nleg_max, P->nleg, 0, n, P->order + t0, gpar,
                                                      grad_coords, status, gate);
         FG_CUDA(cudaGetLastError());

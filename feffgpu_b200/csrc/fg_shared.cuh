@@ -2,24 +2,24 @@
 //
 // A scattering matrix F~_k (before its Euler phase) depends on the leg before the scatterer, the leg after it, the
 // angle between them and the scatterer's potential, and nothing else of the path: the path finder's lists of
-// many-leg paths hold the same triplet of atoms again and again (the 189,419-path benchmark list: 790,095 scatterers,
-// 49,088 different ones).  Here every different (leg length, next leg length, beta, potential) of a call, compared
+// many-leg paths hold the same triplet of atoms again and again (the 189,419-path benchmark list: 789,769 scatterers,
+// 58,897 different ones).  Here every different (leg length, next leg length, beta, potential) of a call, compared
 // bit for bit, is one class; its matrix is formed once per energy and kept in the workspace, and the paths read it:
 //
-//   k_share_geom    a warp per path: geometry, Euler phases, termination rotations (the path's record), the keys
+//   k_share_geom    a thread per (path, leg): geometry, Euler phases, termination rotations (the path's record), the keys
 //   k_share_insert  a thread per scatterer: classes from a hash table of the keys (exact comparison)
 //   k_share_tables  a thread per (class, rotation-table entry): D of every class
 //   k_share_f       a warp per (class, 32 energies): F~ in its two flip blocks; two-leg paths' signals beside them
 //   k_share_chain   a warp per (path, 32 energies): chain product, termination, cfac
-//   k_share_fine    a warp per path (fused calls): fine grid and exact row sums
+//   k_share_fine    a warp per range of paths (fused calls): fine grid and exact row sums
 //
 // Nothing outlives the call: classes are found anew from the call's coordinates.  The arithmetic of every value is
 // that of the one-kernel form (k_fused, k_cchi): the results are the same bits.
 //
 // Measured on B200 (fused forward, 401 energies and k points): 128,844 paths of two to eight legs, 530,707 scatterers
-// in 49,006 classes, mixed form 29.1 -> 9.4 ms (k_share_chain 5.2, k_share_f 2.5, k_share_fine 1.3 ms); 31,142 paths of up
-// to seven legs, FP64 form 14.3 -> 4.5 ms.  What bounds the chain: issue (57 % of cycles) of its 80 complex multiply-adds
-// a step and the latency of the 160 bytes (FP32) of matrix from L1 (13 % hits) and L2 (49 %); fetching the next matrix
+// in 48,885 classes, mixed form 29.1 -> 9.4 ms (k_share_chain 5.2, k_share_f 2.5, k_share_fine 1.3 ms); 31,142 paths of up
+// to seven legs, FP64 form 14.3 -> 4.5 ms.  What bounds the chain: issue (59 % of cycles) of its 80 complex multiply-adds
+// a step and the latency of the 160 bytes (FP32) of matrix from L1 (38 % hits) and L2 (48 %); fetching the next matrix
 // into shared memory while one is multiplied measured the same (5.3 ms), pair instructions 2 % slower, 128 MB passes
 // instead of 1 GB 10 % slower.
 #pragma once
@@ -100,16 +100,22 @@ __device__ __forceinline__ void share_keys(const Share<R> &s, const WarpPath<R> 
 // Records, keys and the list of two-leg paths (a batch that k_validate refused is left alone).  A block takes PB paths
 // at a time, a thread per (path, leg) where path_setup has a warp per path with a lane per leg: same operations, most of
 // the lanes busy (128,844 paths of up to eight legs: 134 us, 292 us with a warp per path).
-// KEYS: the keys and the list of two-leg paths alone (the adjoint, whose records are made once the form is taken).
+// KEYS: the keys and the list of two-leg paths alone (the adjoint, whose records are made once the form is taken), in as much
+// of a record as they need (664 bytes FP32, so that shared memory does not limit the blocks).
+template <typename R, bool KEYS> __host__ __device__ constexpr size_t geom_bytes(size_t rec_bytes)
+{
+    return KEYS ? (__builtin_offsetof(WarpPath<R>, dterm) + 15) / 16 * 16 : rec_bytes;
+}
 template <typename R, typename CT, bool KEYS>
 __global__ void __launch_bounds__(128) k_share_geom(Tables<R> T, Share<R> s, const CT *__restrict__ coords,
                                                     const int64_t *__restrict__ ipots, int *status, int PB)
 {
     if (s.refused()) return;            // not by status: the drop-in call's is the caller's word, whatever it holds
     extern __shared__ __align__(16) unsigned char smem[];
-    double *half = reinterpret_cast<double *>(smem + (size_t)PB * s.rec_bytes);      // cos, sin of beta_nleg / 2
+    const size_t rb = geom_bytes<R, KEYS>(s.rec_bytes);
+    double *half = reinterpret_cast<double *>(smem + (size_t)PB * rb);               // cos, sin of beta_nleg / 2
     const int tid = threadIdx.x, nl = s.nsc_max + 1;
-    auto rec = [&](int l) -> WarpPath<R> & { return *reinterpret_cast<WarpPath<R> *>(smem + (size_t)l * s.rec_bytes); };
+    auto rec = [&](int l) -> WarpPath<R> & { return *reinterpret_cast<WarpPath<R> *>(smem + (size_t)l * rb); };
     for (int64_t i0 = (int64_t)blockIdx.x * PB; i0 < s.n; i0 += (int64_t)gridDim.x * PB) {
         const int cnt = (int)min((int64_t)PB, s.n - i0);
         for (int t = tid; t < cnt * nl * 3; t += 128) {
@@ -530,7 +536,7 @@ fg_status launch_geom(const StageView &sv, const Tables<R> &T, const Share<R> &s
                       int *status, cudaStream_t st)
 {
     const int PB = (int)std::max<int64_t>(1, std::min<int64_t>(128 / (s.nsc_max + 1), s.n / (sv.num_sms * 4)));
-    const size_t gb = PB * (s.rec_bytes + 16);
+    const size_t gb = PB * (geom_bytes<R, KEYS>(s.rec_bytes) + 16);
     int blocks = 0;
     auto kg = k_share_geom<R, CT, KEYS>;
     if (fg_status rc = grid_for(kg, 128, gb, sv.num_sms, (s.n + PB - 1) / PB * 4, blocks)) return rc;
@@ -568,17 +574,10 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
 {
     using K = Kinds<EDGE>;
     constexpr int KIND = K::MS;
-    if (!pl.staged) {
-        FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
-        FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
-    }
-    if (fg_status rc = launch_geom<false>(sv, T, s, coords, ipots, status, st)) return rc;
-    if (pl.staged)
+    if (pl.staged) {
+        if (fg_status rc = launch_geom<false>(sv, T, s, coords, ipots, status, st)) return rc;
         return launch_stage<R, EDGE>(sv, T, s, StagePart<R>{s.tab, s.tab_len, 0, s.n, nullptr}, pl.split, out, st);
-    if (fg_status rc = launch_share_insert(s, st)) return rc;
-    const int64_t tasks = std::min<int64_t>(s.n * s.nsc_max, s.cls_cap) * ncanon(K::MMMS);
-    k_share_tables<R, KIND><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
-    FG_CUDA(cudaGetLastError());
+    }
     const size_t wb = std::max(s.rec_bytes + align_up((size_t)(sv.L1 + 1) * dstride(K::MMSS) * sizeof(R), 16),
                                align_up((size_t)s.tab_len * sizeof(R), 16));
     auto kf = k_share_f<R, EDGE>;
@@ -589,6 +588,13 @@ fg_status ShareLaunch<R, EDGE>::signals(const StageView &sv, const Tables<R> &T,
     const int split = pl.split;
     const size_t wc = 4 * s.rec_bytes;
     if (fg_status rc = grid_for(kc, 128, wc, sv.num_sms, s.n * split, cb)) return rc;
+    FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
+    FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
+    if (fg_status rc = launch_geom<false>(sv, T, s, coords, ipots, status, st)) return rc;
+    if (fg_status rc = launch_share_insert(s, st)) return rc;
+    const int64_t tasks = std::min<int64_t>(s.n * s.nsc_max, s.cls_cap) * ncanon(K::MMMS);
+    k_share_tables<R, KIND><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
+    FG_CUDA(cudaGetLastError());
     for (int pass = 0; pass < pl.passes; ++pass) {
         kf<<<fb, 32 * fw, wb * fw, st>>>(T, s, pass, out, wb);
         kc<<<cb, 128, wc, st>>>(T, s, pass, split, out);
@@ -1141,6 +1147,18 @@ fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T,
     constexpr int KIND = K::MS;
     double *gpar = reinterpret_cast<double *>(ws + pl.gpar);
     s.rec_bytes = geo_bytes<R>() + align_up(sizeof(AdjExtra<R>), 16);
+    // the launches' shapes before the first of them: the short kernels ahead of the matrices leave the host no time
+    auto kf = k_share_f_adj<R, EDGE>;
+    auto kc = k_share_chain_adj<R, EDGE>;
+    auto k2 = k_share_two_adj<R, EDGE>;
+    const size_t wf = align_up(2 * (size_t)s.tab_len * sizeof(R), 16);
+    const size_t w2 = s.rec_bytes + align_up(2 * (size_t)(sv.L1 + 1) * dstride(K::MMSS) * sizeof(R), 16);
+    const int nf = fit_warps(4, wf, sv.max_smem), n2 = fit_warps(4, w2, sv.max_smem), split = pl.split;
+    int bf = 0, bc = 0, b2 = 0;
+    if (fg_status rc = grid_for(kf, 32 * nf, wf * nf, sv.num_sms, s.n * s.nsc_max * pl.chunks * 2, bf)) return rc;
+    const size_t wc = 4 * s.rec_bytes;
+    if (fg_status rc = grid_for(kc, 128, wc, sv.num_sms, s.n * split, bc)) return rc;
+    if (fg_status rc = grid_for(k2, 32 * n2, w2 * n2, sv.num_sms, s.n * split, b2)) return rc;
     FG_CUDA(cudaMemsetAsync(s.head, 0, sizeof(ShareHead), st));
     FG_CUDA(cudaMemsetAsync(s.hash, 0xff, (size_t)pl.hcap * sizeof(unsigned), st));
     const int pb = (int)std::min<int64_t>((s.n + 3) / 4, (int64_t)sv.num_sms * 16);
@@ -1156,17 +1174,6 @@ fg_status ShareLaunch<R, EDGE>::adjoint(const StageView &sv, const Tables<R> &T,
     const int64_t tasks = std::min<int64_t>(s.n * s.nsc_max, s.cls_cap) * ncanon(K::MMMS);
     k_share_tables_adj<R, KIND><<<(int)std::min<int64_t>((tasks + 127) / 128, (int64_t)sv.num_sms * 16), 128, 0, st>>>(T, s);
     FG_CUDA(cudaGetLastError());
-    auto kf = k_share_f_adj<R, EDGE>;
-    auto kc = k_share_chain_adj<R, EDGE>;
-    auto k2 = k_share_two_adj<R, EDGE>;
-    const size_t wf = align_up(2 * (size_t)s.tab_len * sizeof(R), 16);
-    const size_t w2 = s.rec_bytes + align_up(2 * (size_t)(sv.L1 + 1) * dstride(K::MMSS) * sizeof(R), 16);
-    const int nf = fit_warps(4, wf, sv.max_smem), n2 = fit_warps(4, w2, sv.max_smem), split = pl.split;
-    int bf = 0, bc = 0, b2 = 0;
-    if (fg_status rc = grid_for(kf, 32 * nf, wf * nf, sv.num_sms, s.n * s.nsc_max * pl.chunks * 2, bf)) return rc;
-    const size_t wc = 4 * s.rec_bytes;
-    if (fg_status rc = grid_for(kc, 128, wc, sv.num_sms, s.n * split, bc)) return rc;
-    if (fg_status rc = grid_for(k2, 32 * n2, w2 * n2, sv.num_sms, s.n * split, b2)) return rc;
     k2<<<b2, 32 * n2, w2 * n2, st>>>(T, s, split, gbar, gpar, w2);
     for (int pass = 0; pass < pl.passes; ++pass) {
         if (pass == 0) {                                     // beside the two-leg paths' kernel, not after it

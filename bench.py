@@ -901,8 +901,9 @@ def main():
     achieved = flops / (kern_ms * 1e-3) / 1e12 if kern_ms else None
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
             "frac": achieved / peak.value if achieved else None,
-            "kernel": "k_share_f + k_share_chain + k_share_fine, all passes of a step (scattering matrices of the different "
-                      "scatterers, then every path's chain product, termination, cfac and fine grid)",
+            "kernel": "k_share_geom, k_share_insert, k_share_tables, k_share_f, k_share_chain, k_share_fine, all passes of a "
+                      "step (geometry, classes of equal scatterers, their rotation tables and matrices, then every path's "
+                      "chain product, termination, cfac and fine grid; the operations of the last three are counted)",
             "kernel_ms": kern_ms, "flops_per_step": flops, "different_scatterers": classes,
             "reference_loop_flops": ref_flops,
             "peak_source": "measured on this GPU by fg_fp32_fma_peak (FFMA chains on every SM); "

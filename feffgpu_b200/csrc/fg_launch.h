@@ -127,7 +127,8 @@ constexpr int64_t kShareItems = 1 << 16;                   // (path, part of its
 constexpr int64_t kShareSub = 1 << 18;                     // paths per sub-batch (bounds the workspace)
 constexpr int64_t kShareWorth = 1 << 15;                   // (path, 32 energies) items worth looking for classes
 constexpr int64_t kStageWorth = 1 << 12;                   // (path, 32 energies) items from which the staged form pays
-constexpr int64_t kStageSub = 1 << 15;                     // paths per sub-batch of the staged form (its tables stay in L2)
+constexpr int64_t kStageSub = 1 << 15;                     // paths per sub-batch of the staged form (bounds its tables: 110 MB for
+                                                           // three-leg paths at the K edge in FP32)
 constexpr int64_t kShareSmall = 8192;                      // (path, 32 energies) items of a small call
 constexpr size_t kShareMatrixBytes = (size_t)1 << 30;      // the classes' matrices: 2e5 classes, 32 energies, FP32
 struct ShareHead {                      // counters of one sub-batch, in the workspace head

@@ -8,7 +8,8 @@ namespace fg {
 namespace {
 __device__ __forceinline__ unsigned key_hash(const ShareKey &k)
 {
-    // each word's bits spread by an odd multiplier, folded (the finaliser of MurmurHash3, Appleby, public domain)
+    // each word's bits spread by an odd multiplier (2^64 / the golden ratio; the second and third primes of xxHash64, Collet,
+    // BSD), folded by the finaliser of MurmurHash3 (Appleby, public domain)
     unsigned long long h = k.x * 0x9e3779b97f4a7c15ull ^ (k.y * 0xc2b2ae3d27d4eb4full + k.w) ^ (k.z * 0x165667b19e3779f9ull);
     h ^= h >> 33; h *= 0xff51afd7ed558ccdull;
     h ^= h >> 33; h *= 0xc4ceb9fe1a85ec53ull;
@@ -65,7 +66,9 @@ SharePlan share_plan(int64_t n, int nleg_max, int E, int L1, bool fp64, int iord
     // 342 -> 245 us; at the K edge on 60 energies the extra launches cost what the spreading gains: 396 paths forward
     // 421 -> 474 us, backward of 396 and 4,438 paths 445 -> 472 and 1355 -> 1420 us).  Longer paths take it wherever
     // the call is worth the launches that find the classes (about 40 us): at two chunks of energies and 4,438 paths of
-    // up to four legs, 1.27 scatterers per class, looking for them cost 5 %.
+    // up to four legs, 1.27 scatterers per class, looking for them cost 5 %.  Where they are not found, the call goes on in
+    // the staged form (3-4 legs, nothing shared, 401 energies, against the one-kernel form without a search: 700 paths 320
+    // -> 309 us, 1,000 paths, which fill one wave of it, 332 -> 352, 5,000 paths 1,020 -> 983).
     const int chunks = (E + 31) / 32;
     const bool small = n * chunks <= kShareSmall && (chunks >= 4 || ilinit > 1);
     // What is left and large enough takes the staged form (4,438 paths on 60 energies 1.35 -> 1.08 ms a refinement step,

@@ -3,9 +3,9 @@
 The reference keeps path lists as global atom indices and rebuilds the coordinates from the current positions at
 every evaluation (``src/feffgpu/exafs/forward.py:99-163, 664-725``): relative vectors to the absorber under the
 minimum image, absorber first, then ``cchi`` + ``chi_fine`` per chunk and an ``index_add`` into one row per
-absorber/copy.  ``PathModel`` does the same with one ``PathBatch`` and one fused call per evaluation: the gather of
-the coordinates is a differentiable torch indexing (its backward scatters the per-path gradients onto the atoms),
-the stage is ``GPUPathStage.chi_reduce``.  ``GraphedRefinement`` captures one refinement step -- model, R-space
+absorber/copy.  ``PathModel`` does the same with one ``PathBatch`` and one fused call per evaluation: one kernel
+gathers the coordinates of FP64 positions and another sums the per-path gradients onto the atoms in a fixed order
+(differentiable torch indexing for positions of another type or device), the stage is ``GPUPathStage.chi_reduce``.  ``GraphedRefinement`` captures one refinement step -- model, R-space
 misfit, backward and the Adam update -- in a CUDA graph and replays it (the RMC loop of
 ``src/feffgpu/rmc/refine.py:120-260``), re-enumerating the paths and capturing the step again every
 ``refresh_every`` steps as that loop does (``refine.py:176-179``).

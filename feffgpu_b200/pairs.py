@@ -7,8 +7,8 @@ interpolation between grid points, so it is differentiable in the positions) tim
 
 * the tables are one fused-stage call (``GPUPathStage.chi_reduce``): every grid point of every potential a two-leg
   path along z with its own row;
-* the histogram is a CUDA kernel (``fg_pair_histogram``): a block per absorber, weights summed in 2^-32 fixed point
-  with integer atomics (exact, so the result repeats bit for bit);
+* the histogram is a CUDA kernel (``fg_pair_histogram``): a block per absorber, or per four where there are enough to
+  fill the GPU, weights summed in 2^-32 fixed point with integer atomics (exact, so the result repeats bit for bit);
 * ``single_scattering(pos)`` (every atom of every copy an absorber) is the histogram times the tables (a plain
   matrix product), differentiable through its own backward: D = T g per potential, then a kernel
   (``fg_pair_ss_grad``) that gives each atom a block visiting every pair it belongs to.

@@ -8,7 +8,8 @@ window taken on the reference's FP32 R grid.
 
 The transform restricted to the R window is one dense (NR, NK) complex matrix (``transform_matrix``): the same numbers
 as the padded FFT.  The misfit and its gradient are one CUDA kernel (``fg_rspace_misfit``, a cluster of eight blocks
-per row, or, for more than 148 rows, one block per row; FP64, fixed-order sums, the same bits either way): the forward pass already holds dR/dchi, so the backward is a scaling.
+per row, or, for more than 148 rows, one block per row; FP64, fixed-order sums, the same bits either way): the forward
+pass already holds dR/dchi, so the backward is a scaling.
 """
 from __future__ import annotations
 

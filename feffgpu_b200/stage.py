@@ -11,8 +11,8 @@ MD-EXAFS and RMC-EXAFS front ends and their forward model (``src/feffgpu/exafs/f
   ``geometry(coords_bohr) -> (ri, beta, eta)``;
 * attributes ``P``, ``E``, ``rdtype``, ``cdtype``, ``device``, ``iorder``, ``L1``, ``lmax``, ``xk``, ``ck``.
 
-New beside them: ``chi_reduce(batch, q, ...)``, the fused stage: every path of a ``PathBatch`` (mixed leg counts,
-one persistent launch), the fine-grid signal, an optional per-path exp(-2 sigma^2 q^2) and the degeneracy-weighted
+New beside them: ``chi_reduce(batch, q, ...)``, the fused stage: every path of a ``PathBatch`` (mixed leg counts in
+one library call), the fine-grid signal, an optional per-path exp(-2 sigma^2 q^2) and the degeneracy-weighted
 sum into FP64 rows (exact integer sums of the terms rounded to 2^-64: deterministic), differentiable in the
 coordinates and in sigma^2.
 

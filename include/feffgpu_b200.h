@@ -134,7 +134,8 @@ FG_API fg_status fg_chi_fine_backward(const fg_stage *stage, fg_precision prec, 
                                const int32_t *tspan, const void *grad_chi, void *grad_cchi, void *grad_reff,
                                void *stream);
 
-/* A batch of paths with mixed leg counts for the fused stage (one persistent launch over every leg count). */
+/* A batch of paths with mixed leg counts for the fused stage (every leg count in one call: one persistent launch, or, for
+ * batches whose scatterers repeat or whose paths are many and short, a fixed sequence of launches). */
 typedef struct fg_paths {
     int64_t n;               /* paths */
     int32_t nleg_max;        /* leg dimension of coords and ipots (<= 9) */

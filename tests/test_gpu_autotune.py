@@ -33,13 +33,18 @@ def test_shapes_bit_identical_and_tuner_choice(dtype, tmp_path):
     w = torch.randn(b.nrows, len(Q), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
     ref = None
     shapes = [(fw, 4, r, t_) for fw, r, t_ in FWD_SHAPES] + [(4, bw, 0, 0) for bw in BWD_WARPS]
+    q, Sd = torch.as_tensor(Q, device="cuda", dtype=torch.float64), S.double().contiguous()
     for shape in shapes:                         # every forward shape, every adjoint shape
         st.set_launch(*shape)
         x = b.coords.clone().requires_grad_(True)
         s = s2.clone().requires_grad_(True)
         rows = st.chi_reduce(b, Q, S, coords=x, sigma2=s)
         (rows * w).sum().backward()
-        out = (rows.detach(), x.grad, s.grad)
+        # the form that takes the shapes, whichever the call above took
+        one, cc, rf = st._chi_reduce_forward(b, b.coords, s2, q, Sd, st.prec, True, one_kernel=True)
+        grads = st._chi_reduce_backward(b, b.coords, s2, q, Sd, st.prec, w, cc, rf, True, one_kernel=True)
+        assert torch.equal(one, rows.detach())
+        out = (rows.detach(), x.grad, s.grad, one, *grads)
         if ref is None:
             ref = out
         else:
